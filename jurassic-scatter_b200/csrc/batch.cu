@@ -1470,7 +1470,7 @@ static int run_hydro(jsc_batch *b, cudaStream_t s) {
   aa.zmax = b->d_zmax;
   aa.hydz = b->cfg.hydz;
   ev_record(b, JSC_T_HYDRO, 0, s);
-  hydro_kernel<<<(b->n_atm + 127) / 128, 128, 0, s>>>(aa);
+  hydro_kernel<<<b->n_atm, JSC_HYDRO_THREADS, 0, s>>>(aa);
   JSC_LAUNCH_CHECK();
   ev_record(b, JSC_T_HYDRO, 1, s);
   return JSC_OK;

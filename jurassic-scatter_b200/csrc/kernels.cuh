@@ -1,6 +1,6 @@
 // Device kernels of the clear-air forward model.
 //
-//   hydro_kernel      one thread per profile: hydrostatic pressure
+//   hydro_kernel      a block per profile: hydrostatic pressure
 //                     (src/atmosphere.c:163-243) and the profile's z range.
 //   raytrace_kernel   one thread per ray, FP64 refracted ray march
 //                     (src/lineofsight.c:5-190); a counting pass sizes the
@@ -36,28 +36,113 @@ struct AtmArgs {
   double hydz;
 };
 
-// Hydrostatic balance and altitude range of each profile.
-static __global__ void hydro_kernel(AtmArgs a) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= a.n_atm) return;
+// Hydrostatic balance and altitude range of each profile, a block per
+// profile.  The layer means (20 sub-layers each, src/atmosphere.c:206-218)
+// do not depend on the pressures, so the threads take a level each; the
+// pressures themselves are a serial chain of log and exp up and down from
+// the reference level, which every lane of warp 0 runs on layer terms read
+// from shared memory.  Bound by that chain (about 120 x 400 cycles); with a
+// thread per profile the 20 x 120 sub-layers were part of it (1450 us for
+// 20 as for 400 profiles of 121 levels, now 50 us).  A profile whose points
+// do not share one lon/lat holds several columns (jsc_hydrostatic) and runs
+// in one thread.  The operations and their order are those of
+// jsc_hydrostatic_1d.
+#define JSC_HYDRO_THREADS 128
+
+__device__ __forceinline__ double hydro_layer(const double *z, const double *t, const double *qh,
+                                              double latref, int i0, int i1) {
+  const double mmair = 28.96456e-3, mmh2o = 18.0153e-3;
+  const int ipts = 20;
+  double e = 0, mean = 0;
+  for (int i = 0; i < ipts; i++) {
+    const double zz = jsc_lin(0.0, z[i0], ipts - 1.0, z[i1], (double)i);
+    if (qh) e = jsc_lin(0.0, qh[i0], ipts - 1.0, qh[i1], (double)i);
+    mean += (e * mmh2o + (1 - e) * mmair) * jsc_gravity(zz, latref) / JSC_RGAS /
+            jsc_lin(0.0, t[i0], ipts - 1.0, t[i1], (double)i) / ipts;
+  }
+  return mean * 1000 * (z[i1] - z[i0]);
+}
+
+static __global__ void __launch_bounds__(JSC_HYDRO_THREADS) hydro_kernel(AtmArgs a) {
+  __shared__ double term[JSC_HYDRO_THREADS];
+  __shared__ int ref_s;
+  const int i = blockIdx.x, tid = threadIdx.x;
   const int lo = a.off[i], n = a.off[i + 1] - lo;
-  for (int l = 0; l < n; l++) a.p[lo + l] = a.p_in[lo + l];
-  if (a.hydz >= 0 && n > 0) {
-    const double *qh = a.ig_h2o >= 0 ? a.q + (size_t)a.ig_h2o * a.n_levels + lo : nullptr;
-    jsc_hydrostatic(a.hydz, n, a.z + lo, a.lon + lo, a.lat + lo, a.t + lo, qh,
-                    a.p + lo);
+  const double *z = a.z + lo, *lat = a.lat + lo, *lon = a.lon + lo, *t = a.t + lo;
+  double *p = a.p + lo;
+  int mixed = 0;
+  for (int l = tid; l < n; l += JSC_HYDRO_THREADS) {
+    p[l] = a.p_in[lo + l];
+    if (lon[l] != lon[0] || lat[l] != lat[0]) mixed = 1;
+  }
+  // several columns in one profile (a barrier: the copies above are visible)
+  mixed = __syncthreads_or(mixed);
+  const double *qh = a.ig_h2o >= 0 ? a.q + (size_t)a.ig_h2o * a.n_levels + lo : nullptr;
+  if (a.hydz >= 0 && n > 0 && mixed) {
+    if (tid == 0) jsc_hydrostatic(a.hydz, n, z, lon, lat, t, qh, p);
+  } else if (a.hydz >= 0 && n > 0) {
+    if (tid < 32) {  // reference level: the first of the smallest |z - hydz|
+      double best = 1e99;
+      int ib = 0;
+      for (int l = tid; l < n; l += 32)
+        if (fabs(z[l] - a.hydz) < best) {
+          best = fabs(z[l] - a.hydz);
+          ib = l;
+        }
+      for (int o = 16; o > 0; o >>= 1) {
+        const double ob = __shfl_xor_sync(0xffffffffu, best, o);
+        const int oi = __shfl_xor_sync(0xffffffffu, ib, o);
+        if (ob < best || (ob == best && oi < ib)) {
+          best = ob;
+          ib = oi;
+        }
+      }
+      if (tid == 0) ref_s = best < 1e99 ? ib : 0;
+    }
+    __syncthreads();
+    const int ref = ref_s;
+    const double latref = lat[ref];
+    for (int dir = 1; dir >= -1; dir -= 2) {
+      const int cnt = dir > 0 ? n - 1 - ref : ref;  // levels of this direction
+      double pc = p[ref];
+      for (int c0 = 0; c0 < cnt; c0 += JSC_HYDRO_THREADS) {
+        const int k = c0 + tid;
+        if (k < cnt) {
+          const int l = ref + dir * (k + 1);
+          term[tid] = hydro_layer(z, t, qh, latref, l - dir, l);
+        }
+        __syncthreads();
+        if (tid < 32) {
+          const int m = min(JSC_HYDRO_THREADS, cnt - c0);
+          for (int j = 0; j < m; j++) {
+            pc = exp(log(pc) - term[j]);
+            if (tid == 0) p[ref + dir * (c0 + j + 1)] = pc;
+          }
+        }
+        __syncthreads();
+      }
+    }
   }
   // gsl_stats_min/max: first element, then strict comparisons; NaN wins.
-  double mn = n > 0 ? a.z[lo] : 0.0, mx = mn;
+  if (tid >= 32) return;
+  double mn = n > 0 ? z[0] : 0.0, mx = mn;
   bool nan = false;
-  for (int l = 0; l < n; l++) {
-    double v = a.z[lo + l];
+  for (int l = tid; l < n; l += 32) {
+    const double v = z[l];
     if (v < mn) mn = v;
     if (v > mx) mx = v;
     if (isnan(v)) nan = true;
   }
-  a.zmin[i] = nan ? NAN : mn;
-  a.zmax[i] = nan ? NAN : mx;
+  for (int o = 16; o > 0; o >>= 1) {
+    const double a0 = __shfl_xor_sync(0xffffffffu, mn, o), a1 = __shfl_xor_sync(0xffffffffu, mx, o);
+    if (a0 < mn) mn = a0;
+    if (a1 > mx) mx = a1;
+  }
+  nan = __any_sync(0xffffffffu, nan);
+  if (tid == 0) {
+    a.zmin[i] = nan ? NAN : mn;
+    a.zmax[i] = nan ? NAN : mx;
+  }
 }
 
 // --------------------------------------------------------------- raytrace --

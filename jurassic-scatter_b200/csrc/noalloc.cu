@@ -136,7 +136,7 @@ static int noalloc_run(jsc_model *m, const ctl_t *ctl, const jsc_batch_input *in
   aa.zmin = d_zmin;
   aa.zmax = d_zmax;
   aa.hydz = ctl->hydz;
-  hydro_kernel<<<(na + 127) / 128, 128, 0, s>>>(aa);
+  hydro_kernel<<<na, JSC_HYDRO_THREADS, 0, s>>>(aa);
   JSC_LAUNCH_CHECK();
 
   unsigned status = 0;
