@@ -1,5 +1,6 @@
 // Batches: device buffers for many rays over many atmospheric profiles, and
 // the launch sequence of one forward model over them.
+#include <limits.h>
 #include <stdio.h>
 #include <stdlib.h>
 #include <string.h>
@@ -33,6 +34,26 @@ static int batch_alloc_los(jsc_batch *b, int64_t max_seg) {
   return JSC_OK;
 }
 
+// Room in the march pool for n_seg LOS points of max_rays rays: every ray's
+// first chunk, and the chunks that full ones are followed by.
+static int batch_alloc_pool(jsc_batch *b, int64_t n_seg) {
+  cudaFree(b->d_mpts);
+  cudaFree(b->d_mnext);
+  b->d_mpts = nullptr;
+  b->d_mnext = nullptr;
+  b->mcap = 0;
+  const int64_t cap = (int64_t)b->max_rays + n_seg / JSC_CHUNK + 1;
+  if (cap > INT_MAX) {
+    jsc_set_error(JSC_ERR_NOMEM, "%lld LOS points exceed the march pool", (long long)n_seg);
+    return JSC_ERR_NOMEM;
+  }
+  int st;
+  if ((st = jsc_dmalloc(&b->d_mpts, (size_t)cap * JSC_CHUNK * JSC_CHUNK_REC))) return st;
+  if ((st = jsc_dmalloc(&b->d_mnext, (size_t)cap))) return st;
+  b->mcap = (int)cap;
+  return JSC_OK;
+}
+
 extern "C" void jsc_batch_destroy(jsc_batch *b) {
   if (!b) return;
   cudaFree(b->d_atm_off);
@@ -47,6 +68,10 @@ extern "C" void jsc_batch_destroy(jsc_batch *b) {
   cudaFree(b->d_p);
   cudaFree(b->d_zmin);
   cudaFree(b->d_zmax);
+  cudaFree(b->d_lev);
+  cudaFree(b->d_mpts);
+  cudaFree(b->d_mnext);
+  cudaFree(b->d_mcount);
   cudaFree(b->d_ray_atm);
   cudaFree(b->d_ray);
   cudaFree(b->d_nlos);
@@ -180,6 +205,11 @@ extern "C" int jsc_batch_create(jsc_model *m, const ctl_t *ctl, int max_atm,
   st = st ? st : jsc_dmalloc(&b->d_status, 1);
   st = st ? st : jsc_dmalloc(&b->d_counters, 2);
   if (!st) st = batch_alloc_los(b, max_seg > 0 ? max_seg : (int64_t)max_rays * 512);
+  if (b->ip == 1) {
+    st = st ? st : jsc_dmalloc(&b->d_lev, 8 * (size_t)max_levels);
+    st = st ? st : jsc_dmalloc(&b->d_mcount, 1);
+    st = st ? st : batch_alloc_pool(b, b->max_seg);
+  }
   b->scan_tiles = (max_rays + JSC_SCAN_TILE - 1) / JSC_SCAN_TILE + 1;
   st = st ? st : jsc_dmalloc(&b->d_scan, (size_t)b->scan_tiles + 1);
   b->wait_budget = JSC_WAIT_BUDGET;
@@ -191,7 +221,7 @@ extern "C" int jsc_batch_create(jsc_model *m, const ctl_t *ctl, int max_atm,
   b->ctl = (ctl_t *)malloc(sizeof(ctl_t));
   if (!b->ctl) st = st ? st : JSC_ERR_NOMEM;
   else memcpy(b->ctl, ctl, sizeof(ctl_t));
-  if (!st && cudaMallocHost((void **)&b->h_total, sizeof(int64_t)) != cudaSuccess) {
+  if (!st && cudaMallocHost((void **)&b->h_total, 2 * sizeof(int64_t)) != cudaSuccess) {
     jsc_set_error(JSC_ERR_NOMEM, "pinned host allocation");
     st = JSC_ERR_NOMEM;
   }
@@ -666,6 +696,7 @@ static void fill_ray_args(const jsc_batch *b, RayArgs &ra) {
   ra.k = b->d_k;
   ra.zmin = b->d_zmin;
   ra.zmax = b->d_zmax;
+  ra.lev = b->d_lev;
   ra.nlos = b->d_nlos;
   ra.los_off = b->d_los_off;
   ra.W = b->W;
@@ -680,27 +711,16 @@ static void fill_ray_args(const jsc_batch *b, RayArgs &ra) {
   ra.cx = b->cx;
 }
 
-// Counting or storing ray-tracing pass with the batch's interpolation; the
-// pencil batches of a fixed-capacity round pull their rays from the device
-// queue with a persistent grid (7 blocks of 128 per SM, the kernel's cap).
+// Counting or storing ray-tracing pass of a horizontally varying atmosphere.
 template <bool STORE>
-static int launch_raytrace(const jsc_batch *b, const RayArgs &ra, cudaStream_t s) {
-  if (b->d_live) {
-    JSC_CUDA_TRY(cudaMemsetAsync(b->d_qhead, 0, sizeof(unsigned), s));
-    int sms = 148;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, b->m->device);
-    const unsigned g = (unsigned)(sms * 7);
-    if (b->ip == 2) raytrace_queue_kernel<STORE, 2><<<g, 128, 0, s>>>(ra, b->d_qhead, b->d_live);
-    else if (b->ip == 3) raytrace_queue_kernel<STORE, 3><<<g, 128, 0, s>>>(ra, b->d_qhead, b->d_live);
-    else raytrace_queue_kernel<STORE><<<g, 128, 0, s>>>(ra, b->d_qhead, b->d_live);
-    return JSC_OK;
-  }
+static void launch_raytrace(const jsc_batch *b, const RayArgs &ra, cudaStream_t s) {
   const unsigned g = (unsigned)((ra.n_rays + 127) / 128);
   if (b->ip == 2) raytrace_kernel<STORE, 2><<<g, 128, 0, s>>>(ra);
-  else if (b->ip == 3) raytrace_kernel<STORE, 3><<<g, 128, 0, s>>>(ra);
-  else raytrace_kernel<STORE><<<g, 128, 0, s>>>(ra);
-  return JSC_OK;
+  else raytrace_kernel<STORE, 3><<<g, 128, 0, s>>>(ra);
 }
+
+// Eight lanes per ray up to this many rays, a thread per ray above.
+static const int kMarchWide = 16384;
 
 // Live rays of the pencil batches of round `first` (chunk points): the
 // secondary pencils (nalpha per listed point) and the solar pencils.
@@ -886,9 +906,10 @@ static int sun_sources(jsc_batch *b, const double *sp, const int *sp_atm, int n,
                                                   b->d_lat, b->d_psurf);
     JSC_LAUNCH_CHECK();
   }
-  if (b->ip == 2) sun_kernel<2><<<(n + 127) / 128, 128, 0, s>>>(sn);
-  else if (b->ip == 3) sun_kernel<3><<<(n + 127) / 128, 128, 0, s>>>(sn);
-  else sun_kernel<<<(n + 127) / 128, 128, 0, s>>>(sn);
+  if (b->ip == 2) sun_kernel<2, 1><<<(n + 127) / 128, 128, 0, s>>>(sn);
+  else if (b->ip == 3) sun_kernel<3, 1><<<(n + 127) / 128, 128, 0, s>>>(sn);
+  else if (n <= kMarchWide) sun_kernel<1, 8><<<(n + 15) / 16, 128, 0, s>>>(sn);
+  else sun_kernel<1, 1><<<(n + 127) / 128, 128, 0, s>>>(sn);
   JSC_LAUNCH_CHECK();
   int st = batch_run(sc, s);
   if (st) return st;
@@ -1468,6 +1489,7 @@ static int run_hydro(jsc_batch *b, cudaStream_t s) {
   aa.p = b->d_p;
   aa.zmin = b->d_zmin;
   aa.zmax = b->d_zmax;
+  aa.lev = b->d_lev;
   aa.hydz = b->cfg.hydz;
   ev_record(b, JSC_T_HYDRO, 0, s);
   hydro_kernel<<<b->n_atm, JSC_HYDRO_THREADS, 0, s>>>(aa);
@@ -1476,18 +1498,128 @@ static int run_hydro(jsc_batch *b, cudaStream_t s) {
   return JSC_OK;
 }
 
-static int batch_run(jsc_batch *b, cudaStream_t s) {
+static int fixed_unsupported() {
+  jsc_set_error(JSC_ERR_UNSUPPORTED,
+                "fixed-capacity runs cover clear air, aerosol extinction and single "
+                "scattering prepared by jsc_batch_set_fixed");
+  return JSC_ERR_UNSUPPORTED;
+}
+
+// Lines of sight of a run in one-dimensional atmospheres (trace.cuh): march,
+// prefix sum of the counts (with the layer edges), records.  One read-back
+// of the total sizes the LOS buffers (none in a fixed-capacity run).
+static int los_profile(jsc_batch *b, bool refine, cudaStream_t s) {
   const jsc_model *m = b->m;
   const int nr = b->n_rays;
-  for (int k = 0; k < JSC_T_N; k++) b->ran[k] = 0;
-  JSC_CUDA_TRY(cudaMemsetAsync(b->d_status, 0, sizeof(unsigned), s));
-  JSC_CUDA_TRY(cudaMemsetAsync(b->d_counters, 0, 2 * sizeof(unsigned long long), s));
-  {
-    int st = run_hydro(b, s);
-    if (st) return st;
+  int st;
+  RayArgs ra;
+  fill_ray_args(b, ra);
+  ra.nlos = refine ? b->d_nlos_b : b->d_nlos;
+  ExpandArgs xa;
+  memset(&xa, 0, sizeof(xa));
+  xa.n_rays = nr;
+  xa.ng = b->cfg.ng;
+  xa.nw = b->cfg.nw;
+  xa.W = b->W;
+  xa.n_levels = b->n_levels;
+  xa.ig_h2o = m->dv.ig_h2o;
+  xa.ray_atm = b->d_ray_atm;
+  xa.atm_off = b->d_atm_off;
+  xa.z = b->d_z;
+  xa.lev = b->d_lev;
+  xa.q = b->d_q;
+  xa.k = b->d_k;
+  xa.nlos_b = ra.nlos;
+  xa.nlos = b->d_nlos;
+  xa.off = b->d_los_off;
+  xa.tp = b->d_tp;
+  xa.status = b->d_status;
+  if (refine) {
+    xa.E.n_alti = b->n_alti;
+    xa.E.altimax = b->altimax;
+    xa.E.altimin = b->altimin;
+    xa.E.alti = b->d_aero + 3 * NLMAX;
+    xa.nl = b->aero_nl;
+    xa.transs = b->cfg.transs;
+    xa.top = b->d_aero;
+    xa.bottom = b->d_aero + NLMAX;
+    xa.trans = b->d_aero + 2 * NLMAX;
   }
-  if (nr == 0) return JSC_OK;
+  if (m->n_grid == 1) {
+    xa.grid_np = m->grid_np0;
+    xa.grid_p = m->d_grid_p;
+    xa.grid_nt = m->d_grid_nt;
+    xa.grid_t = m->d_grid_t;
+  }
+  const unsigned g32 = (unsigned)(((int64_t)nr * 32 + 127) / 128);
+  if (b->fixed && (b->depth > 1 || (b->depth == 1 && b->fx_rounds < 1))) return fixed_unsupported();
+  for (int pass = 0; pass < 2; pass++) {
+    xa.M.pts = b->d_mpts;
+    xa.M.next = b->d_mnext;
+    xa.M.count = b->d_mcount;
+    xa.M.cap = b->mcap;
+    xa.M.first = nr;
+    xa.max_seg = b->max_seg;
+    JSC_CUDA_TRY(cudaMemsetAsync(b->d_mcount, 0, sizeof(unsigned), s));
+    if (b->d_live) {
+      // rays the queue leaves alone keep no LOS and no surface; a persistent
+      // grid pulls the others
+      JSC_CUDA_TRY(cudaMemsetAsync(ra.nlos, 0, (size_t)nr * sizeof(int), s));
+      JSC_CUDA_TRY(cudaMemsetAsync(b->d_tsurf, 0, (size_t)nr * sizeof(double), s));
+      JSC_CUDA_TRY(cudaMemsetAsync(b->d_qhead, 0, sizeof(unsigned), s));
+      int sms = 148;
+      cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, m->device);
+      march_queue_kernel<<<(unsigned)(sms * 7), 128, 0, s>>>(ra, xa.M, b->d_qhead, b->d_live);
+    } else if (nr <= kMarchWide) {
+      march_kernel<8><<<(unsigned)((nr + 15) / 16), 128, 0, s>>>(ra, xa.M);
+    } else {
+      march_kernel<1><<<(unsigned)((nr + 127) / 128), 128, 0, s>>>(ra, xa.M);
+    }
+    JSC_LAUNCH_CHECK();
+    if (refine) {
+      edge_count_kernel<<<g32, 128, 0, s>>>(xa);
+      JSC_LAUNCH_CHECK();
+    }
+    if ((st = launch_scan(b, b->d_nlos, nr, b->d_los_off, s))) return st;
+    if (b->fixed) {
+      *b->h_total = 0;
+      break;
+    }
+    unsigned *taken = (unsigned *)(b->h_total + 1);
+    JSC_CUDA_TRY(cudaMemcpyAsync(b->h_total, b->d_los_off + nr, sizeof(int64_t),
+                                 cudaMemcpyDeviceToHost, s));
+    JSC_CUDA_TRY(cudaMemcpyAsync(taken, b->d_mcount, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
+    JSC_CUDA_TRY(cudaStreamSynchronize(s));
+    if ((int64_t)*taken + nr <= b->mcap) break;
+    // The pool was too small: the counts of the march are complete all the
+    // same, so the next pass fits.
+    if (refine) {
+      if ((st = launch_scan(b, b->d_nlos_b, nr, b->d_los_off, s))) return st;
+      JSC_CUDA_TRY(cudaMemcpyAsync(b->h_total, b->d_los_off + nr, sizeof(int64_t),
+                                   cudaMemcpyDeviceToHost, s));
+      JSC_CUDA_TRY(cudaStreamSynchronize(s));
+    }
+    if ((st = batch_alloc_pool(b, *b->h_total + *b->h_total / 4 + 1024))) return st;
+  }
+  if (*b->h_total > b->max_seg) {
+    if ((st = batch_alloc_los(b, *b->h_total + *b->h_total / 4 + 1024))) return st;
+  }
+  b->n_points = b->fixed ? b->max_seg : *b->h_total;
+  xa.geo = b->d_geo;
+  xa.pts = b->d_pts;
+  xa.max_seg = b->max_seg;
+  if (refine) expand_kernel<true><<<g32, 128, 0, s>>>(xa);
+  else expand_kernel<false><<<g32, 128, 0, s>>>(xa);
+  JSC_LAUNCH_CHECK();
+  return JSC_OK;
+}
 
+// Lines of sight of a run in a horizontally varying atmosphere (IP 2/3): a
+// counting and a storing pass, then the layer edges as a pass over the raw
+// records.
+static int los_geo(jsc_batch *b, bool refine, cudaStream_t s) {
+  const jsc_model *m = b->m;
+  const int nr = b->n_rays;
   RayArgs ra;
   fill_ray_args(b, ra);
   if (m->n_grid == 1) {
@@ -1496,29 +1628,16 @@ static int batch_run(jsc_batch *b, cudaStream_t s) {
     ra.grid_nt = m->d_grid_nt;
     ra.grid_t = m->d_grid_t;
   }
-  const bool refine = b->cfg.sca_n > 0;
-  if (refine && !b->d_aero) {
-    jsc_set_error(JSC_ERR_ARG, "SCA_N > 0 needs jsc_batch_set_aero before jsc_batch_run");
-    return JSC_ERR_ARG;
-  }
   ra.raw_q = refine;
   ra.nlos = refine ? b->d_nlos_b : b->d_nlos;
   ra.los_off = refine ? b->d_los_off_b : b->d_los_off;
-  ev_record(b, JSC_T_RAYTRACE, 0, s);
-  if (b->ip != 1) {  // surface positions of the profiles (IP 2) or levels (IP 3)
+  {  // surface positions of the profiles (IP 2) or levels (IP 3)
     const int n = b->ip == 2 ? b->n_atm : b->n_levels;
     psurf_kernel<<<(n + 127) / 128, 128, 0, s>>>(n, b->ip == 3, b->d_atm_off, b->d_lon, b->d_lat,
                                                  b->d_psurf);
     JSC_LAUNCH_CHECK();
   }
-  if (b->d_live) {  // rays the queue leaves alone keep no LOS and no surface
-    JSC_CUDA_TRY(cudaMemsetAsync(ra.nlos, 0, (size_t)nr * sizeof(int), s));
-    JSC_CUDA_TRY(cudaMemsetAsync(b->d_tsurf, 0, (size_t)nr * sizeof(double), s));
-  }
-  {
-    const int st = launch_raytrace<false>(b, ra, s);
-    if (st) return st;
-  }
+  launch_raytrace<false>(b, ra, s);
   JSC_LAUNCH_CHECK();
   {
     const int st = launch_scan(b, ra.nlos, nr, (int64_t *)ra.los_off, s);
@@ -1534,13 +1653,7 @@ static int batch_run(jsc_batch *b, cudaStream_t s) {
                                  cudaMemcpyDeviceToHost, s));
     JSC_CUDA_TRY(cudaStreamSynchronize(s));
   }
-  if (b->fixed && (b->depth > 1 || (b->depth == 1 && b->fx_rounds < 1) ||
-                   (refine && b->max_seg_b < b->max_seg))) {
-    jsc_set_error(JSC_ERR_UNSUPPORTED,
-                  "fixed-capacity runs cover clear air, aerosol extinction and single "
-                  "scattering prepared by jsc_batch_set_fixed");
-    return JSC_ERR_UNSUPPORTED;
-  }
+  if (b->fixed && refine && b->max_seg_b < b->max_seg) return fixed_unsupported();
   if (refine) {
     if (*b->h_total > b->max_seg_b) {
       int st = batch_alloc_los_b(b, *b->h_total + *b->h_total / 4 + 1024);
@@ -1559,10 +1672,7 @@ static int batch_run(jsc_batch *b, cudaStream_t s) {
     ra.pts = b->d_pts;
     ra.max_seg = b->max_seg;
   }
-  {
-    const int st = launch_raytrace<true>(b, ra, s);
-    if (st) return st;
-  }
+  launch_raytrace<true>(b, ra, s);
   JSC_LAUNCH_CHECK();
   if (refine) {
     if (b->fixed) {  // keep the refinement's reads inside the base buffer
@@ -1640,10 +1750,34 @@ static int batch_run(jsc_batch *b, cudaStream_t s) {
     {
       const unsigned g = (unsigned)(((int64_t)nr * 32 + 127) / 128);
       if (b->ip == 2) refine_store_kernel<2><<<g, 128, 0, s>>>(fa);
-      else if (b->ip == 3) refine_store_kernel<3><<<g, 128, 0, s>>>(fa);
-      else refine_store_kernel<<<g, 128, 0, s>>>(fa);
+      else refine_store_kernel<3><<<g, 128, 0, s>>>(fa);
     }
     JSC_LAUNCH_CHECK();
+  }
+  return JSC_OK;
+}
+
+static int batch_run(jsc_batch *b, cudaStream_t s) {
+  const jsc_model *m = b->m;
+  const int nr = b->n_rays;
+  for (int k = 0; k < JSC_T_N; k++) b->ran[k] = 0;
+  JSC_CUDA_TRY(cudaMemsetAsync(b->d_status, 0, sizeof(unsigned), s));
+  JSC_CUDA_TRY(cudaMemsetAsync(b->d_counters, 0, 2 * sizeof(unsigned long long), s));
+  {
+    int st = run_hydro(b, s);
+    if (st) return st;
+  }
+  if (nr == 0) return JSC_OK;
+
+  const bool refine = b->cfg.sca_n > 0;
+  if (refine && !b->d_aero) {
+    jsc_set_error(JSC_ERR_ARG, "SCA_N > 0 needs jsc_batch_set_aero before jsc_batch_run");
+    return JSC_ERR_ARG;
+  }
+  ev_record(b, JSC_T_RAYTRACE, 0, s);
+  {
+    const int st = b->ip == 1 ? los_profile(b, refine, s) : los_geo(b, refine, s);
+    if (st) return st;
   }
   if (b->fixed) {
     clamp_los_kernel<<<(nr + 127) / 128, 128, 0, s>>>(b->d_nlos, b->d_los_off, nr, b->max_seg);
@@ -2026,8 +2160,11 @@ extern "C" int jsc_batch_set_fixed(jsc_batch *b, int on) {
   if (on) {
     int st;
     if (b->depth > 0 && (st = prepare_fixed_scattering(b))) return st;
-    if (b->cfg.sca_n > 0 && b->max_seg_b < b->max_seg &&
+    if (b->ip != 1 && b->cfg.sca_n > 0 && b->max_seg_b < b->max_seg &&
         (st = batch_alloc_los_b(b, b->max_seg)))
+      return st;
+    if (b->ip == 1 && (int64_t)b->mcap < (int64_t)b->max_rays + b->max_seg / JSC_CHUNK + 1 &&
+        (st = batch_alloc_pool(b, b->max_seg)))
       return st;
     if (!b->h_status && cudaMallocHost((void **)&b->h_status, sizeof(unsigned)) != cudaSuccess) {
       jsc_set_error(JSC_ERR_NOMEM, "pinned host allocation");

@@ -89,6 +89,7 @@ struct jsc_batch {
   double *d_z, *d_lon, *d_lat, *d_p_in, *d_t, *d_q, *d_k;
   double *d_p;              // pressure after hydrostatic balance
   double *d_zmin, *d_zmax;  // per profile
+  double *d_lev;            // [max_levels][8] level records of the ray march (IP 1)
   int ip;                   // atmosphere interpolation (1 profile, 2, 3)
   double cz, cx;            // IP 3 influence lengths [km]
   double *d_psurf;          // IP 2/3 surface positions [profiles or levels][3]
@@ -103,7 +104,7 @@ struct jsc_batch {
   double *d_beta;           // beta_e, beta_s, beta_a: [3][nl][nd]
   double *d_phase;          // [nl][nd][NTHETA]
   int *d_nlos_b;            // LOS points before the refinement
-  int64_t *d_los_off_b;
+  int64_t *d_los_off_b;     // (IP 2/3, as the records before it)
   double *d_geo_b, *d_pts_b;
   int64_t max_seg_b;
   aero_t *h_aero;           // host copy for child batches
@@ -166,6 +167,13 @@ struct jsc_batch {
   cudaGraphExec_t gexec;
   jsc_batch_input gin;      // host inputs the graph copies from
   int graph_ready, graph_kernels;
+
+  // Pool of the ray march (IP 1): chunks of 32 points, the first max_rays of
+  // them one per ray (trace.cuh).
+  double *d_mpts;
+  int *d_mnext;
+  unsigned *d_mcount;
+  int mcap;
 
   // Line of sight.
   int *d_nlos;

@@ -33,6 +33,7 @@ struct AtmArgs {
   const int *off;
   const double *z, *lon, *lat, *p_in, *t, *q, *k;
   double *p, *zmin, *zmax;
+  double *lev;  // [n_levels][8] level records of the ray march, or null
   double hydz;
 };
 
@@ -123,6 +124,27 @@ static __global__ void __launch_bounds__(JSC_HYDRO_THREADS) hydro_kernel(AtmArgs
       }
     }
   }
+  if (a.lev) {
+    // Level record l: altitudes, pressure and temperature of the interval
+    // [l, l+1], the quotients of EXP (LIN where a pressure is not positive)
+    // and LIN, which of the two, and whether the profile strictly ascends.
+    int down = 0;
+    for (int l = tid; l + 1 < n; l += JSC_HYDRO_THREADS) down |= !(z[l] < z[l + 1]);
+    down = __syncthreads_or(down);  // and the pressures are visible
+    for (int l = tid; l + 1 < n; l += JSC_HYDRO_THREADS) {
+      double *r = a.lev + 8 * (size_t)(lo + l);
+      const double p0 = p[l], p1 = p[l + 1];
+      const bool ex = p0 > 0 && p1 > 0;
+      r[0] = z[l];
+      r[1] = z[l + 1];
+      r[2] = p0;
+      r[3] = t[l];
+      r[4] = ex ? log(p1 / p0) / (z[l + 1] - z[l]) : (p1 - p0) / (z[l + 1] - z[l]);
+      r[5] = (t[l + 1] - t[l]) / (z[l + 1] - z[l]);
+      r[6] = ex ? 1.0 : 0.0;
+      r[7] = down ? 0.0 : 1.0;
+    }
+  }
   // gsl_stats_min/max: first element, then strict comparisons; NaN wins.
   if (tid >= 32) return;
   double mn = n > 0 ? z[0] : 0.0, mx = mn;
@@ -154,6 +176,7 @@ struct RayArgs {
   const int *ray_atm, *atm_off;
   const double *time, *obsz, *obslon, *obslat, *vpz, *vplon, *vplat;
   const double *z, *p, *t, *q, *k, *zmin, *zmax;
+  const double *lev;  // level records (IP 1)
   int *nlos;
   const int64_t *los_off;
   int64_t max_seg;
@@ -636,31 +659,6 @@ __global__ void __launch_bounds__(128, 7) raytrace_kernel(RayArgs A) {
   const int np = trace_ray<STORE, IP>(A, r);
   if (!STORE) A.nlos[r] = np;
   else if (np != A.nlos[r]) atomicOr(A.status, JSC_DEV_ERR_NLOS);
-}
-
-// The pencils of one round of a fixed-capacity scattering run as a device
-// work queue: a persistent grid pulls them a warp (32 pencils) at a time
-// from the queue head until the round's live count, which only the device
-// knows; slots past it are never traced (their nlos stays 0, cleared
-// before the counting pass).  Pulling balances the uneven pencil lengths
-// across the SMs.
-template <bool STORE, int IP = 1>
-__global__ void __launch_bounds__(128, 7) raytrace_queue_kernel(RayArgs A, unsigned *head,
-                                                               const int *live) {
-  const int lane = threadIdx.x & 31;
-  const int n = *live < A.n_rays ? *live : A.n_rays;
-  for (;;) {
-    int r0 = 0;
-    if (lane == 0) r0 = (int)atomicAdd(head, 32u);
-    r0 = __shfl_sync(0xffffffffu, r0, 0);
-    if (r0 >= n) break;
-    const int r = r0 + lane;
-    if (r < n) {
-      const int np = trace_ray<STORE, IP>(A, r);
-      if (!STORE) A.nlos[r] = np;
-      else if (np != A.nlos[r]) atomicOr(A.status, JSC_DEV_ERR_NLOS);
-    }
-  }
 }
 
 // ------------------------------------------------------ aerosol layers --

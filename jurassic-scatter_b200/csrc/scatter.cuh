@@ -18,7 +18,7 @@
 // child batches of one scattering order less), then the radiative transfer
 // with the scattering source at every scattering point.
 #pragma once
-#include "kernels.cuh"
+#include "trace.cuh"
 
 #define JSC_SP_REC 10     // doubles per scattering point record
 #define JSC_NPHI_SCA 180  // azimuth steps of the source integral
@@ -395,25 +395,24 @@ __device__ inline void refined_prev(const SunArgs &A, const double *g0, const do
     if (zp > z1 && zc < z1) znew = z1;
     else if (zp < z2 && zc > z2) znew = z2;
     else continue;
-    double x1[3], x2[3];
-    const double frac = (zp - znew) / (zp - zc);
-    jsc_geo2cart(g0[0], g0[1], g0[2], x1);
-    jsc_geo2cart(g1[0], g1[1], g1[2], x2);
-    for (int i = 0; i < 3; i++) x2[i] = x1[i] + frac * (x2[i] - x1[i]);
-    jsc_cart2geo(x2, &out[0], &out[1], &out[2]);
+    segment_point(g0, g1, znew, out);
   }
 }
 
 // Solar pencil of each scattering point: search the zenith angle whose
 // refracted ray arrives from the sun's direction (up to 10 corrections),
 // then, when that ray does not end on the ground, hand it to the solar
-// child batch with the scattering angle to the LOS direction.
-template <int IP = 1>
+// child batch with the scattering angle to the LOS direction.  LANES (IP 1):
+// lanes of the march per point, as in march_kernel.
+template <int IP, int LANES>
 __global__ void __launch_bounds__(128) sun_kernel(SunArgs A) {
-  const int k = blockIdx.x * blockDim.x + threadIdx.x;
-  if (k >= A.n_pts) return;
+  const int k = (blockIdx.x * blockDim.x + threadIdx.x) / LANES;
+  const int role = LANES == 1 ? 0 : (int)(threadIdx.x & (LANES - 1));
+  const unsigned gmask = LANES == 1 ? 0u : ((1u << LANES) - 1u) << ((threadIdx.x & 31) - role);
+  if (k >= A.n_pts) return;  // whole groups leave together
   if (k >= live_points(A.n_total, A.first, A.n_pts)) {  // null solar pencil, no term
     const int n = A.n_pts;
+    if (role) return;
     A.ray_atm[k] = 0;
     for (int i = 0; i < 7; i++) A.ray[(size_t)i * n + k] = (i == 1 || i == 4) ? JSC_NULL_Z : 0.0;
     A.theta2[k] = -1.0;
@@ -429,7 +428,7 @@ __global__ void __launch_bounds__(128) sun_kernel(SunArgs A) {
   jsc_cart2geo(x, &in.obsz, &in.obslon, &in.obslat);
   jsc_suncoord(o[SP_TIME], in.obslon, in.obslat, &azi, &sza);
   double sza_cor = sza;
-  RayEnd end;
+  RayEnd end = {};
   end.tsurf = -999;
   for (int i2 = 0; i2 < 10; i2++) {
     for (int i = 0; i < 3; i++) {
@@ -439,7 +438,14 @@ __global__ void __launch_bounds__(128) sun_kernel(SunArgs A) {
       x1[i] = x[i] + 10 * ek[i];
     }
     jsc_cart2geo(x1, &in.vpz, &in.vplon, &in.vplat);
-    const int np = trace_core<2, IP>(A.ra, ai, 0, in, &end);
+    int np;
+    if constexpr (IP == 1) {
+      double ts;
+      end.tsurf = -999;
+      np = march_ray<LANES, true>(A.ra, MarchPool(), ai, 0, in, gmask, role, &end, &ts);
+    } else {
+      np = trace_core<2, IP>(A.ra, ai, 0, in, &end);
+    }
     if (np < 2) break;
     double g0[3], xa[3], xb[3], dout[3];
     refined_prev(A, end.g[0], end.g[1], g0);
@@ -451,6 +457,7 @@ __global__ void __launch_bounds__(128) sun_kernel(SunArgs A) {
     sza_cor -= 0.61803 * (sza_beam - sza);
     sza_cor = fmin(fmax(sza_cor, 0.0), 180.0);
   }
+  if (role) return;
   const int n = A.n_pts;
   A.ray_atm[k] = ai;
   A.ray[k] = 0;

@@ -1,0 +1,631 @@
+// Lines of sight of one-dimensional atmospheres (IP 1): the refracted ray
+// march (src/lineofsight.c:5-190) once per ray, and everything that a LOS
+// point needs beside it in parallel over the points.
+//
+//   march_kernel     the march: per ray the number of points, the surface
+//                    temperature and, per point, its position, step and
+//                    smoothed step, in chunks of 32 points
+//   edge_count_kernel  points that the aerosol/cloud layer edges add
+//                    (src/lineofsight.c:193-372), a warp per ray
+//   expand_kernel    the LOS records (state, columns, table brackets, layer
+//                    edges) from the chunks, a warp per ray, a lane per point
+//
+// A march cannot know its length, so it stores as it goes: the first chunk
+// of ray r is chunk r of a pool, further ones are taken from a counter and
+// linked.  The prefix sum of the counts then places the records.
+#pragma once
+#include <limits.h>
+
+#include "kernels.cuh"
+
+#define JSC_CHUNK 32     // points per chunk
+#define JSC_CHUNK_REC 5  // doubles per point: position (3), step, smoothed step
+
+struct MarchPool {
+  double *pts;      // [cap][JSC_CHUNK][JSC_CHUNK_REC]
+  int *next;        // [cap] following chunk of the same ray, -1: none
+  unsigned *count;  // chunks taken beyond the first of each ray
+  int cap, first;   // chunks of the pool; chunks 0 .. first-1 are the rays' first ones
+};
+
+// Pressure and temperature at altitude x (src/atmosphere.c:298-315) from the
+// level records that hydro_kernel builds: the quotients log(p1/p0)/(z1-z0)
+// and (t1-t0)/(z1-z0) that the reference's EXP and LIN evaluate first depend
+// on the level only.  h: level guess; on a strictly ascending profile the
+// level whose altitudes bracket x is the one that jsc_locate finds, so the
+// guess is moved level by level, else (or after four moves) it is searched.
+__device__ __forceinline__ void level_state(const double *__restrict__ lev,
+                                            const double *__restrict__ zl, int n, double x, int &h,
+                                            double *p, double *t) {
+  const double2 *q = reinterpret_cast<const double2 *>(lev) + 4 * (size_t)h;
+  double2 zz = __ldg(q), pt = __ldg(q + 1), sl = __ldg(q + 2), fl = __ldg(q + 3);
+  int moves = 0;
+  while (!(fl.y != 0 && (!(zz.x > x) || h == 0) && (zz.y > x || h == n - 2))) {
+    if (fl.y != 0 && x == x && ++moves <= 4) h += zz.x > x ? -1 : 1;
+    else h = jsc_locate(zl, n, x);
+    q = reinterpret_cast<const double2 *>(lev) + 4 * (size_t)h;
+    zz = __ldg(q);
+    pt = __ldg(q + 1);
+    sl = __ldg(q + 2);
+    fl = __ldg(q + 3);
+    if (fl.y == 0 || !(x == x)) break;  // searched: nothing to verify
+  }
+  const double dz = x - zz.x;
+  *p = fl.x != 0 ? pt.x * exp(sl.x * dz) : pt.x + sl.x * dz;
+  *t = pt.y + sl.y * dz;
+}
+
+// Where the segment from g0 to g1 (z, lon, lat) crosses altitude z
+// (intersection_point, src/lineofsight.c:385-407).
+__device__ __forceinline__ void segment_point(const double *g0, const double *g1, double z,
+                                              double *go) {
+  double x1[3], x2[3];
+  const double frac = (g0[0] - z) / (g0[0] - g1[0]);
+  jsc_geo2cart(g0[0], g0[1], g0[2], x1);
+  jsc_geo2cart(g1[0], g1[1], g1[2], x2);
+  for (int i = 0; i < 3; i++) x2[i] = x1[i] + frac * (x2[i] - x1[i]);
+  jsc_cart2geo(x2, &go[0], &go[1], &go[2]);
+}
+
+__device__ __forceinline__ double radius_of(const double *x) {
+  return sqrt(x[0] * x[0] + x[1] * x[1] + x[2] * x[2]);
+}
+
+// The march of one ray.  LANES 8: a group of eight lanes per ray (gmask:
+// the group's lanes, role: the lane's number in it) holds the same ray
+// state; a refracted step needs the state at five positions (the point, the
+// middle of the step, and that displaced along each axis), and each lane
+// looks up one.  LANES 1: a thread per ray looks them up one after another.
+// ENDS: store nothing, report the last two points in *end (the solar
+// direction search).  Returns the number of points.
+template <int LANES, bool ENDS>
+__device__ __forceinline__ int march_ray(const RayArgs &A, const MarchPool &M, int ai, int r,
+                                         const RayIn &in, unsigned gmask, int role, RayEnd *end,
+                                         double *tsurf) {
+  const int lo = A.atm_off[ai], n = A.atm_off[ai + 1] - lo;
+  const double *__restrict__ lev = A.lev + 8 * (size_t)lo;
+  const double *__restrict__ zl = A.z + lo;
+  const double zmin = A.zmin[ai], zmax = A.zmax[ai];
+  *tsurf = -999;
+  if (in.obsz < zmin) {
+    if (role == 0) atomicOr(A.status, JSC_DEV_ERR_OBSERVER);
+    return 0;
+  }
+  if (in.vpz > zmax - 0.001) return 0;
+
+  double x[3], ex0[3], xp[3] = {0, 0, 0}, xpp[3] = {0, 0, 0};
+  {
+    double xobs[3], xvp[3];
+    jsc_geo2cart(in.obsz, in.obslon, in.obslat, xobs);
+    jsc_geo2cart(in.vpz, in.vplon, in.vplat, xvp);
+    for (int i = 0; i < 3; i++) ex0[i] = xvp[i] - xobs[i];
+    const double norm = radius_of(ex0);
+    for (int i = 0; i < 3; i++) ex0[i] /= norm;
+    for (int i = 0; i < 3; i++) x[i] = xobs[i];
+    // Observer above the atmosphere: bisect for the entry point.
+    if (in.obsz > zmax) {
+      double dmin = 0, dmax = norm;
+      while (fabs(dmin - dmax) > 0.001) {
+        const double d = (dmax + dmin) / 2;
+        for (int i = 0; i < 3; i++) x[i] = xobs[i] + d * ex0[i];
+        const double z = radius_of(x) - JSC_RE;
+        if (z <= zmax && z > zmax - 0.001) break;
+        if (z < zmax - 0.0005) dmax = d; else dmin = d;
+      }
+    }
+  }
+
+  int np = 0, chunk = r, h0 = n - 2, h1 = n - 2;
+  double rprev = 0, dprev = 0, tlast = 0, zlast = 0;
+  bool bent = true;  // tlast holds the temperature looked up last
+  while (1) {
+    if (np >= NLOS) {
+      if (role == 0) atomicOr(A.status, JSC_DEV_ERR_NLOS);
+      return np;
+    }
+    const double norm = radius_of(x), z = norm - JSC_RE;
+    double *rec = nullptr;
+    if (!ENDS) {
+      if ((np & (JSC_CHUNK - 1)) == 0 && np > 0 && chunk >= 0) {  // the next chunk
+        int id = 0;
+        if (role == 0) {
+          id = M.first + (int)atomicAdd(M.count, 1u);
+          if (id >= M.cap || id < 0) id = -1;
+          M.next[chunk] = id;
+        }
+        chunk = LANES == 1 ? id : __shfl_sync(gmask, id, 0, LANES);
+      }
+      if (chunk >= 0)
+        rec = M.pts + ((size_t)chunk * JSC_CHUNK + (np & (JSC_CHUNK - 1))) * JSC_CHUNK_REC;
+    }
+    if (z < zmin + 0.001 || z > zmax + 0.001) {
+      // Last point: where the segment from the previous point crosses the
+      // boundary.  It is stored as (z, lon, lat) with a step of 0.
+      const int stop = z < zmin + 0.001 ? 2 : 1;
+      double g0[3], g1[3], g[3];
+      jsc_cart2geo(x, &g1[0], &g1[1], &g1[2]);
+      if (np > 0) jsc_cart2geo(xp, &g0[0], &g0[1], &g0[2]);
+      else for (int i = 0; i < 3; i++) g0[i] = g1[i];
+      segment_point(g0, g1, stop == 2 ? zmin : zmax, g);
+      if (rec && role == 0) {
+        rec[0] = g[0];
+        rec[1] = g[1];
+        rec[2] = g[2];
+        rec[3] = 0.;
+        rec[4] = np == 0 ? 0. : 0.5 * (dprev + 0.);
+      }
+      np++;
+      if (stop == 2) {
+        if (!bent) {
+          double p;
+          level_state(lev, zl, n, zlast, h0, &p, &tlast);
+        }
+        *tsurf = tlast;
+      }
+      // A last point that follows a too-short step is dropped
+      // (src/lineofsight.c:170-171).
+      const bool dropped = np >= 3 && rprev < 1e-3;
+      if (dropped) np--;
+      if (ENDS) {
+        end->tsurf = *tsurf;
+        if (dropped) jsc_cart2geo(xpp, &end->g[0][0], &end->g[0][1], &end->g[0][2]);
+        for (int i = 0; i < 3; i++) {
+          if (!dropped) end->g[0][i] = g0[i];
+          end->g[1][i] = dropped ? g0[i] : g[i];
+        }
+      }
+      break;
+    }
+    double ds = A.rayds;
+    if (A.raydz > 0) {
+      double xh[3];
+      for (int i = 0; i < 3; i++) xh[i] = x[i] / norm;
+      const double cosa = fabs(ex0[0] * xh[0] + ex0[1] * xh[1] + ex0[2] * xh[2]);
+      if (cosa != 0) {
+        const double dz = A.raydz / cosa;
+        ds = (A.rayds < dz ? A.rayds : dz);  // GSL_MIN
+      }
+    }
+    // Steps are smoothed along the ray (src/lineofsight.c:177-179).
+    const double dsm = np == 0 ? 0.5 * ds : 0.5 * (dprev + ds);
+    if (rec) {
+      if (LANES == 1) {
+        rec[0] = x[0];
+        rec[1] = x[1];
+        rec[2] = x[2];
+        rec[3] = ds;
+        rec[4] = dsm;
+      } else if (role < JSC_CHUNK_REC) {
+        rec[role] = role == 0 ? x[0] : role == 1 ? x[1] : role == 2 ? x[2] : role == 3 ? ds : dsm;
+      }
+    }
+    np++;
+    rprev = ds;
+    dprev = dsm;
+    if (ENDS)
+      for (int i = 0; i < 3; i++) xpp[i] = xp[i];
+    for (int i = 0; i < 3; i++) xp[i] = x[i];
+
+    // Refraction (src/lineofsight.c:122-166).
+    bent = A.refrac && z <= JSC_ZREFRAC;
+    double ex1[3], ng[3] = {0, 0, 0}, nr = 1;
+    if (bent) {
+      double xm[3];
+      for (int i = 0; i < 3; i++) xm[i] = x[i] + 0.5 * ds * ex0[i];
+      double p, t;
+      if (LANES > 1) {
+        // lane 0 the point, 1 the middle, 2-4 the middle displaced; the
+        // reference displaces in place, so an axis displaced before keeps
+        // the rounding of + step - step
+        for (int i = 0; i < 3; i++) {
+          const double up = xm[i] + JSC_FD_STEP;
+          if (role == 2 + i) xm[i] = up;
+          else if (role > 2 + i) xm[i] = up - JSC_FD_STEP;
+        }
+        if (role == 0 || role > 4)
+          for (int i = 0; i < 3; i++) xm[i] = x[i];
+        level_state(lev, zl, n, radius_of(xm) - JSC_RE, h0, &p, &t);
+        const double rf = jsc_refractivity(p, t);
+        nr = 1 + __shfl_sync(gmask, rf, 0, LANES);
+        const double g = (rf - __shfl_sync(gmask, rf, 1, LANES)) / JSC_FD_STEP;
+        for (int i = 0; i < 3; i++) ng[i] = __shfl_sync(gmask, g, 2 + i, LANES);
+        tlast = __shfl_sync(gmask, t, 4, LANES);
+      } else {
+        level_state(lev, zl, n, z, h0, &p, &t);
+        nr = 1 + jsc_refractivity(p, t);
+        level_state(lev, zl, n, radius_of(xm) - JSC_RE, h1, &p, &t);
+        const double rm = jsc_refractivity(p, t);
+        int h2 = h1;
+#pragma unroll
+        for (int i = 0; i < 3; i++) {
+          xm[i] += JSC_FD_STEP;
+          level_state(lev, zl, n, radius_of(xm) - JSC_RE, h2, &p, &t);
+          ng[i] = (jsc_refractivity(p, t) - rm) / JSC_FD_STEP;
+          xm[i] -= JSC_FD_STEP;
+        }
+        tlast = t;
+      }
+    } else {
+      zlast = z;
+    }
+    for (int i = 0; i < 3; i++) ex1[i] = ex0[i] * nr;
+    for (int i = 0; i < 3; i++) ex1[i] += ds * ng[i];
+    const double en = radius_of(ex1);
+    for (int i = 0; i < 3; i++) ex1[i] /= en;
+    for (int i = 0; i < 3; i++) x[i] += 0.5 * ds * (ex0[i] + ex1[i]);
+    for (int i = 0; i < 3; i++) ex0[i] = ex1[i];
+  }
+  return np;
+}
+
+template <int LANES>
+__device__ __forceinline__ void march_one(const RayArgs &A, const MarchPool &M, int r,
+                                          unsigned gmask, int role) {
+  const RayIn in = {A.obsz[r], A.obslon[r], A.obslat[r], A.vpz[r], A.vplon[r], A.vplat[r]};
+  double tsurf;
+  const int np = march_ray<LANES, false>(A, M, A.ray_atm[r], r, in, gmask, role, nullptr, &tsurf);
+  if (role == 0) {
+    A.nlos[r] = np;
+    A.tsurf[r] = tsurf;
+    if (np == 0) {
+      A.tp[r] = in.vpz;
+      A.tp[A.n_rays + r] = in.vplon;
+      A.tp[2 * A.n_rays + r] = in.vplat;
+    }
+  }
+}
+
+template <int LANES>
+__global__ void __launch_bounds__(128) march_kernel(RayArgs A, MarchPool M) {
+  const int tid = blockIdx.x * blockDim.x + threadIdx.x, r = tid / LANES;
+  const int role = LANES == 1 ? 0 : (int)(threadIdx.x & (LANES - 1));
+  const unsigned gmask = LANES == 1 ? 0u : ((1u << LANES) - 1u) << ((threadIdx.x & 31) - role);
+  if (r >= A.n_rays) return;  // whole groups leave together
+  march_one<LANES>(A, M, r, gmask, role);
+}
+
+// The pencils of one round of a fixed-capacity scattering run as a device
+// work queue: a persistent grid pulls them a warp (32 pencils) at a time
+// from the queue head until the round's live count, which only the device
+// knows; slots past it are never traced (their nlos stays 0, cleared
+// before).  Pulling balances the uneven pencil lengths across the SMs.
+static __global__ void __launch_bounds__(128) march_queue_kernel(RayArgs A, MarchPool M,
+                                                                 unsigned *head, const int *live) {
+  const int lane = threadIdx.x & 31;
+  const int n = *live < A.n_rays ? *live : A.n_rays;
+  for (;;) {
+    int r0 = 0;
+    if (lane == 0) r0 = (int)atomicAdd(head, 32u);
+    r0 = __shfl_sync(0xffffffffu, r0, 0);
+    if (r0 >= n) break;
+    if (r0 + lane < n) march_one<1>(A, M, r0 + lane, 0u, 0);
+  }
+}
+
+// ------------------------------------------------------ aerosol layers --
+
+// Layer edges as the refinement sees them (n_alti altitudes, top down).
+struct EdgeSet {
+  int n_alti;
+  double altimax, altimin;
+  const double *alti;
+};
+
+// Crossings of the segment from altitude zp to zc with the edges
+// (src/lineofsight.c:252-290).
+__device__ __forceinline__ bool edge_window(const EdgeSet &E, double zp, double zc) {
+  return (zp < E.altimax || zc < E.altimax) && (zp > E.altimin || zc > E.altimin);
+}
+
+__device__ __forceinline__ int edge_crossings(const EdgeSet &E, double zp, double zc) {
+  int c = 0;
+  if (edge_window(E, zp, zc))
+    for (int il = 0; il < E.n_alti; il++) {
+      const double z1 = E.alti[il], z2 = E.alti[E.n_alti - il - 1];
+      c += (zp > z1 && zc < z1) + (zp < z2 && zc > z2);
+    }
+  return c;
+}
+
+__device__ __forceinline__ double chunk_altitude(const double *rec) {
+  return rec[3] == 0. ? rec[0] : radius_of(rec) - JSC_RE;
+}
+
+struct ExpandArgs {
+  int n_rays, ng, nw, W, n_levels, ig_h2o;
+  const int *ray_atm, *atm_off;
+  const double *z, *lev, *q, *k;   // profiles
+  MarchPool M;
+  const int *nlos_b;               // points of the march
+  int *nlos;                       // points with the layer edges
+  const int64_t *off;
+  double *geo, *pts, *tp;
+  int64_t max_seg;
+  EdgeSet E;
+  int nl;                          // aerosol/cloud layers
+  double transs;
+  const double *top, *bottom, *trans;
+  int grid_np;                     // (p, T) grid shared by every table
+  const double *grid_p, *grid_t;
+  const int *grid_nt;
+  unsigned *status;
+};
+
+// Points of each ray with the layer edges: its marched points plus the
+// crossings of its segments.
+static __global__ void __launch_bounds__(128) edge_count_kernel(ExpandArgs A) {
+  const int r = (int)(((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+  const int lane = threadIdx.x & 31;
+  if (r >= A.n_rays) return;  // whole warps leave together
+  const int nb = A.nlos_b[r];
+  int o = 0, chunk = r;
+  double carry = 0;  // altitude of the point before the chunk
+  for (int c0 = 0; c0 < nb && chunk >= 0; c0 += JSC_CHUNK) {
+    const int ip = c0 + lane;
+    double zc = 0;
+    if (ip < nb) zc = chunk_altitude(A.M.pts + ((size_t)chunk * JSC_CHUNK + lane) * JSC_CHUNK_REC);
+    double zp = __shfl_up_sync(0xffffffffu, zc, 1);
+    if (lane == 0) zp = carry;
+    carry = __shfl_sync(0xffffffffu, zc, 31);
+    if (ip < nb) o += 1 + (ip > 0 ? edge_crossings(A.E, zp, zc) : 0);
+    if (c0 + JSC_CHUNK < nb) chunk = A.M.next[chunk];
+  }
+  o = __reduce_add_sync(0xffffffffu, o);
+  if (lane) return;
+  if (o > NLOS || o > A.max_seg) {
+    atomicOr(A.status, JSC_DEV_ERR_NLOS);
+    o = 0;
+  }
+  A.nlos[r] = o;
+}
+
+// Record of a LOS point: the state at its altitude z, the column densities
+// over its step ds (src/lineofsight.c:182-185), the table brackets, and the
+// layer factor (af, ai).
+__device__ __forceinline__ void write_record(const ExpandArgs &A, const Profile &a,
+                                             const double *lev, double *rec, double z, double ds,
+                                             double af, double ai) {
+  // level guess for evenly spaced altitudes
+  const double zf = a.z[0];
+  int h = (int)fmin(fmax((z - zf) / (a.z[a.n - 1] - zf) * (a.n - 1), 0.0), (double)(a.n - 2));
+  double p, t;
+  level_state(lev, a.z, a.n, z, h, &p, &t);
+  rec[REC_P] = p;
+  rec[REC_T] = t;
+  rec[REC_DS] = ds;
+  rec[REC_QH2O] = A.ig_h2o >= 0 ? atm_lin(a.q + (size_t)A.ig_h2o * a.stride, a, h, z) : 0.0;
+  rec[REC_GRID] = A.grid_p ? (double)grid_code(A.grid_np, A.grid_p, A.grid_nt, A.grid_t, p, t) : -1.0;
+  rec[REC_PLK] = (double)planck_index(t);
+  rec[REC_AF] = af;
+  rec[REC_AI] = ai;
+  for (int w = 0; w < A.nw; w++) rec[REC_K + w] = atm_lin(a.k + (size_t)w * a.stride, a, h, z);
+  for (int g = 0; g < A.ng; g++) {
+    const double q = atm_lin(a.q + (size_t)g * a.stride, a, h, z);
+    rec[REC_K + A.nw + g] = 10 * q * p / (JSC_KBOLTZ * t) * ds;
+  }
+}
+
+// Aerosol/cloud layer and factor of a point at altitude z whose predecessor
+// lies at zprev (src/lineofsight.c:332-372).
+__device__ __forceinline__ void layer_factor(const ExpandArgs &A, double zprev, double z,
+                                             double *af, double *ai) {
+  int aeroi = -999;
+  double aerofac = 0.;
+  if (edge_window(A.E, zprev, z)) {
+    for (int il = 0; il < A.nl; il++) {
+      if (z <= A.top[il] && z >= A.bottom[il]) {
+        aeroi = il;
+        aerofac = 1.;
+      }
+      if (A.trans[il] > A.transs && z <= (A.top[il] + A.trans[il]) && z > A.top[il]) {
+        aeroi = il;
+        aerofac = (A.top[il] + A.trans[il] - z) / A.trans[il];
+      }
+      if (A.trans[il] > A.transs && z < A.bottom[il] && z >= (A.bottom[il] - A.trans[il])) {
+        aeroi = il;
+        aerofac = fabs(A.bottom[il] - A.trans[il] - z) / A.trans[il];
+      }
+    }
+  }
+  *af = aerofac;
+  *ai = (double)aeroi;
+}
+
+// Geometry and step of marched point ip of ray r (walks the ray's chunks).
+__device__ inline double marched_point(const MarchPool &M, int r, int ip, double *g) {
+  int chunk = r;
+  for (int c = ip / JSC_CHUNK; c > 0 && chunk >= 0; c--) chunk = M.next[chunk];
+  if (chunk < 0) {
+    g[0] = g[1] = g[2] = 0;
+    return 0;
+  }
+  const double *rec = M.pts + ((size_t)chunk * JSC_CHUNK + (ip & (JSC_CHUNK - 1))) * JSC_CHUNK_REC;
+  if (rec[3] == 0.)
+    for (int i = 0; i < 3; i++) g[i] = rec[i];
+  else
+    jsc_cart2geo(rec, &g[0], &g[1], &g[2]);
+  return rec[3];
+}
+
+// Tangent point of ray r with np marched points whose lowest is m
+// (src/lineofsight.c:411-452).
+__device__ inline void tangent_point(const ExpandArgs &A, int r, int np, int m) {
+  double g0[3], g1[3], g2[3], tp[3];
+  if (m <= 0 || m >= np - 1) {
+    marched_point(A.M, r, np - 1, tp);
+  } else {
+    marched_point(A.M, r, m - 1, g0);
+    const double d1 = marched_point(A.M, r, m, g1), d2 = marched_point(A.M, r, m + 1, g2);
+    const double yy0 = g0[0], yy1 = g1[0], yy2 = g2[0];
+    const double x1 = sqrt(d1 * d1 - (yy1 - yy0) * (yy1 - yy0));
+    const double x2 = x1 + sqrt(d2 * d2 - (yy2 - yy1) * (yy2 - yy1));
+    const double aa = 1 / (x1 - x2) * (-(yy0 - yy1) / x1 + (yy0 - yy2) / x2);
+    const double bb = -(yy0 - yy1) / x1 - aa * x1;
+    const double cc = yy0;
+    const double xx = -bb / (2 * aa);
+    double v0[3], v2[3], v[3], dummy;
+    tp[0] = aa * xx * xx + bb * xx + cc;
+    jsc_geo2cart(g0[0], g0[1], g0[2], v0);
+    jsc_geo2cart(g2[0], g2[1], g2[2], v2);
+    for (int i = 0; i < 3; i++) v[i] = jsc_lin(0.0, v0[i], x2, v2[i], xx);
+    jsc_cart2geo(v, &dummy, &tp[1], &tp[2]);
+  }
+  for (int i = 0; i < 3; i++) A.tp[(size_t)i * A.n_rays + r] = tp[i];
+}
+
+// LOS records of a ray by one warp.  EDGES: the points where segments cross
+// layer edges go in between (add_aerosol_layers, src/lineofsight.c:193-372):
+// lanes take 32 marched points at a time, a warp scan of their output counts
+// (crossings of the segment before the point, then the point) places the
+// geometry, then lanes take 32 points at a time for the records, with the
+// neighbours' Cartesian positions passed by shuffles for the chord steps.
+template <bool EDGES>
+__global__ void __launch_bounds__(128, 6) expand_kernel(ExpandArgs A) {
+  const int r = (int)(((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+  const int lane = threadIdx.x & 31;
+  const unsigned full = 0xffffffffu;
+  if (r >= A.n_rays) return;  // whole warps leave together
+  const int nb = A.nlos_b[r];
+  if (nb == 0) return;
+  const int ai = A.ray_atm[r], lo = A.atm_off[ai];
+  Profile a;
+  a.n = A.atm_off[ai + 1] - lo;
+  a.stride = A.n_levels;
+  a.z = A.z + lo;
+  a.q = A.q + lo;
+  a.k = A.k + lo;
+  a.p = a.t = nullptr;
+  const double *lev = A.lev + 8 * (size_t)lo;
+  const int64_t base = A.off[r];
+  const int nmax = EDGES ? A.nlos[r] : nb;
+  // lowest marched point: the first NaN, else the first smallest altitude
+  double zlow = 0;
+  int mlow = INT_MAX, mnan = INT_MAX;
+  double prev[3] = {0, 0, 0};  // geometry of the point before the chunk
+  int chunk = r, o = 0;
+  for (int c0 = 0; c0 < nb; c0 += JSC_CHUNK) {
+    if (chunk < 0) {  // the march ran out of chunks
+      if (lane == 0) atomicOr(A.status, JSC_DEV_ERR_NLOS);
+      return;
+    }
+    const int ip = c0 + lane;
+    const double *rec = A.M.pts + ((size_t)chunk * JSC_CHUNK + lane) * JSC_CHUNK_REC;
+    double g[3] = {0, 0, 0}, raw = 0, ds = 0;
+    if (ip < nb) {
+      const double c[3] = {rec[0], rec[1], rec[2]};
+      raw = rec[3];
+      ds = rec[4];
+      if (raw == 0.)
+        for (int i = 0; i < 3; i++) g[i] = c[i];
+      else
+        jsc_cart2geo(c, &g[0], &g[1], &g[2]);
+      if (isnan(g[0])) mnan = min(mnan, ip);
+      else if (mlow == INT_MAX || g[0] < zlow) {
+        zlow = g[0];
+        mlow = ip;
+      }
+    }
+    if (!EDGES) {
+      if (ip < nb) {
+        if (base + ip >= A.max_seg) {
+          atomicOr(A.status, JSC_DEV_ERR_NLOS);
+        } else {
+          double *go = A.geo + (base + ip) * 4;
+          go[0] = g[0];
+          go[1] = g[1];
+          go[2] = g[2];
+          go[3] = raw;
+          write_record(A, a, lev, A.pts + (base + ip) * A.W, g[0], ds, 0.0, -999.0);
+        }
+      }
+    } else {
+      double gp[3];
+      for (int i = 0; i < 3; i++) {
+        gp[i] = __shfl_up_sync(full, g[i], 1);
+        if (lane == 0) gp[i] = prev[i];
+        prev[i] = __shfl_sync(full, g[i], 31);
+      }
+      const int add = ip < nb && ip > 0 ? edge_crossings(A.E, gp[0], g[0]) : 0;
+      const int cnt = ip < nb ? 1 + add : 0;
+      int incl = cnt;
+      for (int d = 1; d < 32; d <<= 1) {
+        const int v = __shfl_up_sync(full, incl, d);
+        if (lane >= d) incl += v;
+      }
+      const int total = __shfl_sync(full, incl, 31);
+      if (o + total > nmax || base + o + total > A.max_seg) {
+        if (lane == 0) atomicOr(A.status, JSC_DEV_ERR_NLOS);
+        return;
+      }
+      if (ip < nb) {
+        double *go = A.geo + (base + o + incl - cnt) * 4;  // first output slot of this lane
+        if (add)
+          for (int il = 0; il < A.E.n_alti; il++) {
+            const double z1 = A.E.alti[il], z2 = A.E.alti[A.E.n_alti - il - 1];
+            if (gp[0] > z1 && g[0] < z1) {
+              segment_point(gp, g, z1, go);
+              go += 4;
+            }
+            if (gp[0] < z2 && g[0] > z2) {
+              segment_point(gp, g, z2, go);
+              go += 4;
+            }
+          }
+        go[0] = g[0];
+        go[1] = g[1];
+        go[2] = g[2];
+      }
+      o += total;
+    }
+    if (c0 + JSC_CHUNK < nb) chunk = A.M.next[chunk];
+  }
+  for (int d = 16; d > 0; d >>= 1) {
+    const double oz = __shfl_xor_sync(full, zlow, d);
+    const int om = __shfl_xor_sync(full, mlow, d);
+    if (om != INT_MAX && (mlow == INT_MAX || oz < zlow || (oz == zlow && om < mlow))) {
+      zlow = oz;
+      mlow = om;
+    }
+  }
+  mnan = __reduce_min_sync(full, mnan);
+  if (lane == 0) tangent_point(A, r, nb, mnan != INT_MAX ? mnan : mlow);
+  if (!EDGES) return;
+  __syncwarp();  // the geometry written above, for every lane
+  const double *go = A.geo + base * 4;
+  double carry[3] = {0, 0, 0};  // position of the point before the 32
+  for (int i0 = 0; i0 < o; i0 += 32) {
+    const int i = i0 + lane;
+    double xc[3] = {0, 0, 0}, xp[3], xn[3], z = 0;
+    if (i < o) {
+      z = go[(size_t)i * 4];
+      jsc_geo2cart(z, go[(size_t)i * 4 + 1], go[(size_t)i * 4 + 2], xc);
+    }
+    for (int c = 0; c < 3; c++) {
+      const double up = __shfl_up_sync(full, xc[c], 1);
+      const double dn = __shfl_down_sync(full, xc[c], 1);
+      xp[c] = lane == 0 ? carry[c] : up;
+      xn[c] = dn;
+      carry[c] = __shfl_sync(full, xc[c], 31);
+    }
+    if (lane == 31 && i + 1 < o)
+      jsc_geo2cart(go[(size_t)(i + 1) * 4], go[(size_t)(i + 1) * 4 + 1],
+                   go[(size_t)(i + 1) * 4 + 2], xn);
+    if (i < o) {
+      // chord step (src/lineofsight.c:300-330)
+      double ds = 0;
+      if (o > 1) {
+        const double back = sqrt((xp[0] - xc[0]) * (xp[0] - xc[0]) + (xp[1] - xc[1]) * (xp[1] - xc[1]) +
+                                 (xp[2] - xc[2]) * (xp[2] - xc[2]));
+        const double ahead = sqrt((xc[0] - xn[0]) * (xc[0] - xn[0]) + (xc[1] - xn[1]) * (xc[1] - xn[1]) +
+                                  (xc[2] - xn[2]) * (xc[2] - xn[2]));
+        ds = i == 0 ? 0.5 * ahead : i == o - 1 ? 0.5 * back : 0.5 * (back + ahead);
+      }
+      A.geo[(base + i) * 4 + 3] = ds;
+      // At i = 0 the reference compares z[-1]; the first point, at the top
+      // of the atmosphere and outside every layer, stands in for it.
+      double af, la;
+      layer_factor(A, go[(size_t)(i > 0 ? i - 1 : 0) * 4], z, &af, &la);
+      write_record(A, a, lev, A.pts + (base + i) * A.W, z, ds, af, la);
+    }
+  }
+}

@@ -1,9 +1,12 @@
 """Edge sizes of the batch kernels against host restatements: sizes at the
 ends of a kernel's tiles, remainders and the branches that a rule on sizes
 selects."""
+import os
+
 import numpy as np
 import pytest
 
+from conftest import GOLDEN
 from helpers import max_rel
 
 pytestmark = pytest.mark.gpu
@@ -61,3 +64,70 @@ def test_hydrostatic_levels(workdir, levels, hydz, columns):
     assert np.all(want["rad"] > 0)
     assert max_rel(got["rad"], want["rad"]) <= 1e-9
     assert max_rel(got["tau"], want["tau"]) <= 1e-9
+
+
+def _mixed_rays(n, seed=5):
+    from jscat import synth
+    rng = np.random.default_rng(seed)
+    a = synth.limb_geometry(rng.uniform(4.0, 70.0, n))
+    b = synth.nadir_geometry(rng.uniform(0.0, 75.0, n))
+    odd = np.arange(n) % 2 == 1
+    geom = {k: np.where(odd, b[k], a[k]) for k in a}
+    geom["obsz"][::7] = 30.0                       # observers inside the atmosphere
+    geom["vpz"][3::11] = 130.0                     # and rays that miss it
+    return geom
+
+
+@pytest.mark.parametrize("grid", ["even", "uneven", "descending", "doubled", "two"])
+@pytest.mark.parametrize("hydz", [0.0, -999.0])
+def test_march_against_two_pass_tracing(workdir, grid, hydz):
+    """The march over level records and its records of points against the
+    counting and storing passes that jsc_formod_batch_noalloc keeps: the same
+    operations, so the same bits, on profiles whose altitudes are evenly
+    spaced, uneven, descending, doubled, or only two."""
+    from jscat import api, synth, structs as S
+    z = {"even": np.arange(0.0, 121.0), "uneven": 120.0 * np.linspace(0, 1, 90) ** 1.7,
+         "descending": np.arange(120.0, -1.0, -1.0), "two": np.array([0.0, 120.0]),
+         "doubled": np.sort(np.concatenate([np.arange(0.0, 121.0, 2.0), [14.0, 50.0]]))}[grid]
+    kw, atm, _ = _limb_inputs(workdir, z)
+    ctl = S.make_ctl(hydz=hydz, **kw)
+    geom = _mixed_rays(97)
+    inp = synth.batch_from([atm, dict(atm, t=atm["t"] + 3.0)], np.arange(97) % 2, geom)
+    m = api.Model(ctl)
+    got, want = api.formod_batch(ctl, inp, model=m), api.formod_batch_noalloc(ctl, inp, m)
+    for k in ("nlos", "rad", "tau", "tpz", "tplon", "tplat"):
+        np.testing.assert_array_equal(got[k], want[k])
+
+
+@pytest.mark.parametrize("refine", [False, True])
+def test_march_lanes_and_pool(workdir, refine):
+    """A thread per ray (above 16384 rays) and eight lanes per ray give the
+    same bits, and so does a pool that starts too small and grows."""
+    from jscat import api, synth, structs as S
+    kw, atm, _ = _limb_inputs(workdir, np.arange(0.0, 121.0))
+    aero = None
+    if refine:
+        aero = S.AeroT.from_buffer_copy(np.load(os.path.join(GOLDEN, "aero_ice8.npz"))["aero"].tobytes())
+        kw.update(sca_n=1, sca_mult=0)
+    ctl = S.make_ctl(hydz=0.0, **kw)
+    n = 16385
+    geom = _mixed_rays(n)
+    m = api.Model(ctl)
+    inp = synth.batch_from([atm], np.zeros(n, np.int32), geom)
+    many = api.formod_batch(ctl, inp, model=m, aero=aero)
+    for k in (1, 15, 17):
+        part = synth.batch_from([atm], np.zeros(k, np.int32), {c: v[n - k:] for c, v in geom.items()})
+        few = api.formod_batch(ctl, part, model=m, aero=aero)
+        for c in few:
+            np.testing.assert_array_equal(few[c], many[c][n - k:])
+        b = api.Batch(m, ctl, 1, len(inp["z"]), k, max_seg=600 if refine else 1)
+        try:
+            if aero is not None:
+                b.set_aero(aero)
+            b.upload(part)
+            b.run()
+            few = b.download()
+        finally:
+            b.close()
+        for c in few:
+            np.testing.assert_array_equal(few[c], many[c][n - k:])
