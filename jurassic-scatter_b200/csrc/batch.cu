@@ -94,6 +94,7 @@ extern "C" void jsc_batch_destroy(jsc_batch *b) {
   cudaFree(b->d_aero);
   cudaFree(b->d_beta);
   cudaFree(b->d_phase);
+  cudaFree(b->d_wt);
   cudaFree(b->d_nlos_b);
   cudaFree(b->d_los_off_b);
   cudaFree(b->d_geo_b);
@@ -370,11 +371,13 @@ extern "C" int jsc_batch_set_aero(jsc_batch *b, const aero_t *aero) {
   cudaFree(b->d_aero);
   cudaFree(b->d_beta);
   cudaFree(b->d_phase);
+  cudaFree(b->d_wt);
   b->d_aero = nullptr;
-  b->d_beta = b->d_phase = nullptr;
+  b->d_beta = b->d_phase = b->d_wt = nullptr;
   int st = jsc_dmalloc(&b->d_aero, nh);
   if (!st) st = jsc_dmalloc(&b->d_beta, (size_t)3 * (nl > 0 ? nl : 1) * nd);
   if (!st) st = jsc_dmalloc(&b->d_phase, (size_t)(nl > 0 ? nl : 1) * nd * NTHETA);
+  if (!st) st = jsc_dmalloc(&b->d_wt, (size_t)(nl > 0 ? nl : 1) * nd * (JSC_NTH_SCA + 1));
   if (!st && cudaMemcpy(b->d_aero, h, nh * sizeof(double), cudaMemcpyHostToDevice) != cudaSuccess) st = JSC_ERR_CUDA;
   if (!st && cudaMemcpy(b->d_beta, beta, (size_t)3 * (nl > 0 ? nl : 1) * nd * sizeof(double),
                         cudaMemcpyHostToDevice) != cudaSuccess) st = JSC_ERR_CUDA;
@@ -932,6 +935,18 @@ static int sun_sources(jsc_batch *b, const double *sp, const int *sp_atm, int n,
 // Scattering points per chunk of the 3-D source (32,400 pencils each).
 static const int64_t kScatterChunk3 = 16;
 
+// Polar weights of the layers' phase functions for the source integrals.
+static int polar_weights(jsc_batch *b, cudaStream_t s) {
+  const int nd = b->cfg.nd;
+  JSC_CUDA_TRY(cudaFuncSetAttribute(sp_integral_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    JSC_INT1_SHMEM));
+  if (b->aero_nl < 1) return JSC_OK;
+  sp_weights_kernel<<<dim3(nd, b->aero_nl), JSC_INT1_THREADS, 0, s>>>(
+      nd, b->d_phase, b->d_wt, b->d_wt + (size_t)b->aero_nl * JSC_NTH_SCA * nd);
+  JSC_LAUNCH_CHECK();
+  return JSC_OK;
+}
+
 static int plain_sources(jsc_batch *b, const double *sp, const int *sp_atm, int64_t n_pts,
                          double *src, cudaStream_t s) {
   int st = JSC_OK;
@@ -960,14 +975,7 @@ static int plain_sources(jsc_batch *b, const double *sp, const int *sp_atm, int6
   if ((st = copy_profiles(b, b->child, s))) return st;
   if ((st = copy_profiles(b, b->sun_child, s))) return st;
 
-  jsc_batch *c = b->child, *sc = b->sun_child;
-  const size_t shmem = ((size_t)JSC_NTH_SCA * nd + (size_t)na * (nd | 1) + 4 * JSC_NTH_SCA +
-                        (JSC_INT_THREADS / 32) * JSC_INT_CH + (size_t)na * (JSC_INT_CH + 1) +
-                        (size_t)na) *
-                       sizeof(double);
-  if (shmem > 48 * 1024)
-    JSC_CUDA_TRY(cudaFuncSetAttribute(sp_integral_kernel,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shmem));
+  jsc_batch *c = b->child;
   for (int64_t c0 = 0; c0 < n_pts && three_d; c0 += chunk) {
     const int n = (int)((n_pts - c0) < chunk ? (n_pts - c0) : chunk);
     // Pencils in every direction around the line of sight (src/scatter.c:835-856).
@@ -994,6 +1002,7 @@ static int plain_sources(jsc_batch *b, const double *sp, const int *sp_atm, int6
     JSC_LAUNCH_CHECK();
     if ((st = sun_sources(b, pa.sp, pa.sp_atm, n, src + c0 * nd, s))) return st;
   }
+  if (!three_d && (st = polar_weights(b, s))) return st;
   for (int64_t c0 = 0; c0 < n_pts && !three_d; c0 += chunk) {
     const int n = (int)((n_pts - c0) < chunk ? (n_pts - c0) : chunk);
     // Secondary pencils (src/scatter.c:717-736).
@@ -1020,13 +1029,13 @@ static int plain_sources(jsc_batch *b, const double *sp, const int *sp_atm, int6
     ia.n_total = nullptr;
     ia.first = c0;
     ia.nd = nd;
-    ia.nl = b->aero_nl;
     ia.sp = pa.sp;
     memcpy(ia.alpha, b->alpha, sizeof(ia.alpha));
     ia.rad = c->d_rad;
-    ia.phase = b->d_phase;
+    ia.wt = b->d_wt;
+    ia.wsum = b->d_wt + (size_t)b->aero_nl * JSC_NTH_SCA * nd;
     ia.src = src + c0 * nd;
-    sp_integral_kernel<<<n, JSC_INT_THREADS, shmem, s>>>(ia);
+    sp_integral_kernel<<<n, JSC_INT1_THREADS, JSC_INT1_SHMEM, s>>>(ia);
     JSC_LAUNCH_CHECK();
     if ((st = sun_sources(b, pa.sp, pa.sp_atm, n, src + c0 * nd, s))) return st;
   }
@@ -1070,13 +1079,10 @@ static int fixed_sources(jsc_batch *b, cudaStream_t s) {
   JSC_LAUNCH_CHECK();
   if ((st = copy_profiles(b, b->child, s))) return st;
   if ((st = copy_profiles(b, b->sun_child, s))) return st;
+  if ((st = polar_weights(b, s))) return st;
   const int64_t *n_total = reinterpret_cast<const int64_t *>(b->d_sp_listed);
   const int chunk = (int)b->fx_chunk;
   jsc_batch *c = b->child;
-  const size_t shmem = ((size_t)JSC_NTH_SCA * nd + (size_t)na * (nd | 1) + 4 * JSC_NTH_SCA +
-                        (JSC_INT_THREADS / 32) * JSC_INT_CH + (size_t)na * (JSC_INT_CH + 1) +
-                        (size_t)na) *
-                       sizeof(double);
   for (int r = 0; r < b->fx_rounds; r++) {
     const int64_t c0 = (int64_t)r * chunk;
     SpawnArgs pa;
@@ -1104,13 +1110,13 @@ static int fixed_sources(jsc_batch *b, cudaStream_t s) {
     ia.n_total = n_total;
     ia.first = c0;
     ia.nd = nd;
-    ia.nl = b->aero_nl;
     ia.sp = pa.sp;
     memcpy(ia.alpha, b->alpha, sizeof(ia.alpha));
     ia.rad = c->d_rad;
-    ia.phase = b->d_phase;
+    ia.wt = b->d_wt;
+    ia.wsum = b->d_wt + (size_t)b->aero_nl * JSC_NTH_SCA * nd;
     ia.src = b->d_src + c0 * nd;
-    sp_integral_kernel<<<chunk, JSC_INT_THREADS, shmem, s>>>(ia);
+    sp_integral_kernel<<<chunk, JSC_INT1_THREADS, JSC_INT1_SHMEM, s>>>(ia);
     JSC_LAUNCH_CHECK();
     if ((st = sun_sources(b, pa.sp, pa.sp_atm, chunk, b->d_src + c0 * nd, s, n_total, c0)))
       return st;
@@ -1169,13 +1175,6 @@ static int prepare_fixed_scattering(jsc_batch *b) {
     if ((st = jsc_dmalloc(&b->d_theta2, (size_t)b->sun_child->max_rays))) return st;
     b->n_theta2 = b->sun_child->max_rays;
   }
-  const size_t shmem = ((size_t)JSC_NTH_SCA * nd + (size_t)na * (nd | 1) + 4 * JSC_NTH_SCA +
-                        (JSC_INT_THREADS / 32) * JSC_INT_CH + (size_t)na * (JSC_INT_CH + 1) +
-                        (size_t)na) *
-                       sizeof(double);
-  if (shmem > 48 * 1024)
-    JSC_CUDA_TRY(cudaFuncSetAttribute(sp_integral_kernel,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)shmem));
   return JSC_OK;
 }
 

@@ -103,6 +103,7 @@ struct jsc_batch {
   double *d_aero;           // top[NLMAX] bottom[NLMAX] trans[NLMAX] alti[...]
   double *d_beta;           // beta_e, beta_s, beta_a: [3][nl][nd]
   double *d_phase;          // [nl][nd][NTHETA]
+  double *d_wt;             // polar weights [nl][180][nd] and their sums [nl][nd]
   int *d_nlos_b;            // LOS points before the refinement
   int64_t *d_los_off_b;     // (IP 2/3, as the records before it)
   double *d_geo_b, *d_pts_b;

@@ -7,7 +7,8 @@
 //                       direction, layer, observation time, profile
 //   sp_spawn_kernel     the secondary pencils of a chunk of points, written
 //                       as the rays of a child batch (src/scatter.c:698-735)
-//   sp_integral_kernel  phase-function weighted integral of the secondary
+//   sp_weights_kernel, sp_integral_kernel
+//                       phase-function weighted integral of the secondary
 //                       radiances over 180 x 180 directions (:737-800)
 //   sun_kernel          solar direction search by repeated ray tracing and
 //                       the solar pencil of each point (:899-995)
@@ -212,60 +213,23 @@ static __global__ void sp_spawn_kernel(SpawnArgs A) {
 
 // --------------------------------------------------------- source integral --
 
-struct IntegralArgs {
-  int n_pts, nalpha, nd, nl;
-  const int64_t *n_total;   // device count of the whole list (null: all real)
-  int64_t first;
-  const double *sp;          // first record of the chunk
-  double alpha[JSC_NALPHA_MAX];
-  const double *rad;         // [n_pts * nalpha][nd] secondary radiances
-  const double *phase;       // [nl][nd][NTHETA]
-  double *src;               // [n_pts][nd] of the chunk
-};
+#define JSC_INT_THREADS 256    // sp_integral3_kernel
+#define JSC_INT_CH 16          // channels per pass over the directions
+#define JSC_INT1_THREADS 192   // sp_integral_kernel: a thread per polar step, 12 groups of 16
+#define JSC_INT1_SL 29         // odd row stride of the interval sums (28 pencils, 27 intervals)
+static_assert(JSC_INT1_THREADS >= JSC_NTH_SCA && JSC_INT1_THREADS % JSC_INT_CH == 0, "block shape");
+static_assert(JSC_INT1_SL >= JSC_NALPHA_REF, "interval sums");
 
-#define JSC_INT_THREADS 256
-#define JSC_INT_CH 16  // channels per pass over the directions
-
-// One block per scattering point.  Directions (itheta, iphi) are spread
-// over the threads; the polar factor sin(theta2) * phase(theta2) of each
-// (itheta, channel), the secondary radiances, their slopes and the pencil
-// angles sit in shared memory.  The radiance and slope rows have odd
-// strides in doubles, so lanes whose directions fall in different alpha
-// intervals read different banks.  Weighted sums follow
-// src/scatter.c:737-805 up to the order of the sum.
-static __global__ void __launch_bounds__(JSC_INT_THREADS)
-sp_integral_kernel(IntegralArgs A) {
-  extern __shared__ double sh[];
-  const int k = blockIdx.x;
-  if (k >= live_points(A.n_total, A.first, A.n_pts)) return;
-  const int nd = A.nd, na = A.nalpha;
-  const int ndp = nd | 1, SL = JSC_INT_CH + 1;      // odd row strides
-  double *wt = sh;                                   // [JSC_NTH_SCA][nd]
-  double *rd = wt + (size_t)JSC_NTH_SCA * nd;        // [na][ndp]
-  double *trig = rd + (size_t)na * ndp;              // sin/cos of theta2 and phi
-  double *red = trig + 4 * JSC_NTH_SCA;              // [JSC_INT_THREADS / 32][JSC_INT_CH]
-  double *slp = red + (JSC_INT_THREADS / 32) * JSC_INT_CH;  // [na - 1][SL]
-  double *alf = slp + (size_t)na * SL;               // [na] pencil angles
-  const double *o = A.sp + (size_t)k * JSC_SP_REC;
-  const int il = (int)o[SP_IL];
-  for (int i = threadIdx.x; i < JSC_NTH_SCA; i += blockDim.x) {
-    const double th = (0.5 + i) * M_PI / 180.;
-    const double ph = 2. * (0.5 + i) * M_PI / 180.;
-    trig[i] = sin(th);
-    trig[JSC_NTH_SCA + i] = cos(th);
-    trig[2 * JSC_NTH_SCA + i] = sin(ph);
-    trig[3 * JSC_NTH_SCA + i] = cos(ph);
-  }
-  for (int i = threadIdx.x; i < na * nd; i += blockDim.x) {
-    const int ir = i / nd, id = i - ir * nd;
-    rd[(size_t)ir * ndp + id] = A.rad[((size_t)k * na + ir) * nd + id];
-  }
-  for (int i = threadIdx.x; i < na; i += blockDim.x) alf[i] = A.alpha[i];
-  __syncthreads();
-  // Polar weight sin(theta2) * phase(theta2); phase on the 1-degree grid.
-  const double *ph = A.phase + (size_t)il * nd * NTHETA;
-  for (int i = threadIdx.x; i < JSC_NTH_SCA * nd; i += blockDim.x) {
-    const int it = i / nd, id = i - it * nd;
+// Polar weights sin(theta2) phase(theta2) of layer blockIdx.y and channel
+// blockIdx.x on the 180 polar steps (phase interpolated on its 1-degree
+// grid), wt[nl][180][nd], and their sum over all directions, wsum[nl][nd]
+// (src/scatter.c:760-800).
+static __global__ void __launch_bounds__(JSC_INT1_THREADS)
+sp_weights_kernel(int nd, const double *phase, double *wt, double *wsum) {
+  __shared__ double sh[JSC_NTH_SCA];
+  const int id = blockIdx.x, il = blockIdx.y, it = threadIdx.x;
+  const double *ph = phase + ((size_t)il * nd + id) * NTHETA;
+  if (it < JSC_NTH_SCA) {
     const double th = (0.5 + it) * M_PI / 180.;
     // locate(theta, NTHETA, theta2) on theta[i] = i * pi / 180
     int j = 0, hi = NTHETA - 1;
@@ -274,71 +238,145 @@ sp_integral_kernel(IntegralArgs A) {
       if ((double)mid * M_PI / 180. > th) hi = mid; else j = mid;
     }
     const double a0 = (double)j * M_PI / 180., a1 = (double)(j + 1) * M_PI / 180.;
-    const double phase2 = jsc_lin(a0, ph[(size_t)id * NTHETA + j], a1, ph[(size_t)id * NTHETA + j + 1], th);
-    wt[i] = trig[it] * phase2;
+    const double w = sin(th) * jsc_lin(a0, ph[j], a1, ph[j + 1], th);
+    sh[it] = w;
+    wt[((size_t)il * JSC_NTH_SCA + it) * nd + id] = w;
   }
   __syncthreads();
-
-  double x[3], dx[3], lx[3], ly[3], lz[3], sx[3], sy[3], sz[3], mlz[3];
-  for (int i = 0; i < 3; i++) {
-    x[i] = o[SP_X + i];
-    dx[i] = o[SP_DX + i];
+  if (it == 0) {
+    double s = 0;
+    for (int i = 0; i < JSC_NTH_SCA; i++) s += sh[i];
+    wsum[(size_t)il * nd + id] = s * JSC_NPHI_SCA;
   }
-  local_frame(x, lx, ly, lz);
-  jsc_bascoord(dx, x, sx, sy, sz);
-  for (int i = 0; i < 3; i++) mlz[i] = -1. * lz[i];
-  const int ndir = JSC_NTH_SCA * JSC_NPHI_SCA;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (int c0 = 0; c0 < nd; c0 += JSC_INT_CH) {
-    // slopes (r1 - r0) / (a1 - a0) of the pass's channels per alpha
-    // interval, the quotient jsc_lin evaluates first
-    for (int i = threadIdx.x; i < (na - 1) * JSC_INT_CH; i += blockDim.x) {
-      const int lo = i / JSC_INT_CH, c = i - lo * JSC_INT_CH;
-      if (c0 + c < nd)
-        slp[lo * SL + c] = (rd[(size_t)(lo + 1) * ndp + c0 + c] - rd[(size_t)lo * ndp + c0 + c]) /
-                           (alf[lo + 1] - alf[lo]);
-    }
-    __syncthreads();
-    double acc[JSC_INT_CH];
-#pragma unroll
-    for (int c = 0; c < JSC_INT_CH; c++) acc[c] = 0;
-    for (int dir = threadIdx.x; dir < ndir; dir += blockDim.x) {
-      const int it = dir / JSC_NPHI_SCA, iq = dir - it * JSC_NPHI_SCA;
-      const double st = trig[it], ct = trig[JSC_NTH_SCA + it];
-      const double sp = trig[2 * JSC_NTH_SCA + iq], cp = trig[3 * JSC_NTH_SCA + iq];
-      double ek[3];
-      for (int i = 0; i < 3; i++) ek[i] = st * sp * sx[i] + st * cp * sy[i] + ct * sz[i];
-      const double alpha2 = jsc_angle(mlz, ek);
-      // locate(alpha, nalpha, alpha2): alpha increases from 0 to pi
-      int lo = 0, hi = na - 1;
-      while (hi > lo + 1) {
-        const int mid = (hi + lo) >> 1;
-        if (alf[mid] > alpha2) hi = mid; else lo = mid;
+}
+
+struct IntegralArgs {
+  int n_pts, nalpha, nd;
+  const int64_t *n_total;   // device count of the whole list (null: all real)
+  int64_t first;
+  const double *sp;          // first record of the chunk
+  double alpha[JSC_NALPHA_MAX];
+  const double *rad;         // [n_pts * nalpha][nd] secondary radiances
+  const double *wt, *wsum;   // polar weights (sp_weights_kernel)
+  double *src;               // [n_pts][nd] of the chunk
+};
+
+// Source integral of one scattering point per block (src/scatter.c:737-805).
+// The secondary radiance of a direction is linear in its angle alpha to the
+// zenith between two pencils, and its weight depends on the polar step only.
+// So the sum over the azimuth of a polar step needs, per pencil interval,
+// the number of its directions and the sum of their alpha - alpha[lo]: a
+// thread per polar step walks the azimuth once for all channels and keeps
+// them (run sums in registers, added to shared memory when the interval
+// changes).  The channels then take 180 x 27 of these sums each instead of
+// 32,400 directions.  The zenith has no component across the plane of the
+// zenith and the line of sight, so alpha is even in the azimuth and half of
+// it suffices (all of it should the component exceed rounding).
+// Bound by the FP64 acos of 16,200 directions a point.  Evaluating every
+// channel in every direction took 9.0 ms for 11,600 points of 16 channels
+// and 61.8 ms for a depth-2 batch of 12 rays, this form 1.7 and 12.6.
+#define JSC_INT1_SHMEM (JSC_NTH_SCA * JSC_INT1_SL * 9)
+
+static __global__ void __launch_bounds__(JSC_INT1_THREADS, 4) sp_integral_kernel(IntegralArgs A) {
+  extern __shared__ double ss[];  // [180][JSC_INT1_SL] sums of alpha - alpha[lo]
+  unsigned char *sn =             // [180][JSC_INT1_SL] directions (at most 180)
+      reinterpret_cast<unsigned char *>(ss + JSC_NTH_SCA * JSC_INT1_SL);
+  __shared__ double rd[JSC_NALPHA_REF][JSC_INT_CH], slp[JSC_NALPHA_REF][JSC_INT_CH];
+  __shared__ double cph[JSC_NPHI_SCA], alf[JSC_NALPHA_MAX];
+  __shared__ double red[JSC_INT1_THREADS];
+  const int k = blockIdx.x;
+  if (k >= live_points(A.n_total, A.first, A.n_pts)) return;
+  const int nd = A.nd, na = A.nalpha, tid = threadIdx.x;
+  const double *o = A.sp + (size_t)k * JSC_SP_REC;
+  const int il = (int)o[SP_IL];
+  for (int i = tid; i < JSC_NPHI_SCA; i += JSC_INT1_THREADS)
+    cph[i] = cos(2. * (0.5 + i) * M_PI / 180.);
+  for (int i = tid; i < na; i += JSC_INT1_THREADS) alf[i] = A.alpha[i];
+  for (int i = tid; i < JSC_NTH_SCA * JSC_INT1_SL; i += JSC_INT1_THREADS) {
+    ss[i] = 0;
+    sn[i] = 0;
+  }
+  // components of the downward zenith (-lz) along the axes of the scattering frame
+  double ax, ay, az;
+  {
+    const double x[3] = {o[SP_X], o[SP_X + 1], o[SP_X + 2]};
+    const double dx[3] = {o[SP_DX], o[SP_DX + 1], o[SP_DX + 2]};
+    double lx[3], ly[3], lz[3], sx[3], sy[3], sz[3];
+    local_frame(x, lx, ly, lz);
+    jsc_bascoord(dx, x, sx, sy, sz);
+    ax = -(lz[0] * sx[0] + lz[1] * sx[1] + lz[2] * sx[2]);
+    ay = -(lz[0] * sy[0] + lz[1] * sy[1] + lz[2] * sy[2]);
+    az = -(lz[0] * sz[0] + lz[1] * sz[1] + lz[2] * sz[2]);
+  }
+  const bool even = fabs(ax) <= 1e-14;
+  __syncthreads();
+  if (tid < JSC_NTH_SCA) {
+    const double th = (0.5 + tid) * M_PI / 180.;
+    const double st = sin(th), ct = cos(th);
+    const double c1 = st * ay, c0 = ct * az, c2 = st * ax;
+    const int row = tid * JSC_INT1_SL, m = even ? JSC_NPHI_SCA / 2 : JSC_NPHI_SCA;
+    int lo = 0, n = 0;
+    double s = 0;
+    for (int iq = 0; iq < m; iq++) {
+      double c = c1 * cph[iq] + c0;
+      if (!even) c += c2 * sin(2. * (0.5 + iq) * M_PI / 180.);
+      const double alpha2 = acos(fmin(fmax(c, -1.0), 1.0));
+      // locate(alpha, nalpha, alpha2) from the interval before
+      int l = lo;
+      while (l < na - 2 && !(alf[l + 1] > alpha2)) l++;
+      while (l > 0 && alf[l] > alpha2) l--;
+      if (l != lo) {
+        ss[row + lo] += s;
+        sn[row + lo] += (unsigned char)n;
+        s = 0;
+        n = 0;
+        lo = l;
       }
-      const double da = alpha2 - alf[lo];
-      const double *w = wt + (size_t)it * nd + c0;
-      const double *r0 = rd + (size_t)lo * ndp + c0, *s0 = slp + lo * SL;
-#pragma unroll
-      for (int c = 0; c < JSC_INT_CH; c++)
-        if (c0 + c < nd) acc[c] += w[c] * (r0[c] + s0[c] * da);  // jsc_lin, slope precomputed
+      s += alpha2 - alf[l];
+      n++;
     }
-    // block reduction per channel
-#pragma unroll
-    for (int c = 0; c < JSC_INT_CH; c++) {
-      double v = acc[c];
-      for (int off = 16; off > 0; off >>= 1) v += __shfl_down_sync(0xffffffffu, v, off);
-      if (lane == 0) red[warp * JSC_INT_CH + c] = v;
+    ss[row + lo] += s;
+    sn[row + lo] += (unsigned char)n;
+  }
+  const int c = tid & (JSC_INT_CH - 1), grp = tid / JSC_INT_CH;
+  constexpr int NG = JSC_INT1_THREADS / JSC_INT_CH, PER = JSC_NTH_SCA / NG;
+  static_assert(PER * NG == JSC_NTH_SCA, "polar steps per group");
+  for (int ch0 = 0; ch0 < nd; ch0 += JSC_INT_CH) {
+    __syncthreads();
+    for (int i = tid; i < na * JSC_INT_CH; i += JSC_INT1_THREADS) {
+      const int lo = i / JSC_INT_CH, cc = i - lo * JSC_INT_CH;
+      if (ch0 + cc < nd) {
+        const double *r = A.rad + ((size_t)k * na + lo) * nd + ch0 + cc;
+        rd[lo][cc] = r[0];
+        if (lo + 1 < na) slp[lo][cc] = (r[nd] - r[0]) / (alf[lo + 1] - alf[lo]);
+      }
     }
     __syncthreads();
-    if (threadIdx.x < JSC_INT_CH && c0 + threadIdx.x < nd) {
-      const int id = c0 + threadIdx.x;
-      double s = 0, wsum = 0;
-      for (int w = 0; w < (int)(blockDim.x >> 5); w++) s += red[w * JSC_INT_CH + threadIdx.x];
-      for (int it = 0; it < JSC_NTH_SCA; it++) wsum += wt[(size_t)it * nd + id];
-      wsum *= JSC_NPHI_SCA;
-      A.src[(size_t)k * nd + id] = s / wsum;
+    double acc = 0;
+    const int id = ch0 + c;
+    if (id < nd) {
+      double v[PER];  // polar steps grp, grp + NG, ... of this channel
+#pragma unroll
+      for (int j = 0; j < PER; j++) v[j] = 0;
+      for (int lo = 0; lo < na - 1; lo++) {
+        const double r0 = rd[lo][c], s0 = slp[lo][c];
+#pragma unroll
+        for (int j = 0; j < PER; j++) {
+          const int q = (grp + j * NG) * JSC_INT1_SL + lo;
+          v[j] += (double)sn[q] * r0 + ss[q] * s0;
+        }
+      }
+      const double *w = A.wt + ((size_t)il * JSC_NTH_SCA + grp) * nd + id;
+#pragma unroll
+      for (int j = 0; j < PER; j++) acc += w[(size_t)j * NG * nd] * v[j];
     }
+    red[tid] = acc;
     __syncthreads();
+    if (tid < JSC_INT_CH && id < nd) {
+      double t = 0;
+      for (int g = 0; g < NG; g++) t += red[g * JSC_INT_CH + c];
+      A.src[(size_t)k * nd + id] = (even ? 2 * t : t) / A.wsum[(size_t)il * nd + id];
+    }
   }
 }
 

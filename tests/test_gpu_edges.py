@@ -131,3 +131,31 @@ def test_march_lanes_and_pool(workdir, refine):
             b.close()
         for c in few:
             np.testing.assert_array_equal(few[c], many[c][n - k:])
+
+
+@pytest.mark.parametrize("nd,nalpha,layer", [(1, 10, "aero_sulfate16"), (16, 28, "aero_sulfate16"), (8, 20, "aero_ice8")])
+def test_source_integral_against_port(workdir, nd, nalpha, layer):
+    """Single-scattering radiances (source integral over pencil intervals)
+    against the C restatement, which evaluates every direction: channel
+    counts of one, part of and a whole channel pass, the fewest and the most
+    pencils, a limb and an oblique ray and one that looks straight down,
+    where the scattering frame is degenerate.  1e-9, the parity bound."""
+    from jscat import api, synth, structs as S
+    from oracle import refrun
+    g = np.load(os.path.join(GOLDEN, layer + ".npz"))
+    full = S.AeroT.from_buffer_copy(g["aero"].tobytes())
+    kw, atm, _ = _limb_inputs(workdir, np.arange(0.0, 121.0))
+    nus = [float(v) for v in g["nus"]][:nd]
+    kw.update(nus=nus, tblbase=synth.write_tables(workdir, kw["emitters"], [float(v) for v in g["nus"]], 20261203),
+              sca_n=1, sca_mult=1, hydz=0.0, ctm_co2=0, ctm_h2o=0)
+    geom = {k: np.concatenate([a, b]) for (k, a), b in zip(
+        synth.limb_geometry([17.3 if "sulfate" in layer else 9.7]).items(),
+        synth.nadir_geometry([0.0, 41.0]).values())}
+    geom["time"] = np.array([3600.0, 40000.0, 43200.0])
+    inp = synth.batch_from([atm], np.zeros(3, np.int32), geom)
+    got = api.formod_batch(S.make_ctl(**kw), inp, aero=full, nalpha=nalpha)
+    ref = refrun.run_port(kw, [atm], np.zeros(3, int), geom, aero=bytes(full), threads=os.cpu_count(),
+                          nalpha=nalpha, timeout=900)
+    assert np.all(np.isfinite(ref["rad"])) and np.all(ref["rad"] > 0)
+    assert max_rel(got["rad"], ref["rad"]) <= 1e-9
+    assert max_rel(got["tau"], ref["tau"]) <= 1e-9
