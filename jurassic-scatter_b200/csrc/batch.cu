@@ -15,42 +15,50 @@
 static int sca_alpha(double *alpha, int nalpha);
 static int map_status(unsigned st);
 
-static void batch_free_los(jsc_batch *b) {
+// LOS geometry and records of max_seg points.
+static int batch_alloc_los(jsc_batch *b, int64_t max_seg) {
   cudaFree(b->d_geo);
   cudaFree(b->d_pts);
-  cudaFree(b->d_ctm);
-  cudaFree(b->d_srcp);
-  b->d_geo = b->d_pts = b->d_ctm = b->d_srcp = nullptr;
-}
-
-static int batch_alloc_los(jsc_batch *b, int64_t max_seg) {
-  batch_free_los(b);
+  b->d_geo = b->d_pts = nullptr;
   int st;
   if ((st = jsc_dmalloc(&b->d_geo, (size_t)max_seg * 4))) return st;
   if ((st = jsc_dmalloc(&b->d_pts, (size_t)max_seg * b->W))) return st;
-  if ((st = jsc_dmalloc(&b->d_ctm, (size_t)max_seg * b->cfg.nd))) return st;
-  if ((st = jsc_dmalloc(&b->d_srcp, (size_t)max_seg * b->cfg.nd))) return st;
   b->max_seg = max_seg;
   return JSC_OK;
 }
 
-// Room in the march pool for n_seg LOS points of max_rays rays: every ray's
-// first chunk, and the chunks that full ones are followed by.
-static int batch_alloc_pool(jsc_batch *b, int64_t n_seg) {
-  cudaFree(b->d_mpts);
-  cudaFree(b->d_mnext);
+// Continuum extinction and Planck source of max_seg points.  Until the LOS
+// records are written the first of them holds the pool of the ray march
+// (IP 1): chunks of 32 points for pool_seg points, every ray's first chunk
+// among them.
+static int batch_alloc_ctm(jsc_batch *b, int64_t pool_seg) {
+  cudaFree(b->d_ctm);
+  cudaFree(b->d_srcp);
+  b->d_ctm = b->d_srcp = nullptr;
   b->d_mpts = nullptr;
   b->d_mnext = nullptr;
   b->mcap = 0;
-  const int64_t cap = (int64_t)b->max_rays + n_seg / JSC_CHUNK + 1;
-  if (cap > INT_MAX) {
-    jsc_set_error(JSC_ERR_NOMEM, "%lld LOS points exceed the march pool", (long long)n_seg);
-    return JSC_ERR_NOMEM;
+  const size_t chunk = JSC_CHUNK * JSC_CHUNK_REC * sizeof(double);
+  size_t n = (size_t)b->max_seg * b->cfg.nd;
+  if (b->ip == 1) {
+    const int64_t cap = (int64_t)b->max_rays + pool_seg / JSC_CHUNK + 1;
+    if (cap > INT_MAX) {
+      jsc_set_error(JSC_ERR_NOMEM, "%lld LOS points exceed the march pool", (long long)pool_seg);
+      return JSC_ERR_NOMEM;
+    }
+    const size_t need = ((size_t)cap * (chunk + sizeof(int)) + sizeof(double) - 1) / sizeof(double);
+    if (n < need) n = need;
   }
   int st;
-  if ((st = jsc_dmalloc(&b->d_mpts, (size_t)cap * JSC_CHUNK * JSC_CHUNK_REC))) return st;
-  if ((st = jsc_dmalloc(&b->d_mnext, (size_t)cap))) return st;
-  b->mcap = (int)cap;
+  if ((st = jsc_dmalloc(&b->d_ctm, n))) return st;
+  if ((st = jsc_dmalloc(&b->d_srcp, (size_t)b->max_seg * b->cfg.nd))) return st;
+  if (b->ip == 1) {
+    const size_t cap = n * sizeof(double) / (chunk + sizeof(int));
+    b->mcap = cap < INT_MAX ? (int)cap : INT_MAX;
+    b->d_mpts = b->d_ctm;
+    b->d_mnext = (int *)((char *)b->d_ctm + (size_t)b->mcap * chunk);
+  }
+  b->ctm_seg = b->max_seg;
   return JSC_OK;
 }
 
@@ -69,14 +77,16 @@ extern "C" void jsc_batch_destroy(jsc_batch *b) {
   cudaFree(b->d_zmin);
   cudaFree(b->d_zmax);
   cudaFree(b->d_lev);
-  cudaFree(b->d_mpts);
-  cudaFree(b->d_mnext);
+  cudaFree(b->d_qs);
   cudaFree(b->d_mcount);
   cudaFree(b->d_ray_atm);
   cudaFree(b->d_ray);
   cudaFree(b->d_nlos);
   cudaFree(b->d_los_off);
-  batch_free_los(b);
+  cudaFree(b->d_geo);
+  cudaFree(b->d_pts);
+  cudaFree(b->d_ctm);
+  cudaFree(b->d_srcp);
   cudaFree(b->d_tsurf);
   cudaFree(b->d_tp);
   cudaFree(b->d_rkeys);
@@ -206,10 +216,11 @@ extern "C" int jsc_batch_create(jsc_model *m, const ctl_t *ctl, int max_atm,
   st = st ? st : jsc_dmalloc(&b->d_status, 1);
   st = st ? st : jsc_dmalloc(&b->d_counters, 2);
   if (!st) st = batch_alloc_los(b, max_seg > 0 ? max_seg : (int64_t)max_rays * 512);
+  st = st ? st : batch_alloc_ctm(b, b->max_seg);
   if (b->ip == 1) {
     st = st ? st : jsc_dmalloc(&b->d_lev, 8 * (size_t)max_levels);
+    st = st ? st : jsc_dmalloc(&b->d_qs, (size_t)(ctl->ng + ctl->nw) * max_levels);
     st = st ? st : jsc_dmalloc(&b->d_mcount, 1);
-    st = st ? st : batch_alloc_pool(b, b->max_seg);
   }
   b->scan_tiles = (max_rays + JSC_SCAN_TILE - 1) / JSC_SCAN_TILE + 1;
   st = st ? st : jsc_dmalloc(&b->d_scan, (size_t)b->scan_tiles + 1);
@@ -1489,6 +1500,7 @@ static int run_hydro(jsc_batch *b, cudaStream_t s) {
   aa.zmin = b->d_zmin;
   aa.zmax = b->d_zmax;
   aa.lev = b->d_lev;
+  aa.qs = b->d_qs;
   aa.hydz = b->cfg.hydz;
   ev_record(b, JSC_T_HYDRO, 0, s);
   hydro_kernel<<<b->n_atm, JSC_HYDRO_THREADS, 0, s>>>(aa);
@@ -1526,6 +1538,7 @@ static int los_profile(jsc_batch *b, bool refine, cudaStream_t s) {
   xa.atm_off = b->d_atm_off;
   xa.z = b->d_z;
   xa.lev = b->d_lev;
+  xa.qs = b->d_qs;
   xa.q = b->d_q;
   xa.k = b->d_k;
   xa.nlos_b = ra.nlos;
@@ -1598,7 +1611,7 @@ static int los_profile(jsc_batch *b, bool refine, cudaStream_t s) {
                                    cudaMemcpyDeviceToHost, s));
       JSC_CUDA_TRY(cudaStreamSynchronize(s));
     }
-    if ((st = batch_alloc_pool(b, *b->h_total + *b->h_total / 4 + 1024))) return st;
+    if ((st = batch_alloc_ctm(b, *b->h_total + *b->h_total / 4 + 1024))) return st;
   }
   if (*b->h_total > b->max_seg) {
     if ((st = batch_alloc_los(b, *b->h_total + *b->h_total / 4 + 1024))) return st;
@@ -1610,6 +1623,10 @@ static int los_profile(jsc_batch *b, bool refine, cudaStream_t s) {
   if (refine) expand_kernel<true><<<g32, 128, 0, s>>>(xa);
   else expand_kernel<false><<<g32, 128, 0, s>>>(xa);
   JSC_LAUNCH_CHECK();
+  tangent_kernel<<<(unsigned)((nr + 127) / 128), 128, 0, s>>>(xa);
+  JSC_LAUNCH_CHECK();
+  // after the records: this takes the pool's memory
+  if (b->ctm_seg < b->max_seg && (st = batch_alloc_ctm(b, b->max_seg))) return st;
   return JSC_OK;
 }
 
@@ -1664,6 +1681,7 @@ static int los_geo(jsc_batch *b, bool refine, cudaStream_t s) {
   } else {
     if (*b->h_total > b->max_seg) {
       int st = batch_alloc_los(b, *b->h_total + *b->h_total / 4 + 1024);
+      if (!st) st = batch_alloc_ctm(b, 0);
       if (st) return st;
     }
     b->n_points = b->fixed ? b->max_seg : *b->h_total;
@@ -1734,6 +1752,7 @@ static int los_geo(jsc_batch *b, bool refine, cudaStream_t s) {
     }
     if (*b->h_total > b->max_seg) {
       int st = batch_alloc_los(b, *b->h_total + *b->h_total / 4 + 1024);
+      if (!st) st = batch_alloc_ctm(b, 0);
       if (st) return st;
     }
     b->n_points = b->fixed ? b->max_seg : *b->h_total;
@@ -2162,9 +2181,7 @@ extern "C" int jsc_batch_set_fixed(jsc_batch *b, int on) {
     if (b->ip != 1 && b->cfg.sca_n > 0 && b->max_seg_b < b->max_seg &&
         (st = batch_alloc_los_b(b, b->max_seg)))
       return st;
-    if (b->ip == 1 && (int64_t)b->mcap < (int64_t)b->max_rays + b->max_seg / JSC_CHUNK + 1 &&
-        (st = batch_alloc_pool(b, b->max_seg)))
-      return st;
+
     if (!b->h_status && cudaMallocHost((void **)&b->h_status, sizeof(unsigned)) != cudaSuccess) {
       jsc_set_error(JSC_ERR_NOMEM, "pinned host allocation");
       return JSC_ERR_NOMEM;

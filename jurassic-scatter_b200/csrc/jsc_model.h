@@ -90,6 +90,7 @@ struct jsc_batch {
   double *d_p;              // pressure after hydrostatic balance
   double *d_zmin, *d_zmax;  // per profile
   double *d_lev;            // [max_levels][8] level records of the ray march (IP 1)
+  double *d_qs;             // [ng + nw][n_levels] level slopes of VMRs and extinctions
   int ip;                   // atmosphere interpolation (1 profile, 2, 3)
   double cz, cx;            // IP 3 influence lengths [km]
   double *d_psurf;          // IP 2/3 surface positions [profiles or levels][3]
@@ -169,8 +170,8 @@ struct jsc_batch {
   jsc_batch_input gin;      // host inputs the graph copies from
   int graph_ready, graph_kernels;
 
-  // Pool of the ray march (IP 1): chunks of 32 points, the first max_rays of
-  // them one per ray (trace.cuh).
+  // Pool of the ray march (IP 1), chunks of 32 points (trace.cuh): the memory
+  // of d_ctm, which is written after the pool has been read.
   double *d_mpts;
   int *d_mnext;
   unsigned *d_mcount;
@@ -181,7 +182,8 @@ struct jsc_batch {
   int64_t *d_los_off;       // [max_rays+1]
   double *d_geo;            // [max_seg][4]: z lon lat raw-ds
   double *d_pts;            // [max_seg][W]: p t ds qh2o k[nw] u[ng]
-  double *d_ctm, *d_srcp;   // [max_seg][nd]: continuum extinction, Planck source
+  double *d_ctm, *d_srcp;   // [ctm_seg][nd]: continuum extinction, Planck source
+  int64_t ctm_seg;
   int64_t n_points;         // LOS points of the current run
   double *d_tsurf;          // [max_rays]
   double *d_tp;             // [3][max_rays]

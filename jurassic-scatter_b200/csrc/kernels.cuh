@@ -34,6 +34,7 @@ struct AtmArgs {
   const double *z, *lon, *lat, *p_in, *t, *q, *k;
   double *p, *zmin, *zmax;
   double *lev;  // [n_levels][8] level records of the ray march, or null
+  double *qs;   // [ng + nw][n_levels] slopes of the VMRs and extinctions (with lev)
   double hydz;
 };
 
@@ -143,6 +144,11 @@ static __global__ void __launch_bounds__(JSC_HYDRO_THREADS) hydro_kernel(AtmArgs
       r[5] = (t[l + 1] - t[l]) / (z[l + 1] - z[l]);
       r[6] = ex ? 1.0 : 0.0;
       r[7] = down ? 0.0 : 1.0;
+      for (int c = 0; c < a.ng + a.nw; c++) {
+        const double *v = (c < a.ng ? a.q + (size_t)c * a.n_levels
+                                    : a.k + (size_t)(c - a.ng) * a.n_levels) + lo + l;
+        a.qs[(size_t)c * a.n_levels + lo + l] = (v[1] - v[0]) / (z[l + 1] - z[l]);
+      }
     }
   }
   // gsl_stats_min/max: first element, then strict comparisons; NaN wins.

@@ -135,7 +135,7 @@ static int noalloc_run(jsc_model *m, const ctl_t *ctl, const jsc_batch_input *in
   aa.p = d_p;
   aa.zmin = d_zmin;
   aa.zmax = d_zmax;
-  aa.lev = nullptr;
+  aa.lev = aa.qs = nullptr;
   aa.hydz = ctl->hydz;
   hydro_kernel<<<na, JSC_HYDRO_THREADS, 0, s>>>(aa);
   JSC_LAUNCH_CHECK();

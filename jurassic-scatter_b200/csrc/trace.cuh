@@ -334,7 +334,7 @@ __device__ __forceinline__ double chunk_altitude(const double *rec) {
 struct ExpandArgs {
   int n_rays, ng, nw, W, n_levels, ig_h2o;
   const int *ray_atm, *atm_off;
-  const double *z, *lev, *q, *k;   // profiles
+  const double *z, *lev, *q, *k, *qs;  // profiles
   MarchPool M;
   const int *nlos_b;               // points of the march
   int *nlos;                       // points with the layer edges
@@ -379,28 +379,62 @@ static __global__ void __launch_bounds__(128) edge_count_kernel(ExpandArgs A) {
   A.nlos[r] = o;
 }
 
+// Geography to position and back as calls: they are used at several places
+// of the kernels below, whose instructions would not stay in the
+// instruction cache if each were inlined.
+struct Vec3 {
+  double v[3];
+};
+
+static __device__ __noinline__ Vec3 cart_of(double z, double lon, double lat) {
+  Vec3 x;
+  jsc_geo2cart(z, lon, lat, x.v);
+  return x;
+}
+
+static __device__ __noinline__ Vec3 geo_of(double x0, double x1, double x2) {
+  const double x[3] = {x0, x1, x2};
+  Vec3 g;
+  jsc_cart2geo(x, &g.v[0], &g.v[1], &g.v[2]);
+  return g;
+}
+
+// The point of segment_point.
+__device__ __forceinline__ Vec3 crossing_of(const double *g0, const double *g1, double z) {
+  const double frac = (g0[0] - z) / (g0[0] - g1[0]);
+  const Vec3 a = cart_of(g0[0], g0[1], g0[2]), b = cart_of(g1[0], g1[1], g1[2]);
+  double x[3];
+  for (int i = 0; i < 3; i++) x[i] = a.v[i] + frac * (b.v[i] - a.v[i]);
+  return geo_of(x[0], x[1], x[2]);
+}
+
 // Record of a LOS point: the state at its altitude z, the column densities
 // over its step ds (src/lineofsight.c:182-185), the table brackets, and the
-// layer factor (af, ai).
-__device__ __forceinline__ void write_record(const ExpandArgs &A, const Profile &a,
-                                             const double *lev, double *rec, double z, double ds,
-                                             double af, double ai) {
+// layer factor (af, ai).  The LIN quotients of a level are in qs.
+static __device__ __noinline__ void write_record(const ExpandArgs &A, int lo, int n, double *rec,
+                                                 double z, double ds, double af, double ai) {
+  const double *zl = A.z + lo, *lev = A.lev + 8 * (size_t)lo;
   // level guess for evenly spaced altitudes
-  const double zf = a.z[0];
-  int h = (int)fmin(fmax((z - zf) / (a.z[a.n - 1] - zf) * (a.n - 1), 0.0), (double)(a.n - 2));
+  const double zf = zl[0];
+  int h = (int)fmin(fmax((z - zf) / (zl[n - 1] - zf) * (n - 1), 0.0), (double)(n - 2));
   double p, t;
-  level_state(lev, a.z, a.n, z, h, &p, &t);
+  level_state(lev, zl, n, z, h, &p, &t);
+  const double dz = z - zl[h];
+  const size_t nl = (size_t)A.n_levels, l = (size_t)lo + h;
   rec[REC_P] = p;
   rec[REC_T] = t;
   rec[REC_DS] = ds;
-  rec[REC_QH2O] = A.ig_h2o >= 0 ? atm_lin(a.q + (size_t)A.ig_h2o * a.stride, a, h, z) : 0.0;
+  rec[REC_QH2O] = A.ig_h2o >= 0 ? A.q[A.ig_h2o * nl + l] + A.qs[A.ig_h2o * nl + l] * dz : 0.0;
   rec[REC_GRID] = A.grid_p ? (double)grid_code(A.grid_np, A.grid_p, A.grid_nt, A.grid_t, p, t) : -1.0;
   rec[REC_PLK] = (double)planck_index(t);
   rec[REC_AF] = af;
   rec[REC_AI] = ai;
-  for (int w = 0; w < A.nw; w++) rec[REC_K + w] = atm_lin(a.k + (size_t)w * a.stride, a, h, z);
+#pragma unroll 1
+  for (int w = 0; w < A.nw; w++)
+    rec[REC_K + w] = A.k[w * nl + l] + A.qs[(A.ng + w) * nl + l] * dz;
+#pragma unroll 1
   for (int g = 0; g < A.ng; g++) {
-    const double q = atm_lin(a.q + (size_t)g * a.stride, a, h, z);
+    const double q = A.q[g * nl + l] + A.qs[g * nl + l] * dz;
     rec[REC_K + A.nw + g] = 10 * q * p / (JSC_KBOLTZ * t) * ds;
   }
 }
@@ -440,16 +474,19 @@ __device__ inline double marched_point(const MarchPool &M, int r, int ip, double
     return 0;
   }
   const double *rec = M.pts + ((size_t)chunk * JSC_CHUNK + (ip & (JSC_CHUNK - 1))) * JSC_CHUNK_REC;
-  if (rec[3] == 0.)
-    for (int i = 0; i < 3; i++) g[i] = rec[i];
-  else
-    jsc_cart2geo(rec, &g[0], &g[1], &g[2]);
+  const Vec3 x = rec[3] == 0. ? Vec3{{rec[0], rec[1], rec[2]}} : geo_of(rec[0], rec[1], rec[2]);
+  for (int i = 0; i < 3; i++) g[i] = x.v[i];
   return rec[3];
 }
 
-// Tangent point of ray r with np marched points whose lowest is m
-// (src/lineofsight.c:411-452).
-__device__ inline void tangent_point(const ExpandArgs &A, int r, int np, int m) {
+// Tangent point of each ray, a thread per ray, from its marched points
+// (src/lineofsight.c:411-452); tp[r] holds the number of the lowest one.
+static __global__ void __launch_bounds__(128) tangent_kernel(ExpandArgs A) {
+  const int r = blockIdx.x * blockDim.x + threadIdx.x;
+  if (r >= A.n_rays) return;
+  const int np = A.nlos_b[r];
+  if (np == 0) return;
+  const int m = (int)A.tp[r];
   double g0[3], g1[3], g2[3], tp[3];
   if (m <= 0 || m >= np - 1) {
     marched_point(A.M, r, np - 1, tp);
@@ -463,39 +500,38 @@ __device__ inline void tangent_point(const ExpandArgs &A, int r, int np, int m) 
     const double bb = -(yy0 - yy1) / x1 - aa * x1;
     const double cc = yy0;
     const double xx = -bb / (2 * aa);
-    double v0[3], v2[3], v[3], dummy;
+    const Vec3 v0 = cart_of(g0[0], g0[1], g0[2]), v2 = cart_of(g2[0], g2[1], g2[2]);
+    double v[3];
+    for (int i = 0; i < 3; i++) v[i] = jsc_lin(0.0, v0.v[i], x2, v2.v[i], xx);
+    const Vec3 g = geo_of(v[0], v[1], v[2]);
     tp[0] = aa * xx * xx + bb * xx + cc;
-    jsc_geo2cart(g0[0], g0[1], g0[2], v0);
-    jsc_geo2cart(g2[0], g2[1], g2[2], v2);
-    for (int i = 0; i < 3; i++) v[i] = jsc_lin(0.0, v0[i], x2, v2[i], xx);
-    jsc_cart2geo(v, &dummy, &tp[1], &tp[2]);
+    tp[1] = g.v[1];
+    tp[2] = g.v[2];
   }
   for (int i = 0; i < 3; i++) A.tp[(size_t)i * A.n_rays + r] = tp[i];
 }
 
 // LOS records of a ray by one warp.  EDGES: the points where segments cross
-// layer edges go in between (add_aerosol_layers, src/lineofsight.c:193-372):
-// lanes take 32 marched points at a time, a warp scan of their output counts
-// (crossings of the segment before the point, then the point) places the
-// geometry, then lanes take 32 points at a time for the records, with the
-// neighbours' Cartesian positions passed by shuffles for the chord steps.
+// layer edges go in between (add_aerosol_layers, src/lineofsight.c:193-372).
+// Lanes take 32 marched points at a time; a warp scan of their output counts
+// (crossings of the segment before the point, then the point) numbers the
+// output points, and lanes then take output points, so that the crossings of
+// one segment (a dozen where it enters a layer with a transition zone) run in
+// parallel.  A second pass takes 32 output points at a time for the records,
+// with the neighbours' Cartesian positions passed by shuffles for the chord
+// steps.  Bound by instruction issue; with the crossings in the lane of
+// their segment, every function inlined and the tangent point in lane 0 the
+// warps waited for instructions (9.9 of 17 cycles an issue, 11.7 lanes
+// active), 9.6 ms for 232,000 pencils, now 3.2.
 template <bool EDGES>
-__global__ void __launch_bounds__(128, 6) expand_kernel(ExpandArgs A) {
+__global__ void __launch_bounds__(128, 6) expand_kernel(const __grid_constant__ ExpandArgs A) {
   const int r = (int)(((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
   const int lane = threadIdx.x & 31;
   const unsigned full = 0xffffffffu;
   if (r >= A.n_rays) return;  // whole warps leave together
   const int nb = A.nlos_b[r];
   if (nb == 0) return;
-  const int ai = A.ray_atm[r], lo = A.atm_off[ai];
-  Profile a;
-  a.n = A.atm_off[ai + 1] - lo;
-  a.stride = A.n_levels;
-  a.z = A.z + lo;
-  a.q = A.q + lo;
-  a.k = A.k + lo;
-  a.p = a.t = nullptr;
-  const double *lev = A.lev + 8 * (size_t)lo;
+  const int ai = A.ray_atm[r], lo = A.atm_off[ai], nlev = A.atm_off[ai + 1] - lo;
   const int64_t base = A.off[r];
   const int nmax = EDGES ? A.nlos[r] : nb;
   // lowest marched point: the first NaN, else the first smallest altitude
@@ -505,20 +541,20 @@ __global__ void __launch_bounds__(128, 6) expand_kernel(ExpandArgs A) {
   int chunk = r, o = 0;
   for (int c0 = 0; c0 < nb; c0 += JSC_CHUNK) {
     if (chunk < 0) {  // the march ran out of chunks
-      if (lane == 0) atomicOr(A.status, JSC_DEV_ERR_NLOS);
+      if (lane == 0) {
+        atomicOr(A.status, JSC_DEV_ERR_NLOS);
+        A.tp[r] = 0;
+      }
       return;
     }
     const int ip = c0 + lane;
     const double *rec = A.M.pts + ((size_t)chunk * JSC_CHUNK + lane) * JSC_CHUNK_REC;
     double g[3] = {0, 0, 0}, raw = 0, ds = 0;
     if (ip < nb) {
-      const double c[3] = {rec[0], rec[1], rec[2]};
       raw = rec[3];
       ds = rec[4];
-      if (raw == 0.)
-        for (int i = 0; i < 3; i++) g[i] = c[i];
-      else
-        jsc_cart2geo(c, &g[0], &g[1], &g[2]);
+      const Vec3 x = raw == 0. ? Vec3{{rec[0], rec[1], rec[2]}} : geo_of(rec[0], rec[1], rec[2]);
+      for (int i = 0; i < 3; i++) g[i] = x.v[i];
       if (isnan(g[0])) mnan = min(mnan, ip);
       else if (mlow == INT_MAX || g[0] < zlow) {
         zlow = g[0];
@@ -535,7 +571,7 @@ __global__ void __launch_bounds__(128, 6) expand_kernel(ExpandArgs A) {
           go[1] = g[1];
           go[2] = g[2];
           go[3] = raw;
-          write_record(A, a, lev, A.pts + (base + ip) * A.W, g[0], ds, 0.0, -999.0);
+          write_record(A, lo, nlev, A.pts + (base + ip) * A.W, g[0], ds, 0.0, -999.0);
         }
       }
     } else {
@@ -545,8 +581,7 @@ __global__ void __launch_bounds__(128, 6) expand_kernel(ExpandArgs A) {
         if (lane == 0) gp[i] = prev[i];
         prev[i] = __shfl_sync(full, g[i], 31);
       }
-      const int add = ip < nb && ip > 0 ? edge_crossings(A.E, gp[0], g[0]) : 0;
-      const int cnt = ip < nb ? 1 + add : 0;
+      const int cnt = ip < nb ? 1 + (ip > 0 ? edge_crossings(A.E, gp[0], g[0]) : 0) : 0;
       int incl = cnt;
       for (int d = 1; d < 32; d <<= 1) {
         const int v = __shfl_up_sync(full, incl, d);
@@ -554,26 +589,44 @@ __global__ void __launch_bounds__(128, 6) expand_kernel(ExpandArgs A) {
       }
       const int total = __shfl_sync(full, incl, 31);
       if (o + total > nmax || base + o + total > A.max_seg) {
-        if (lane == 0) atomicOr(A.status, JSC_DEV_ERR_NLOS);
+        if (lane == 0) {
+          atomicOr(A.status, JSC_DEV_ERR_NLOS);
+          A.tp[r] = 0;
+        }
         return;
       }
-      if (ip < nb) {
-        double *go = A.geo + (base + o + incl - cnt) * 4;  // first output slot of this lane
-        if (add)
-          for (int il = 0; il < A.E.n_alti; il++) {
-            const double z1 = A.E.alti[il], z2 = A.E.alti[A.E.n_alti - il - 1];
-            if (gp[0] > z1 && g[0] < z1) {
-              segment_point(gp, g, z1, go);
-              go += 4;
+#pragma unroll 1
+      for (int s0 = 0; s0 < total; s0 += 32) {
+        // output point s of the chunk: the k-th crossing before marched point
+        // src, or (k = its crossings) that point
+        const int s = s0 + lane;
+        int src = 0;
+        for (int d = 16; d > 0; d >>= 1)
+          if (__shfl_sync(full, incl, src + d - 1) <= s) src += d;
+        src = min(src, 31);
+        const int cs = __shfl_sync(full, cnt, src);
+        int k = s - (__shfl_sync(full, incl, src) - cs);
+        double a[3], b[3];
+        for (int i = 0; i < 3; i++) {
+          a[i] = __shfl_sync(full, gp[i], src);
+          b[i] = __shfl_sync(full, g[i], src);
+        }
+        if (s < total) {
+          if (k < cs - 1) {
+            double znew = 0;
+            for (int il = 0; il < A.E.n_alti && k >= 0; il++) {
+              const double z1 = A.E.alti[il], z2 = A.E.alti[A.E.n_alti - il - 1];
+              if (a[0] > z1 && b[0] < z1 && k-- == 0) znew = z1;
+              if (a[0] < z2 && b[0] > z2 && k-- == 0) znew = z2;
             }
-            if (gp[0] < z2 && g[0] > z2) {
-              segment_point(gp, g, z2, go);
-              go += 4;
-            }
+            const Vec3 x = crossing_of(a, b, znew);
+            for (int i = 0; i < 3; i++) b[i] = x.v[i];
           }
-        go[0] = g[0];
-        go[1] = g[1];
-        go[2] = g[2];
+          double *go = A.geo + (base + o + s) * 4;
+          go[0] = b[0];
+          go[1] = b[1];
+          go[2] = b[2];
+        }
       }
       o += total;
     }
@@ -588,36 +641,41 @@ __global__ void __launch_bounds__(128, 6) expand_kernel(ExpandArgs A) {
     }
   }
   mnan = __reduce_min_sync(full, mnan);
-  if (lane == 0) tangent_point(A, r, nb, mnan != INT_MAX ? mnan : mlow);
+  if (lane == 0) A.tp[r] = (double)(mnan != INT_MAX ? mnan : mlow);
   if (!EDGES) return;
   __syncwarp();  // the geometry written above, for every lane
   const double *go = A.geo + base * 4;
   double carry[3] = {0, 0, 0};  // position of the point before the 32
+#pragma unroll 1
   for (int i0 = 0; i0 < o; i0 += 32) {
     const int i = i0 + lane;
-    double xc[3] = {0, 0, 0}, xp[3], xn[3], z = 0;
+    double xp[3], xn[3], z = 0;
+    Vec3 xc = {{0, 0, 0}};
     if (i < o) {
       z = go[(size_t)i * 4];
-      jsc_geo2cart(z, go[(size_t)i * 4 + 1], go[(size_t)i * 4 + 2], xc);
+      xc = cart_of(z, go[(size_t)i * 4 + 1], go[(size_t)i * 4 + 2]);
     }
     for (int c = 0; c < 3; c++) {
-      const double up = __shfl_up_sync(full, xc[c], 1);
-      const double dn = __shfl_down_sync(full, xc[c], 1);
+      const double up = __shfl_up_sync(full, xc.v[c], 1);
+      const double dn = __shfl_down_sync(full, xc.v[c], 1);
       xp[c] = lane == 0 ? carry[c] : up;
       xn[c] = dn;
-      carry[c] = __shfl_sync(full, xc[c], 31);
+      carry[c] = __shfl_sync(full, xc.v[c], 31);
     }
-    if (lane == 31 && i + 1 < o)
-      jsc_geo2cart(go[(size_t)(i + 1) * 4], go[(size_t)(i + 1) * 4 + 1],
-                   go[(size_t)(i + 1) * 4 + 2], xn);
+    if (lane == 31 && i + 1 < o) {
+      const Vec3 x = cart_of(go[(size_t)(i + 1) * 4], go[(size_t)(i + 1) * 4 + 1],
+                             go[(size_t)(i + 1) * 4 + 2]);
+      for (int c = 0; c < 3; c++) xn[c] = x.v[c];
+    }
     if (i < o) {
       // chord step (src/lineofsight.c:300-330)
       double ds = 0;
       if (o > 1) {
-        const double back = sqrt((xp[0] - xc[0]) * (xp[0] - xc[0]) + (xp[1] - xc[1]) * (xp[1] - xc[1]) +
-                                 (xp[2] - xc[2]) * (xp[2] - xc[2]));
-        const double ahead = sqrt((xc[0] - xn[0]) * (xc[0] - xn[0]) + (xc[1] - xn[1]) * (xc[1] - xn[1]) +
-                                  (xc[2] - xn[2]) * (xc[2] - xn[2]));
+        const double *c = xc.v;
+        const double back = sqrt((xp[0] - c[0]) * (xp[0] - c[0]) + (xp[1] - c[1]) * (xp[1] - c[1]) +
+                                 (xp[2] - c[2]) * (xp[2] - c[2]));
+        const double ahead = sqrt((c[0] - xn[0]) * (c[0] - xn[0]) + (c[1] - xn[1]) * (c[1] - xn[1]) +
+                                  (c[2] - xn[2]) * (c[2] - xn[2]));
         ds = i == 0 ? 0.5 * ahead : i == o - 1 ? 0.5 * back : 0.5 * (back + ahead);
       }
       A.geo[(base + i) * 4 + 3] = ds;
@@ -625,7 +683,7 @@ __global__ void __launch_bounds__(128, 6) expand_kernel(ExpandArgs A) {
       // of the atmosphere and outside every layer, stands in for it.
       double af, la;
       layer_factor(A, go[(size_t)(i > 0 ? i - 1 : 0) * 4], z, &af, &la);
-      write_record(A, a, lev, A.pts + (base + i) * A.W, z, ds, af, la);
+      write_record(A, lo, nlev, A.pts + (base + i) * A.W, z, ds, af, la);
     }
   }
 }
