@@ -460,8 +460,8 @@ int jsc_formod_batch(jsc_model *m, const ctl_t *ctl, const jsc_batch_input *in,
  * that must not allocate device memory while they run the forward model
  * (see below).
  *
- * Same arguments, same clear-air kernels and launch variant, same results
- * as jsc_formod_batch; host inputs and outputs as there.  Every per-call
+ * Same arguments, same operations in the same order, same results as
+ * jsc_formod_batch; host inputs and outputs as there.  Every per-call
  * device buffer (inputs, hydrostatic pressures, LOS records, outputs) is
  * carved from one static device array of JSC_NOALLOC_SCRATCH_BYTES per
  * device, so the call neither allocates nor frees (jsc_formod_batch
@@ -492,7 +492,8 @@ int jsc_formod_batch_noalloc(jsc_model *m, const ctl_t *ctl,
  * kernel: "hydrostatic", "raytrace", "scatter" (scattering sources: the
  * secondary and solar pencils and the source integrals, or the surrogate
  * path), "surrogate" (the network's inference inside it), "continua" (the
- * lane variants' pre-pass), "ega_rt".  Returns milliseconds, or a
+ * lane variants' pre-pass; the segment pass of the variants 21-22, whose
+ * "ega_rt" spans it), "ega_rt".  Returns milliseconds, or a
  * negative value when timing is off or the kernel did not run. */
 void jsc_batch_set_timing(jsc_batch *b, int on);
 double jsc_batch_kernel_ms(const jsc_batch *b, const char *kernel);
@@ -540,13 +541,17 @@ int jsc_batch_graph_capture(jsc_batch *b, const jsc_batch_input *in,
                             const jsc_batch_output *out, void *stream);
 int jsc_batch_graph_launch(jsc_batch *b, void *stream);
 
-/* Select the EGA launch variant by hand (-1: the default, variant 17, or
- * the lane variant 13 above 16 emitters).  Variants 0-8
+/* Select the EGA launch variant by hand (-1: the default, 21 or 22 by the
+ * run's size, or 17 for table grids with an interval of no width or tables
+ * above 4 GB).  Variants 0-8
  * run a thread per (ray, channel) with every emitter's path state; 9-13 a
  * lane per (ray, channel, emitter) after a separate continuum/Planck pass;
  * 14-20 (up to 16 emitters) lanes over a tile of 32 rays sorted by
- * geometry, a warp per emitter, after the same pass.  All variants compute
- * the same operations in the same order. */
+ * geometry, a warp per emitter, after the same pass; 21-22 the gas
+ * transmittance by a warp per emitter with four lanes or one lane per ray,
+ * then a pass over the (point, channel) segments and one along the rays.
+ * 14-20 fall back to 13 above 16 emitters.  All variants compute the same
+ * operations in the same order. */
 int jsc_batch_set_variant(jsc_batch *b, int variant);
 double jsc_batch_variant_ms(const jsc_batch *b, int variant);
 

@@ -8,7 +8,7 @@
 
 #include "kernels.cuh"
 #include "ega_kernel.cuh"
-#include "ega_lane.cuh"
+#include "ega_gas.cuh"
 #include "scatter.cuh"
 #include "surrogate.h"
 
@@ -111,6 +111,7 @@ extern "C" void jsc_batch_destroy(jsc_batch *b) {
   cudaFree(b->d_pts_b);
   cudaFree(b->d_nsp);
   cudaFree(b->d_sp_off);
+  cudaFree(b->d_sp_idx);
   cudaFree(b->d_sp);
   cudaFree(b->d_sp_atm);
   cudaFree(b->d_src);
@@ -608,7 +609,8 @@ extern "C" int jsc_scan_selftest(int device, int n, unsigned budget, int stall) 
 // ray 2: ega_ray_rot_kernel, the emitter warps take the transfer step in
 // turn (block 32 emitter warps); 16 and 19-20 order the blocks
 // channel-major.  More than 16 emitters run the lane variant 13 instead.
-// jsc_batch_autotune picks one.
+// 21 and 22 (ray 3): minb lanes per ray and emitter, the transfer as passes
+// of its own (ega_gas.cuh).  jsc_batch_autotune picks one.
 struct EgaVariant { int blk, minb, roll, lane, ray; };
 static const EgaVariant kEgaVariants[] = {
     {128, 4, 0, 0, 0}, {128, 6, 0, 0, 0}, {128, 8, 0, 0, 0}, {256, 3, 0, 0, 0},
@@ -616,47 +618,88 @@ static const EgaVariant kEgaVariants[] = {
     {256, 6, 1, 0, 0}, {128, 12, 0, 1, 0}, {128, 8, 0, 1, 0}, {256, 4, 0, 1, 0},
     {256, 5, 0, 1, 0}, {512, 2, 0, 1, 0}, {0, 3, 0, 1, 1}, {0, 4, 0, 1, 1},
     {0, 4, 0, 1, 1},   {0, 4, 0, 1, 2},   {0, 5, 0, 1, 2}, {0, 4, 0, 1, 2},
-    {0, 5, 0, 1, 2}};
-static const int kNumEgaVariants = 21;
+    {0, 5, 0, 1, 2},   {0, 4, 0, 0, 3},
+    {0, 1, 0, 0, 3}};
+static const int kNumEgaVariants = 23;
 static_assert(kNumEgaVariants <= 32, "ega_variant_ms holds 32 timings");
 static const int kLaneBase = 9;
 static const int kRayBase = 14;
+
+static bool gas_variant(int v) { return kEgaVariants[v].ray == 3; }
 
 // Emitter warps of the ray-tile kernel for ng emitters (0: not available).
 static int ray_warps(int ng) {
   return ng <= 2 ? 2 : ng <= 4 ? 4 : ng <= 8 ? 8 : ng <= 16 ? 16 : 0;
 }
-// Default launch variant of clear-air runs: the ray-tile kernel with the
-// transfer step taken in turn (422 ms against 631 ms for the fastest lane
-// variant and 716 ms for the thread-per-channel variant 6 on 100k rays,
-// 8 emitters, 64 channels).
-static const int kEgaDefault = 17;
-
-// Default launch variant of runs with aerosol/cloud layers (the scattering
-// path and its child batches): the same ray-tile kernel (819 ms per plain
-// single-scattering step of 4000 limb rays, 16 channels, 2 emitters,
-// against 847 ms for the lane variant 10).
-static const int kScatterDefault = 17;
+// Default launch variants: four lanes per ray up to kGasNarrow warps of one
+// lane per ray, one lane above; the ray-tile kernel for table grids with an
+// interval of no width and for tables above 4 GB.  The line: 1664 warps 1.09
+// ms with four lanes and 1.14 with one, 2016 warps 1.44 and 1.40 (limb rays,
+// 16 channels; with nadir rays between them, whose lanes then idle, it lies at
+// about 3500).
+static const int kEgaDefault = 21;
+static const int kEgaWide = 22;
+static const int kEgaNoWidths = 17;
+static const int64_t kGasNarrow = 2048;
 
 // The variant a run of b launches (-1 resolves to the default for its
 // configuration).
 static int run_variant(const jsc_batch *b) {
-  if (b->ega_variant >= 0 && b->ega_variant < kNumEgaVariants) return b->ega_variant;
-  return b->cfg.sca_n > 0 ? kScatterDefault : kEgaDefault;
+  int v = b->ega_variant;
+  if (v < 0 || v >= kNumEgaVariants) {
+    const int64_t warps = ((int64_t)b->n_rays + 31) / 32 * b->cfg.nd * (b->cfg.ng > 0 ? b->cfg.ng : 1);
+    v = warps <= kGasNarrow ? kEgaDefault : kEgaWide;
+  }
+  return gas_variant(v) && !b->m->dv.grid_dt ? kEgaNoWidths : v;
 }
 
 static bool lane_variant(int variant) {
-  const int v = (variant >= 0 && variant < kNumEgaVariants) ? variant : kEgaDefault;
-  return kEgaVariants[v].lane != 0;
+  return kEgaVariants[variant].lane != 0;
 }
 
-static int launch_ega(const EgaArgs &ea, int nr, int ndp, int ng, int variant,
+static void ev_record(jsc_batch *b, int k, int end, cudaStream_t s) {
+  if (b->timing) cudaEventRecord(b->ev[2 * k + end], s);
+  if (end) b->ran[k] = 1;
+}
+
+// Gas transmittance, segment terms and transfer of the gas variants.
+static int launch_gas(jsc_batch *b, const EgaArgs &ea, int lanes, cudaStream_t s) {
+  GasArgs ga;
+  ga.e = ea;
+  ga.tg = b->d_ctm;
+  jsc_ega_gas_launch(ga, lanes, s);
+  JSC_LAUNCH_CHECK();
+  SegmentArgs sa;
+  sa.m = ea.m;
+  sa.cfg = ea.cfg;
+  sa.n_points = b->n_points;
+  sa.n_live = b->fixed ? b->d_los_off + ea.n_rays : nullptr;
+  sa.W = ea.W;
+  sa.pts = ea.pts;
+  sa.x = b->d_ctm;
+  sa.src = b->d_srcp;
+  sa.beta = ea.beta;
+  sa.aero_nl = ea.aero_nl;
+  sa.src_sca = ea.src_sca;
+  sa.sp_idx = b->d_sp_idx;
+  sa.n_sp = b->max_sp;
+  ev_record(b, JSC_T_CTM, 0, s);
+  jsc_segment_launch(sa, s);
+  JSC_LAUNCH_CHECK();
+  ev_record(b, JSC_T_CTM, 1, s);
+  jsc_transfer_launch(ea, b->d_ctm, b->d_srcp, s);
+  JSC_LAUNCH_CHECK();
+  return JSC_OK;
+}
+
+static int launch_ega(jsc_batch *b, const EgaArgs &ea, int nr, int ndp, int ng, int variant,
                       cudaStream_t s) {
   const int64_t threads = (int64_t)nr * ndp;
   const unsigned g128 = (unsigned)((threads + 127) / 128);
   const unsigned g256 = (unsigned)((threads + 255) / 256);
-  const int v = (variant >= 0 && variant < kNumEgaVariants) ? variant : kEgaDefault;
+  const int v = gas_variant(variant) && !b->m->dv.grid_dt ? kEgaNoWidths : variant;
   const bool dig = ea.digest != nullptr;  // index digests (every variant has them)
+  if (gas_variant(v)) return launch_gas(b, ea, kEgaVariants[v].minb, s);
   if (kEgaVariants[v].ray && ray_warps(ng) && ea.order) {
     jsc_ega_ray_launch(ea, v - kRayBase, dig, s);
     JSC_LAUNCH_CHECK();
@@ -675,11 +718,6 @@ static int launch_ega(const EgaArgs &ea, int nr, int ndp, int ng, int variant,
   else jsc_ega_launch_gmax(ea, g128, g256, v, dig, s);
   JSC_LAUNCH_CHECK();
   return JSC_OK;
-}
-
-static void ev_record(jsc_batch *b, int k, int end, cudaStream_t s) {
-  if (b->timing) cudaEventRecord(b->ev[2 * k + end], s);
-  if (end) b->ran[k] = 1;
 }
 
 static void fill_ray_args(const jsc_batch *b, RayArgs &ra) {
@@ -836,6 +874,17 @@ static int reserve_points(jsc_batch *b, int64_t n_sp) {
   return JSC_OK;
 }
 
+// Room for the scattering-point number of every LOS point.
+static int reserve_sp_idx(jsc_batch *b) {
+  if (b->sp_idx_seg >= b->max_seg) return JSC_OK;
+  cudaFree(b->d_sp_idx);
+  b->d_sp_idx = nullptr;
+  b->sp_idx_seg = 0;
+  int st = jsc_dmalloc(&b->d_sp_idx, (size_t)b->max_seg);
+  if (!st) b->sp_idx_seg = b->max_seg;
+  return st;
+}
+
 // Scattering points per ray and their list (src/forwardmodel.c:317-331).
 static int list_scattering_points(jsc_batch *b, cudaStream_t s) {
   const int nr = b->n_rays;
@@ -861,6 +910,7 @@ static int list_scattering_points(jsc_batch *b, cudaStream_t s) {
   sa.nlos_mut = nullptr;
   sa.status = b->d_status;
   sa.n_listed = nullptr;
+  sa.sp_idx = nullptr;
   sp_count_kernel<<<(nr + 127) / 128, 128, 0, s>>>(sa);
   JSC_LAUNCH_CHECK();
   if ((st = launch_scan(b, b->d_nsp, nr, b->d_sp_off, s))) return st;
@@ -870,8 +920,10 @@ static int list_scattering_points(jsc_batch *b, cudaStream_t s) {
   b->n_sp = *b->h_total;
   if ((st = reserve_points(b, b->n_sp))) return st;
   if (b->n_sp == 0) return JSC_OK;
+  if ((st = reserve_sp_idx(b))) return st;
   sa.sp = b->d_sp;
   sa.sp_atm = b->d_sp_atm;
+  sa.sp_idx = b->d_sp_idx;
   sp_list_kernel<<<(nr + 127) / 128, 128, 0, s>>>(sa);
   JSC_LAUNCH_CHECK();
   return JSC_OK;
@@ -1081,6 +1133,7 @@ static int fixed_sources(jsc_batch *b, cudaStream_t s) {
   sa.nlos_mut = b->d_nlos;
   sa.status = b->d_status;
   sa.n_listed = b->d_sp_listed;
+  sa.sp_idx = b->d_sp_idx;
   sp_count_kernel<<<(nr + 127) / 128, 128, 0, s>>>(sa);
   JSC_LAUNCH_CHECK();
   if ((st = launch_scan(b, b->d_nsp, nr, b->d_sp_off, s))) return st;
@@ -1163,6 +1216,7 @@ static int prepare_fixed_scattering(jsc_batch *b) {
     if ((st = jsc_dmalloc(&b->d_sp_off, (size_t)b->max_rays + 1))) return st;
   }
   if ((st = reserve_points(b, b->fx_max_sp))) return st;
+  if ((st = reserve_sp_idx(b))) return st;
   if (!b->d_sp_listed && (st = jsc_dmalloc(&b->d_sp_listed, 1))) return st;
   if ((st = ensure_child(b, &b->child, (int)(chunk * na), 0, JSC_FIXED_PENCIL_LOS))) return st;
   if ((st = ensure_child(b, &b->sun_child, (int)chunk, 0, JSC_FIXED_SUN_LOS))) return st;
@@ -1842,7 +1896,7 @@ static int batch_run(jsc_batch *b, cudaStream_t s) {
   ea.src_pl = b->d_srcp;
   ea.order = nullptr;
   const int variant = run_variant(b);
-  if (kEgaVariants[variant].ray && ray_warps(m->ng)) {
+  if (gas_variant(variant) || (kEgaVariants[variant].ray && ray_warps(m->ng))) {
     int e = jsc_ray_order(nr, b->d_ray_atm, b->d_nlos, b->d_tsurf, b->d_tp, b->d_rkeys,
                           b->d_rorder, b->d_rtmp, b->rtmp_bytes, s);
     if (e) {
@@ -1869,7 +1923,7 @@ static int batch_run(jsc_batch *b, cudaStream_t s) {
   }
   b->last_ega = ea;
   ev_record(b, JSC_T_EGA, 0, s);
-  int st = launch_ega(ea, nr, ndp, m->ng, variant, s);
+  int st = launch_ega(b, ea, nr, ndp, m->ng, variant, s);
   if (st) return st;
   JSC_LAUNCH_CHECK();
   ev_record(b, JSC_T_EGA, 1, s);
@@ -1961,7 +2015,7 @@ extern "C" int jsc_batch_autotune(jsc_batch *b, void *stream) {
   if (st) return st;
   EgaArgs ea = b->last_ega;
   ea.digest = nullptr;
-  if (ray_warps(b->m->ng)) {
+  {
     int e = jsc_ray_order(b->n_rays, b->d_ray_atm, b->d_nlos, b->d_tsurf, b->d_tp, b->d_rkeys,
                           b->d_rorder, b->d_rtmp, b->rtmp_bytes, s);
     if (e) {
@@ -1977,11 +2031,11 @@ extern "C" int jsc_batch_autotune(jsc_batch *b, void *stream) {
     jsc_set_error(JSC_ERR_CUDA, "autotune: cudaEventCreate failed");
     return JSC_ERR_CUDA;
   }
-  int best = kEgaDefault;
+  int best = run_variant(b);
   float best_ms = 1e30f;
   for (int v = 0; v < kNumEgaVariants && !st; v++) {
     cudaError_t e = cudaEventRecord(e0, s);
-    if (e == cudaSuccess) st = launch_ega(ea, b->n_rays, ea.ndp, b->m->ng, v, s);
+    if (e == cudaSuccess) st = launch_ega(b, ea, b->n_rays, ea.ndp, b->m->ng, v, s);
     if (!st && e == cudaSuccess) e = cudaEventRecord(e1, s);
     if (!st && e == cudaSuccess) e = cudaEventSynchronize(e1);
     float ms = -1;
@@ -2022,6 +2076,11 @@ extern "C" int jsc_batch_variant(const jsc_batch *b, int *variant, int *blk, int
   if (!b) return JSC_ERR_ARG;
   const int v = run_variant(b);
   if (variant) *variant = v;
+  if (gas_variant(v)) {
+    if (blk) *blk = 32 * (b->m->ng > 0 ? b->m->ng : 1);
+    if (minb) *minb = 1;
+    return JSC_OK;
+  }
   const int rw = kEgaVariants[v].ray ? ray_warps(b->m->ng) : 0;
   if (blk)
     *blk = kEgaVariants[v].ray

@@ -1,0 +1,49 @@
+// Launchers of the gas transmittance, the segment pass and the transfer pass.
+#include "ega_gas.cuh"
+
+// A warp per emitter; the register budget follows the block size.
+template <bool DIG>
+static void gas_launch(const GasArgs &ga, cudaStream_t s) {
+  const int nw = ga.e.m.ng > 0 ? ga.e.m.ng : 1;
+  const unsigned blocks = (unsigned)(((int64_t)ga.e.n_rays + 31) / 32 * ga.e.m.nd);
+  const size_t sh = gas_shmem(nw, 32, nw <= 8 ? 4 : 2);
+  if (nw <= 2) ega_gas_kernel<DIG, 4, 64, 16><<<blocks, 32 * nw, sh, s>>>(ga);
+  else if (nw <= 4) ega_gas_kernel<DIG, 4, 128, 8><<<blocks, 32 * nw, sh, s>>>(ga);
+  else if (nw <= 8) ega_gas_kernel<DIG, 4, 256, 4><<<blocks, 32 * nw, sh, s>>>(ga);
+  else ega_gas_kernel<DIG, 2, 1024, 1><<<blocks, 32 * nw, sh, s>>>(ga);
+}
+
+template <bool DIG>
+static void gas4_launch(const GasArgs &ga, cudaStream_t s) {
+  const int nw = ga.e.m.ng > 0 ? ga.e.m.ng : 1;
+  const unsigned blocks = (unsigned)(((int64_t)ga.e.n_rays + 7) / 8 * ga.e.m.nd);
+  const size_t sh = gas_shmem(nw, 8, 4);
+  if (nw <= 2) ega_gas4_kernel<DIG, 4, 64, 16><<<blocks, 32 * nw, sh, s>>>(ga);
+  else if (nw <= 4) ega_gas4_kernel<DIG, 4, 128, 8><<<blocks, 32 * nw, sh, s>>>(ga);
+  else if (nw <= 8) ega_gas4_kernel<DIG, 4, 256, 4><<<blocks, 32 * nw, sh, s>>>(ga);
+  else ega_gas4_kernel<DIG, 4, 1024, 1><<<blocks, 32 * nw, sh, s>>>(ga);
+}
+
+void jsc_ega_gas_launch(const GasArgs &ga, int lanes, cudaStream_t s) {
+  if (lanes == 4) {
+    if (ga.e.digest) gas4_launch<true>(ga, s);
+    else gas4_launch<false>(ga, s);
+  } else {
+    if (ga.e.digest) gas_launch<true>(ga, s);
+    else gas_launch<false>(ga, s);
+  }
+}
+
+void jsc_segment_launch(const SegmentArgs &sa, cudaStream_t s) {
+  const int64_t n = sa.n_points * sa.m.nd;
+  if (n <= 0) return;
+  int64_t blocks = (n + 255) / 256;
+  // a count known only on the device: a grid of a few blocks per SM walks it
+  if (sa.n_live && blocks > 148 * 16) blocks = 148 * 16;
+  segment_kernel<<<(unsigned)blocks, 256, 0, s>>>(sa);
+}
+
+void jsc_transfer_launch(const EgaArgs &ea, const double *x, const double *src, cudaStream_t s) {
+  const int64_t n = (int64_t)ea.n_rays * ea.m.nd;
+  transfer_kernel<<<(unsigned)((n + 127) / 128), 128, 0, s>>>(ea, x, src);
+}

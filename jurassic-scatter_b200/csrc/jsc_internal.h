@@ -206,6 +206,13 @@ typedef struct JSC_ALIGN(8) {
   int nf;
 } jsc_row;
 
+/* Per table: log2 of the first column and columns per unit of log2 u where
+ * every row has the same evenly spaced columns (else 0, 0), and 1 where
+ * every row strictly increases in u and eps. */
+typedef struct JSC_ALIGN(16) {
+  float l0, il, strict, pad;
+} jsc_tab_info;
+
 /* Row descriptor flags. */
 #define JSC_ROW_STRICT 1   /* u and eps strictly increasing */
 
@@ -220,8 +227,13 @@ typedef struct {
   const int *grid_nt;
   const double *grid_t;
   const int *tab_grid;       /* [nd*ng] grid id, -1: table unusable (np<2) */
+  const jsc_tab_info *tab_info;  /* [nd*ng] */
   const jsc_row *rows;       /* [TBLNPMAX][TBLNTMAX][ng][nd] */
   const jsc_node *nodes;
+  /* The grids' interval widths and their reciprocals, (width, reciprocal)
+   * per [grid][ip][it] and [grid][ip]; null when an interval has no width or
+   * the nodes exceed 4 GB. */
+  const double *grid_dt, *grid_dp;
   const double *planck_b, *planck_s;   /* [nd][JSC_NPLANCK] */
   const jsc_ctm_coef *ctm;             /* [nd] */
   const double *nu;                    /* [nd] */

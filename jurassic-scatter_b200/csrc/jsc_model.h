@@ -17,7 +17,9 @@ struct jsc_model {
   int *d_grid_np, *d_grid_nt, *d_tab_grid, *d_window;
   double *d_grid_p, *d_grid_t, *d_planck_b, *d_planck_s, *d_nu;
   jsc_row *d_rows;
+  jsc_tab_info *d_tab_info;
   jsc_node *d_nodes;
+  double *d_grid_dt, *d_grid_dp;
   jsc_ctm_coef *d_ctm;
 };
 
@@ -123,6 +125,8 @@ struct jsc_batch {
   int64_t *d_sp_off;        // [max_rays+1]
   double *d_sp;             // [max_sp][JSC_SP_REC]
   int *d_sp_atm;            // [max_sp]
+  int *d_sp_idx;            // [sp_idx_seg] number of a LOS point that scatters
+  int64_t sp_idx_seg;
   double *d_src;            // [max_sp][nd]
   int64_t max_sp, n_sp;
   double *d_theta2;         // [n_theta2] solar scattering angles

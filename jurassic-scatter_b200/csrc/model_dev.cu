@@ -7,6 +7,7 @@
 //    nodes of its interval and computes the slope with the same IEEE
 //    single-precision operations the reference's LIN evaluates;
 //  * Planck source tables with slopes, continuum coefficients per channel.
+#include <math.h>
 #include <stdio.h>
 #include <stdlib.h>
 #include <string.h>
@@ -43,6 +44,61 @@ __global__ void build_nodes_kernel(jsc_row *rows, const int64_t *row_pt,
     }
     if (__all_sync(0xffffffffu, inc) && lane == 0) rows[r].nf |= JSC_ROW_STRICT << 16;
   }
+}
+
+// One block per table: are all its rows strictly increasing, and do they
+// have the same columns, evenly spaced in log2 u to within a third of a
+// column (the guess of a forward interval is then right or one off)?
+// Threads take the rows, the first row with points sets the spacing.
+__global__ void __launch_bounds__(256) table_info_kernel(const jsc_row *rows, const jsc_node *nodes,
+                                                         int ng, int nd, jsc_tab_info *info) {
+  __shared__ int first;
+  const int id = blockIdx.x / ng, ig = blockIdx.x - id * ng;
+  const int nrow = TBLNPMAX * TBLNTMAX;
+  if (threadIdx.x == 0) first = nrow;
+  __syncthreads();
+  int strict = 1, even = 1;
+  for (int s = threadIdx.x; s < nrow; s += blockDim.x) {
+    const jsc_row rd = rows[((size_t)s * ng + ig) * nd + id];
+    if ((rd.nf & 0xffff) < 2) continue;
+    atomicMin(&first, s);
+    if (!((rd.nf >> 16) & JSC_ROW_STRICT)) strict = 0;
+  }
+  strict = __syncthreads_and(strict);
+  float l0 = 0, step = 0;
+  if (first < nrow) {
+    const jsc_row rd = rows[((size_t)first * ng + ig) * nd + id];
+    const int n = rd.nf & 0xffff;
+    const float u0 = nodes[rd.off].u;
+    l0 = log2f(u0);
+    step = (log2f(nodes[rd.off + n - 1].u) - l0) / (float)(n - 1);
+    if (!(u0 > 0 && step > 0)) even = 0;
+  } else {
+    even = 0;
+  }
+  for (int s = threadIdx.x >> 5; s < nrow && even; s += blockDim.x >> 5) {
+    const jsc_row rd = rows[((size_t)s * ng + ig) * nd + id];
+    const int n = rd.nf & 0xffff;
+    if (n < 2) continue;
+    for (int k = threadIdx.x & 31; k < n; k += 32)
+      if (!(fabsf(log2f(nodes[rd.off + k].u) - l0 - (float)k * step) < 0.33f * step)) even = 0;
+  }
+  even = __syncthreads_and(even);
+  if (threadIdx.x == 0)
+    info[blockIdx.x] = {even && strict ? l0 : 0.f, even && strict ? 1.f / step : 0.f,
+                        strict ? 1.f : 0.f, 0.f};
+}
+
+// Grid interval widths and their reciprocals, [n][2]; ok: none is so narrow
+// or wide that dividing by it needs more than the reciprocal.
+static std::vector<double> widths(const double *x, int n, bool *ok) {
+  std::vector<double> w(2 * (size_t)(n > 0 ? n : 0), 0.0);
+  for (int i = 0; i + 1 < n; i++) {
+    w[2 * i] = x[i + 1] - x[i];
+    w[2 * i + 1] = 1.0 / w[2 * i];
+    if (!(fabs(w[2 * i]) > 1e-100 && fabs(w[2 * i]) < 1e100)) *ok = false;
+  }
+  return w;
 }
 
 static uint64_t fnv1a(const void *data, size_t n, uint64_t h) {
@@ -155,13 +211,29 @@ static int model_upload(jsc_model *m, const jsc_host_model *hm) {
           }
         }
 
+  bool known = niv < (1 << 29);  // and 32-bit byte offsets of the nodes
+  std::vector<double> g_dt(2 * g_t.size(), 0.0), g_dp(2 * g_p.size(), 0.0);
+  for (int g = 0; g < ngrid; g++) {
+    const size_t o = (size_t)g * TBLNPMAX;
+    const std::vector<double> wp = widths(&g_p[o], g_np[g], &known);
+    memcpy(&g_dp[2 * o], wp.data(), wp.size() * sizeof(double));
+    for (int ip = 0; ip < g_np[g]; ip++) {
+      const std::vector<double> wt = widths(&g_t[(o + ip) * TBLNTMAX], g_nt[o + ip], &known);
+      memcpy(&g_dt[2 * (o + ip) * TBLNTMAX], wt.data(), wt.size() * sizeof(double));
+    }
+  }
+
   int st;
   if ((st = upload(&m->d_grid_np, g_np.data(), g_np.size()))) return st;
   if ((st = upload(&m->d_grid_p, g_p.data(), g_p.size()))) return st;
   if ((st = upload(&m->d_grid_nt, g_nt.data(), g_nt.size()))) return st;
   if ((st = upload(&m->d_grid_t, g_t.data(), g_t.size()))) return st;
+  if (known && (st = upload(&m->d_grid_dt, g_dt.data(), g_dt.size()))) return st;
+  if (known && (st = upload(&m->d_grid_dp, g_dp.data(), g_dp.size()))) return st;
   if ((st = upload(&m->d_tab_grid, tab_grid.data(), tab_grid.size()))) return st;
   if ((st = upload(&m->d_rows, rows.data(), rows.size()))) return st;
+  if ((st = jsc_dmalloc(&m->d_tab_info, (size_t)ntab))) return st;
+  JSC_CUDA_TRY(cudaMemset(m->d_tab_info, 0, (size_t)(ntab > 0 ? ntab : 1) * sizeof(jsc_tab_info)));
   if ((st = jsc_dmalloc(&m->d_nodes, (size_t)niv))) return st;
   m->n_nodes = niv;
   m->n_grid = ngrid;
@@ -175,6 +247,8 @@ static int model_upload(jsc_model *m, const jsc_host_model *hm) {
     if ((st = upload(&drp, row_pt.data(), row_pt.size()))) return st;
     build_nodes_kernel<<<148 * 8, 256>>>(m->d_rows, drp, (int)nslots, du, de,
                                           m->d_nodes);
+    jsc_count_launch();
+    table_info_kernel<<<ntab, 256>>>(m->d_rows, m->d_nodes, ng, nd, m->d_tab_info);
     jsc_count_launch();
     cudaError_t e = cudaDeviceSynchronize();
     cudaFree(du);
@@ -208,7 +282,10 @@ static int model_upload(jsc_model *m, const jsc_host_model *hm) {
   d.grid_t = m->d_grid_t;
   d.tab_grid = m->d_tab_grid;
   d.rows = m->d_rows;
+  d.tab_info = m->d_tab_info;
   d.nodes = m->d_nodes;
+  d.grid_dt = m->d_grid_dt;
+  d.grid_dp = m->d_grid_dp;
   d.planck_b = m->d_planck_b;
   d.planck_s = m->d_planck_s;
   d.ctm = m->d_ctm;
@@ -259,7 +336,10 @@ extern "C" void jsc_model_destroy(jsc_model *m) {
   cudaFree(m->d_grid_t);
   cudaFree(m->d_tab_grid);
   cudaFree(m->d_rows);
+  cudaFree(m->d_tab_info);
   cudaFree(m->d_nodes);
+  cudaFree(m->d_grid_dt);
+  cudaFree(m->d_grid_dp);
   cudaFree(m->d_planck_b);
   cudaFree(m->d_planck_s);
   cudaFree(m->d_ctm);

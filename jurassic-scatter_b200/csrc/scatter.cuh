@@ -102,6 +102,7 @@ struct SpArgs {
   const int64_t *sp_off;    // [n_rays+1]
   double *sp;               // [n_sp][JSC_SP_REC]
   int *sp_atm;              // [n_sp] profile of the point
+  int *sp_idx;              // [LOS points] number of a point that scatters
   int64_t max_sp;           // capacity of sp (fixed-capacity runs; 0: unbounded)
   int *nlos_mut;            // rays whose points do not fit: their LOS is emptied
   unsigned *status;
@@ -163,6 +164,7 @@ static __global__ void sp_list_kernel(SpArgs A) {
     o[SP_P] = rc[REC_P];
     o[SP_T] = rc[REC_T];
     A.sp_atm[k] = A.ray_atm[r];
+    A.sp_idx[A.los_off[r] + ip] = (int)k;
     k++;
   }
 }

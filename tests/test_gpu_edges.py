@@ -159,3 +159,67 @@ def test_source_integral_against_port(workdir, nd, nalpha, layer):
     assert np.all(np.isfinite(ref["rad"])) and np.all(ref["rad"] > 0)
     assert max_rel(got["rad"], ref["rad"]) <= 1e-9
     assert max_rel(got["tau"], ref["tau"]) <= 1e-9
+
+
+@pytest.mark.parametrize("ng,nd,n", [(1, 1, 1), (2, 3, 7), (3, 2, 8), (5, 4, 9), (8, 2, 33), (9, 2, 17), (16, 1, 8),
+                                     (17, 2, 9), (25, 1, 5)])
+def test_window_variants_against_others(workdir, ng, nd, n):
+    """The window lookups (four lanes and one lane per ray) against the
+    thread-per-channel kernel, which
+    computes the same operations in the same order: the same bits and table
+    indices at emitter counts of every block size and rays at the edges of
+    a tile of 8 and of 32."""
+    from jscat import api, synth, structs as S
+    emitters = (synth.CFG1_EMITTERS + ["X%02d" % i for i in range(25)])[:ng]
+    nus = synth.CFG1_NU[5::20][:nd]
+    ctlkw, atms, ray_atm, geom = synth.batched_case(workdir, n_rays=n, rays_per_atm=4, seed=77,
+                                                    emitters=emitters, nus=nus)
+    ctl = S.make_ctl(**ctlkw)
+    inp = synth.batch_from(atms, ray_atm, geom)
+    m = api.Model(ctl)
+    four, one, want = (api.formod_batch(ctl, inp, model=m, digest=True, variant=v) for v in (21, 22, 6))
+    for k in want:
+        np.testing.assert_array_equal(four[k], want[k])
+        np.testing.assert_array_equal(one[k], want[k])
+
+
+@pytest.mark.parametrize("kind", ["uneven", "ties", "shifted", "grids", "short"])
+def test_gas_variants_on_irregular_tables(workdir, kind):
+    """The default kernels' rules on tables (evenly spaced columns, strictly
+    increasing rows, one grid) against the thread-per-channel kernel on
+    tables that miss each of them: unevenly spaced columns, rows with equal
+    neighbours, columns that differ by row, another (p, T) grid per emitter,
+    and rows of two, one or no point.  The same bits and table indices."""
+    from jscat import api, synth, structs as S
+    rng = np.random.default_rng(11)
+    d = os.path.join(workdir, "irregular_%s" % kind)
+    os.makedirs(d, exist_ok=True)
+    base, nu, emitters = os.path.join(d, "tab"), 800.0, ["CO2", "H2O", "O3"]
+    synth.write_filter("%s_%.4f.filt" % (base, nu), nu)
+    for e in emitters:
+        p, t, rows = synth.emissivity_table(e, nu, 20261203)
+        step = 1 + (kind == "grids") * emitters.index(e)
+        p, t, rows = p[::step], t, rows[::step]
+        for i, line in enumerate(rows):
+            for j, (u, v) in enumerate(line):
+                if kind == "uneven":
+                    keep = np.sort(rng.choice(len(u), max(2, len(u) // 3), replace=False))
+                    line[j] = (u[keep], v[keep])
+                elif kind == "ties":
+                    line[j] = (u, np.minimum(v, np.float32(0.6)))
+                elif kind == "shifted":
+                    line[j] = (u[(i + j) % 7:], v[(i + j) % 7:])
+                elif kind == "short" and (i * 30 + j) % 5 == 0:
+                    n = (i + j) % 3
+                    line[j] = (u[150:150 + n], v[150:150 + n])
+        synth.write_table_bin("%s_%.4f_%s.bin" % (base, nu, e), p, t, rows)
+    ctl = S.make_ctl(emitters, [nu], base, hydz=0.0)
+    atms = [synth.atmosphere(emitters, rng, t_sigma=5.0, vmr_sigma=0.2) for _ in range(3)]
+    n = 41
+    inp = synth.batch_from(atms, np.arange(n) % 3, _mixed_rays(n))
+    m = api.Model(ctl)
+    four, one, want = (api.formod_batch(ctl, inp, model=m, digest=True, variant=v) for v in (21, 22, 6))
+    assert np.any(want["tau"] < 0.9)
+    for k in want:
+        np.testing.assert_array_equal(four[k], want[k])
+        np.testing.assert_array_equal(one[k], want[k])
