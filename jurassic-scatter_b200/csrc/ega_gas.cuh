@@ -445,49 +445,138 @@ struct SegmentArgs {
   const double *src_sca;  // scattering sources [n_sp][nd], or null
   const int *sp_idx;      // scattering point of a LOS point
   int64_t n_sp;
+  int step;               // points per block and step, at most JSC_SEG_POINTS
 };
+
+// What the channels of a LOS point share of jsc_continuum and of the segment
+// terms: the subexpressions in the order of that function.
+struct SegPoint {
+  double T, DS, rDS, P, pp;    // rDS: 1 / DS, or 0 where dividing by it needs more
+  double co2, d1, d2, d3;      // u / N_A / 1000 * P / P0; the three T polynomials
+  double u_h2o, q, h2o_y, h2o_v, h2o_a2;
+  double dtp, af;              // T above its Planck node; layer factor
+  int plk, ia, sp;             // Planck node, layer, scattering point
+};
+
+#define JSC_SEG_POINTS 128
+#define JSC_SEG_THREADS 256
+
+// ctm / DS (div_known within its range).
+__device__ __forceinline__ double per_length(double ctm, const SegPoint &p) {
+  return p.rDS != 0 && (ctm == 0 || fabs(ctm) > 1e-250) ? div_known(ctm, p.DS, p.rDS) : ctm / p.DS;
+}
+
+// jsc_continuum of channel coefficients c at point p.
+__device__ __forceinline__ double segment_continuum(const jsc_dev_model &m, const jsc_run_cfg &cfg,
+                                                    const jsc_ctm_coef *__restrict__ c, double nu,
+                                                    double kwin, const SegPoint &p) {
+  double beta = kwin;
+  if (cfg.ctm_co2) {
+    double ctm = 0;
+    if (m.ig_co2 >= 0 && c->co2_on)
+      ctm = p.co2 * (p.d1 * c->co2_c230 - p.d2 * c->co2_c260 + p.d3 * c->co2_c296);
+    beta += per_length(ctm, p);
+  }
+  if (cfg.ctm_h2o) {
+    double ctm = 0;
+    if (m.ig_h2o >= 0 && c->h2o_on) {
+      const double ctwslf = c->h2o_self296 * pow(c->h2o_ratio, p.h2o_y);
+      const double a1 = nu * p.u_h2o * tanh(p.h2o_v * nu);
+      const double a3 = p.pp * (p.q * ctwslf + (1 - p.q) * c->h2o_frn) * 1e-20;
+      ctm = a1 * p.h2o_a2 * a3;
+    }
+    beta += per_length(ctm, p);
+  }
+  if (cfg.ctm_n2 && c->n2_on) {
+    const double t0 = 273, tr = 296, q_n2 = 0.79, tt = t0 / p.T;
+    beta += 0.1 * (p.pp * p.pp) * (tt * tt) * q_n2 * c->n2_b *
+            exp(c->n2_beta * (1 / tr - 1 / p.T)) *
+            (q_n2 + (1 - q_n2) * (1.294 - 0.4545 * p.T / tr));
+  }
+  if (cfg.ctm_o2 && c->o2_on) {
+    const double t0 = 273, tr = 296, q_o2 = 0.21, tt = t0 / p.T;
+    beta += 0.1 * (p.pp * p.pp) * (tt * tt) * q_o2 * c->o2_b *
+            exp(c->o2_beta * (1 / tr - 1 / p.T));
+  }
+  return beta;
+}
 
 // Transmittance x and source of a segment: x = the gas transmittance times
 // the continuum (and aerosol) attenuation, or, at a scattering point
 // (src/forwardmodel.c:317-363), minus the attenuation by bext, whose
 // radiance is accumulated in another order; the sign tells them apart.
 // Gas transmittance 0 leaves the radiance alone: x = 1, source 0.
-static __global__ void __launch_bounds__(256) segment_kernel(SegmentArgs A) {
+// A block takes 64 or 128 points at a time: what their channels share (nine
+// divisions) is computed once per point into shared memory, then threads
+// take (point, channel) pairs.  Bound by instruction issue (pow, tanh and exp
+// in FP64): 5.3 ms for 20,000 rays x 64 channels, 7.0 ms with the shared part
+// in every pair.
+static __global__ void __launch_bounds__(JSC_SEG_THREADS)
+segment_kernel(const __grid_constant__ SegmentArgs A) {
+  __shared__ SegPoint sp[JSC_SEG_POINTS];
   const int nd = A.m.nd;
   int64_t pts = A.n_points;
   if (A.n_live && *A.n_live < pts) pts = *A.n_live;
-  const int64_t total = pts * nd;
-  for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < total;
-       t += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t pt = t / nd;
-    const int d = (int)(t - pt * nd);
-    const double *rec = A.pts + pt * A.W;
-    const double tau_gas = A.x[t];
-    double x = 1, s = 0;
-    if (tau_gas > 0) {
-      const double P = rec[REC_P], T = rec[REC_T], DS = rec[REC_DS], af = rec[REC_AF];
-      const int w = A.m.window[d];
-      const double beta = continua(A.m, A.cfg, A.m.ctm[d], A.m.nu[d],
-                                   w < A.m.nw ? rec[REC_K + w] : 0.0, P, T, DS, rec[REC_QH2O],
-                                   rec + REC_K + A.m.nw);
-      s = planck_src(A.m, d, (int)rec[REC_PLK], T);
-      const int ia = (int)rec[REC_AI];
-      if (A.src_sca && af > 0) {
-        const int k = A.sp_idx[pt];
-        const double ss = k >= 0 && k < A.n_sp ? A.src_sca[(size_t)k * nd + d] : 0.0;
-        const double be = A.beta[ia * nd + d], bs = A.beta[A.aero_nl * nd + ia * nd + d];
-        const double bext = (-1.) * log(tau_gas) / DS + beta + af * be;
-        x = -exp(-1 * bext * DS);
-        s = ((bext - af * bs) * s + af * bs * ss) / bext;
-      } else if (A.cfg.sca_n == 0 || af == 0) {
-        x = tau_gas * exp(-1. * beta * DS);
-      } else {
-        const double bx = A.beta[(A.cfg.sca_ext_beta_a ? 2 : 0) * A.aero_nl * nd + ia * nd + d];
-        x = tau_gas * exp(-1. * (beta + af * bx) * DS);
-      }
+  for (int64_t p0 = (int64_t)blockIdx.x * A.step; p0 < pts; p0 += (int64_t)gridDim.x * A.step) {
+    const int n = (int)(pts - p0 < A.step ? pts - p0 : A.step);
+    __syncthreads();  // the pairs of the step before
+    if ((int)threadIdx.x < n) {
+      const double *rec = A.pts + (p0 + threadIdx.x) * A.W, *u = rec + REC_K + A.m.nw;
+      const double P = rec[REC_P], T = rec[REC_T], DS = rec[REC_DS];
+      SegPoint p;
+      p.T = T;
+      p.DS = DS;
+      p.rDS = DS > 1e-50 && DS < 1e50 ? 1 / DS : 0.0;
+      p.P = P;
+      p.pp = P / JSC_P0;
+      const double u_co2 = A.m.ig_co2 >= 0 ? u[A.m.ig_co2] : 0.0;
+      p.co2 = u_co2 / JSC_AVOGADRO / 1000 * P / JSC_P0;
+      const double dt230 = T - 230, dt260 = T - 260, dt296 = T - 296;
+      p.d1 = dt260 * 5.050505e-4 * dt296;
+      p.d2 = dt230 * 9.259259e-4 * dt296;
+      p.d3 = dt230 * 4.208754e-4 * dt260;
+      p.u_h2o = A.m.ig_h2o >= 0 ? u[A.m.ig_h2o] : 0.0;
+      p.q = rec[REC_QH2O];
+      p.h2o_y = (296 - T) / (296 - 260);
+      p.h2o_v = .7193876 / T;
+      p.h2o_a2 = 296 / T;
+      p.plk = (int)rec[REC_PLK];
+      p.dtp = T - planck_temp(p.plk);
+      p.af = rec[REC_AF];
+      p.ia = (int)rec[REC_AI];
+      p.sp = A.src_sca && p.af > 0 ? A.sp_idx[p0 + threadIdx.x] : -1;
+      sp[threadIdx.x] = p;
     }
-    A.x[t] = x;
-    A.src[t] = s;
+    __syncthreads();
+    for (int i = threadIdx.x; i < n * nd; i += JSC_SEG_THREADS) {
+      const int k = i / nd, d = i - k * nd;
+      const SegPoint &p = sp[k];
+      const int64_t t = p0 * nd + i;
+      const double tau_gas = A.x[t];
+      double x = 1, s = 0;
+      if (tau_gas > 0) {
+        const int w = A.m.window[d];
+        const double kwin = w < A.m.nw ? A.pts[(p0 + k) * A.W + REC_K + w] : 0.0;
+        const double beta = segment_continuum(A.m, A.cfg, A.m.ctm + d, A.m.nu[d], kwin, p);
+        const size_t o = (size_t)d * JSC_NPLANCK + p.plk;
+        s = A.m.planck_b[o] + A.m.planck_s[o] * p.dtp;
+        if (A.src_sca && p.af > 0) {
+          const double ss =
+              p.sp >= 0 && p.sp < A.n_sp ? A.src_sca[(size_t)p.sp * nd + d] : 0.0;
+          const double be = A.beta[p.ia * nd + d], bs = A.beta[A.aero_nl * nd + p.ia * nd + d];
+          const double bext = (-1.) * log(tau_gas) / p.DS + beta + p.af * be;
+          x = -exp(-1 * bext * p.DS);
+          s = ((bext - p.af * bs) * s + p.af * bs * ss) / bext;
+        } else {
+          double b = beta;
+          if (A.cfg.sca_n != 0 && p.af != 0)
+            b = beta + p.af * A.beta[(A.cfg.sca_ext_beta_a ? 2 : 0) * A.aero_nl * nd + p.ia * nd + d];
+          x = tau_gas * exp(-1. * b * p.DS);
+        }
+      }
+      A.x[t] = x;
+      A.src[t] = s;
+    }
   }
 }
 
@@ -535,5 +624,5 @@ static __global__ void __launch_bounds__(128) transfer_kernel(EgaArgs A, const d
 
 // lanes: 1 or 4 a ray
 void jsc_ega_gas_launch(const GasArgs &ga, int lanes, cudaStream_t s);
-void jsc_segment_launch(const SegmentArgs &sa, cudaStream_t s);
+void jsc_segment_launch(SegmentArgs sa, cudaStream_t s);
 void jsc_transfer_launch(const EgaArgs &ea, const double *x, const double *src, cudaStream_t s);
