@@ -27,7 +27,7 @@ CU_SRCS = ["model_dev.cu", "batch.cu", "ega_g2.cu", "ega_g4.cu", "ega_g8.cu",
            "ega_gmax.cu", "ega_lane_s.cu", "ega_lane_l.cu", "ega_ray.cu", "ega_gas.cu", "noalloc.cu", "surrogate.cu",
            "surrogate_tc.cu", "mie.cu"]
 HEADERS = ["jsc_internal.h", "physics.h", "ckd_tables.h", "jsc_model.h",
-           "cuda_util.cuh", "device_common.cuh", "kernels.cuh", "trace.cuh", "ega_kernel.cuh",
+           "cuda_util.cuh", "device_common.cuh", "device_math.cuh", "kernels.cuh", "trace.cuh", "ega_kernel.cuh",
            "ega_lane.cuh", "ega_gas.cuh", "scatter.cuh", "surrogate.h", "surrogate_tc.h"]
 
 INC = ["-I" + os.path.join(REPO, "include"), "-I" + CSRC]

@@ -11,25 +11,13 @@
 // Only an emitter's path transmittance ties one LOS point to the next; the
 // radiance, whose exponentials depend on the segment only, leaves that chain.
 #pragma once
+#include "device_math.cuh"
 #include "ega_lane.cuh"
 
 struct GasArgs {
   EgaArgs e;
   double *tg;  // [points][nd] gas transmittance
 };
-
-// num / b from the rounded reciprocal y of b, corrected by the exact
-// remainder (Markstein 1990: a quotient within an ulp plus one such step is
-// the rounded quotient); the grids' widths are known beforehand.
-__device__ __forceinline__ double div_known(double num, double b, double y) {
-  const double q = num * y;
-  return __fma_rn(__fma_rn(-b, q, num), y, q);
-}
-
-// jsc_lin with the width b = x1 - x0 and its reciprocal y.
-__device__ __forceinline__ double lin_known(double x0, double y0, double y1, double x, double2 by) {
-  return y0 + div_known(y1 - y0, by.x, by.y) * (x - x0);
-}
 
 // Node at byte offset o of the node array (gas variants run on tables below
 // 4 GB: one 32-bit offset, and neighbours by immediate offsets).

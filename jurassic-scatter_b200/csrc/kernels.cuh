@@ -128,10 +128,17 @@ static __global__ void __launch_bounds__(JSC_HYDRO_THREADS) hydro_kernel(AtmArgs
   if (a.lev) {
     // Level record l: altitudes, pressure and temperature of the interval
     // [l, l+1], the quotients of EXP (LIN where a pressure is not positive)
-    // and LIN, which of the two, and whether the profile strictly ascends.
-    int down = 0;
-    for (int l = tid; l + 1 < n; l += JSC_HYDRO_THREADS) down |= !(z[l] < z[l + 1]);
+    // and LIN, and which of the two.
+    // Last entry: 0, or 1 for a strictly ascending profile, 2 if its
+    // altitudes are evenly spaced besides (to 1 % of the spacing).
+    int down = 0, uneven = 0;
+    const double step = (z[n - 1] - z[0]) / (n - 1);
+    for (int l = tid; l + 1 < n; l += JSC_HYDRO_THREADS) {
+      down |= !(z[l] < z[l + 1]);
+      uneven |= !(fabs(z[l] - z[0] - l * step) < 0.01 * step);
+    }
     down = __syncthreads_or(down);  // and the pressures are visible
+    uneven = __syncthreads_or(uneven);
     for (int l = tid; l + 1 < n; l += JSC_HYDRO_THREADS) {
       double *r = a.lev + 8 * (size_t)(lo + l);
       const double p0 = p[l], p1 = p[l + 1];
@@ -143,7 +150,7 @@ static __global__ void __launch_bounds__(JSC_HYDRO_THREADS) hydro_kernel(AtmArgs
       r[4] = ex ? log(p1 / p0) / (z[l + 1] - z[l]) : (p1 - p0) / (z[l + 1] - z[l]);
       r[5] = (t[l + 1] - t[l]) / (z[l + 1] - z[l]);
       r[6] = ex ? 1.0 : 0.0;
-      r[7] = down ? 0.0 : 1.0;
+      r[7] = down ? 0.0 : uneven ? 1.0 : 2.0;
       for (int c = 0; c < a.ng + a.nw; c++) {
         const double *v = (c < a.ng ? a.q + (size_t)c * a.n_levels
                                     : a.k + (size_t)(c - a.ng) * a.n_levels) + lo + l;

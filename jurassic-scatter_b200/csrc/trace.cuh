@@ -16,6 +16,7 @@
 #pragma once
 #include <limits.h>
 
+#include "device_math.cuh"
 #include "kernels.cuh"
 
 #define JSC_CHUNK 32     // points per chunk
@@ -71,6 +72,13 @@ __device__ __forceinline__ double radius_of(const double *x) {
   return sqrt(x[0] * x[0] + x[1] * x[1] + x[2] * x[2]);
 }
 
+// Level guess of altitude z: from the spacing (zf: lowest altitude, zs: levels
+// per km) on evenly spaced profiles, else (zs 0) the level h of the lookup
+// before.
+__device__ __forceinline__ int level_guess(double zf, double zs, int n, double z, int h) {
+  return zs > 0 ? min(max(__double2int_rz((z - zf) * zs), 0), n - 2) : h;
+}
+
 // The march of one ray.  LANES 8: a group of eight lanes per ray (gmask:
 // the group's lanes, role: the lane's number in it) holds the same ray
 // state; a refracted step needs the state at five positions (the point, the
@@ -86,6 +94,7 @@ __device__ __forceinline__ int march_ray(const RayArgs &A, const MarchPool &M, i
   const double *__restrict__ lev = A.lev + 8 * (size_t)lo;
   const double *__restrict__ zl = A.z + lo;
   const double zmin = A.zmin[ai], zmax = A.zmax[ai];
+  const double zf = zl[0], zs = lev[7] == 2 ? (n - 1) / (zl[n - 1] - zf) : 0.0;
   *tsurf = -999;
   if (in.obsz < zmin) {
     if (role == 0) atomicOr(A.status, JSC_DEV_ERR_OBSERVER);
@@ -179,7 +188,8 @@ __device__ __forceinline__ int march_ray(const RayArgs &A, const MarchPool &M, i
     double ds = A.rayds;
     if (A.raydz > 0) {
       double xh[3];
-      for (int i = 0; i < 3; i++) xh[i] = x[i] / norm;
+      const double rn = 1 / norm;
+      for (int i = 0; i < 3; i++) xh[i] = div_known(x[i], norm, rn);
       const double cosa = fabs(ex0[0] * xh[0] + ex0[1] * xh[1] + ex0[2] * xh[2]);
       if (cosa != 0) {
         const double dz = A.raydz / cosa;
@@ -224,10 +234,13 @@ __device__ __forceinline__ int march_ray(const RayArgs &A, const MarchPool &M, i
         }
         if (role == 0 || role > 4)
           for (int i = 0; i < 3; i++) xm[i] = x[i];
-        level_state(lev, zl, n, radius_of(xm) - JSC_RE, h0, &p, &t);
+        const double zm = radius_of(xm) - JSC_RE;
+        h0 = level_guess(zf, zs, n, zm, h0);
+        level_state(lev, zl, n, zm, h0, &p, &t);
         const double rf = jsc_refractivity(p, t);
         nr = 1 + __shfl_sync(gmask, rf, 0, LANES);
-        const double g = (rf - __shfl_sync(gmask, rf, 1, LANES)) / JSC_FD_STEP;
+        const double g = div_known(rf - __shfl_sync(gmask, rf, 1, LANES), JSC_FD_STEP,
+                                   1 / JSC_FD_STEP);
         for (int i = 0; i < 3; i++) ng[i] = __shfl_sync(gmask, g, 2 + i, LANES);
         tlast = __shfl_sync(gmask, t, 4, LANES);
       } else {
@@ -240,7 +253,7 @@ __device__ __forceinline__ int march_ray(const RayArgs &A, const MarchPool &M, i
         for (int i = 0; i < 3; i++) {
           xm[i] += JSC_FD_STEP;
           level_state(lev, zl, n, radius_of(xm) - JSC_RE, h2, &p, &t);
-          ng[i] = (jsc_refractivity(p, t) - rm) / JSC_FD_STEP;
+          ng[i] = div_known(jsc_refractivity(p, t) - rm, JSC_FD_STEP, 1 / JSC_FD_STEP);
           xm[i] -= JSC_FD_STEP;
         }
         tlast = t;
@@ -250,8 +263,8 @@ __device__ __forceinline__ int march_ray(const RayArgs &A, const MarchPool &M, i
     }
     for (int i = 0; i < 3; i++) ex1[i] = ex0[i] * nr;
     for (int i = 0; i < 3; i++) ex1[i] += ds * ng[i];
-    const double en = radius_of(ex1);
-    for (int i = 0; i < 3; i++) ex1[i] /= en;
+    const double en = radius_of(ex1), re = 1 / en;
+    for (int i = 0; i < 3; i++) ex1[i] = div_known(ex1[i], en, re);
     for (int i = 0; i < 3; i++) x[i] += 0.5 * ds * (ex0[i] + ex1[i]);
     for (int i = 0; i < 3; i++) ex0[i] = ex1[i];
   }
@@ -414,9 +427,8 @@ __device__ __forceinline__ Vec3 crossing_of(const double *g0, const double *g1, 
 static __device__ __noinline__ void write_record(const ExpandArgs &A, int lo, int n, double *rec,
                                                  double z, double ds, double af, double ai) {
   const double *zl = A.z + lo, *lev = A.lev + 8 * (size_t)lo;
-  // level guess for evenly spaced altitudes
   const double zf = zl[0];
-  int h = (int)fmin(fmax((z - zf) / (zl[n - 1] - zf) * (n - 1), 0.0), (double)(n - 2));
+  int h = level_guess(zf, (n - 1) / (zl[n - 1] - zf), n, z, n - 2);
   double p, t;
   level_state(lev, zl, n, z, h, &p, &t);
   const double dz = z - zl[h];
