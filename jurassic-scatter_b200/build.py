@@ -28,7 +28,7 @@ CU_SRCS = ["model_dev.cu", "batch.cu", "ega_g2.cu", "ega_g4.cu", "ega_g8.cu",
            "surrogate_tc.cu", "mie.cu"]
 HEADERS = ["jsc_internal.h", "physics.h", "ckd_tables.h", "jsc_model.h",
            "cuda_util.cuh", "device_common.cuh", "device_math.cuh", "kernels.cuh", "trace.cuh", "ega_kernel.cuh",
-           "ega_lane.cuh", "ega_gas.cuh", "scatter.cuh", "surrogate.h", "surrogate_tc.h"]
+           "ega_lane.cuh", "ega_gas.cuh", "scatter.cuh", "surrogate.h", "surrogate_tc.h", "surrogate_train.cuh"]
 
 INC = ["-I" + os.path.join(REPO, "include"), "-I" + CSRC]
 CFLAGS = ["-O2", "-fPIC", "-fopenmp", "-ffp-contract=off", "-std=gnu11",

@@ -6,8 +6,8 @@
 // Network: x[SUR_NF] -> tanh(W0 x + b0) -> tanh(W1 . + b1) -> tanh(W2 . + b2)
 // -> W3 . + b3 = y[nout], width SUR_W; W_l stored [out][in].
 //
-// Training (FP32, this file): tiled SGEMM forward/backward, tanh, MSE loss
-// on standardised targets, Adam.  Inference: BF16 weights on the tensor
+// Training (FP32, surrogate_train.cuh): forward, MSE loss on standardised
+// targets, backward and Adam.  Inference: BF16 weights on the tensor
 // cores (mma.sync m16n8k16, FP32 accumulation), tanh in FP32.
 //
 // Features of a scattering point (sur_features_kernel): altitude, cosine
@@ -27,6 +27,7 @@
 #include "scatter.cuh"
 #include "surrogate.h"
 #include "surrogate_tc.h"
+#include "surrogate_train.cuh"
 
 // ------------------------------------------------------------ features --
 
@@ -59,170 +60,6 @@ static __global__ void sur_features_kernel(int n, const double *sp, float *feat)
   // elevation above the geometric horizon: 90 - sza + dip, dip = acos(RE / (RE + z))
   const double zz = z > 0 ? z : 0.0;
   f[7] = (float)(90.0 - sza + acos(JSC_RE / (JSC_RE + zz)) * 180 / M_PI);
-}
-
-// ------------------------------------------------------- FP32 training --
-
-#define TG_M 64
-#define TG_N 64
-#define TG_K 16
-
-// C[M][N] (ldc) = op(A) op(B) (+ bias[n]) with op(A)(m,k) = TA ? A[k*lda+m]
-// : A[m*lda+k] and op(B)(k,n) = TB ? B[n*ldb+k] : B[k*ldb+n].  256 threads,
-// a 64 x 64 tile per block, 4 x 4 outputs per thread.  With gridDim.z > 1
-// the K range is split over blockIdx.z and block z writes its partial
-// product to the slice C + z M ldc (no bias); ksum_kernel adds the slices
-// in order, so training is deterministic.
-template <bool TA, bool TB>
-static __global__ void __launch_bounds__(256)
-sgemm_kernel(int M, int N, int K, const float *A, int lda, const float *B, int ldb, float *C,
-             int ldc, const float *bias) {
-  __shared__ float As[TG_K][TG_M + 4];
-  __shared__ float Bs[TG_K][TG_N + 4];
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
-  const int m0 = blockIdx.y * TG_M, n0 = blockIdx.x * TG_N;
-  const int kchunk = (K + (int)gridDim.z - 1) / (int)gridDim.z;
-  const int kb = (int)blockIdx.z * kchunk, ke = min(K, kb + kchunk);
-  float acc[4][4] = {};
-  for (int k0 = kb; k0 < ke; k0 += TG_K) {
-    for (int i = threadIdx.x; i < TG_K * TG_M; i += 256) {
-      const int kk = i / TG_M, mm = i - kk * TG_M;
-      const int m = m0 + mm, k = k0 + kk;
-      As[kk][mm] = (m < M && k < ke) ? (TA ? A[(size_t)k * lda + m] : A[(size_t)m * lda + k]) : 0.f;
-    }
-    for (int i = threadIdx.x; i < TG_K * TG_N; i += 256) {
-      const int kk = i / TG_N, nn = i - kk * TG_N;
-      const int n = n0 + nn, k = k0 + kk;
-      Bs[kk][nn] = (n < N && k < ke) ? (TB ? B[(size_t)n * ldb + k] : B[(size_t)k * ldb + n]) : 0.f;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int kk = 0; kk < TG_K; kk++) {
-      float a[4], b[4];
-#pragma unroll
-      for (int i = 0; i < 4; i++) {
-        a[i] = As[kk][ty * 4 + i];
-        b[i] = Bs[kk][tx * 4 + i];
-      }
-#pragma unroll
-      for (int i = 0; i < 4; i++)
-#pragma unroll
-        for (int j = 0; j < 4; j++) acc[i][j] += a[i] * b[j];
-    }
-    __syncthreads();
-  }
-#pragma unroll
-  for (int i = 0; i < 4; i++)
-#pragma unroll
-    for (int j = 0; j < 4; j++) {
-      const int m = m0 + ty * 4 + i, n = n0 + tx * 4 + j;
-      if (m < M && n < N) {
-        if (gridDim.z > 1) C[((size_t)blockIdx.z * M + m) * ldc + n] = acc[i][j];
-        else C[(size_t)m * ldc + n] = acc[i][j] + (bias ? bias[n] : 0.f);
-      }
-    }
-}
-
-// C[i] = sum over z = 0 .. nz-1, in that order, of ws[z mn + i].
-static __global__ void ksum_kernel(int64_t mn, int nz, const float *ws, float *c) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= mn) return;
-  float t = 0;
-  for (int z = 0; z < nz; z++) t += ws[(size_t)z * mn + i];
-  c[i] = t;
-}
-
-// Most K slices of a split product (sizes the workspace).
-#define SUR_KSPLIT_MAX 64
-
-// ksplit > 1: split-K for products with a long K and a small output (the
-// weight gradients: K = batch), partial products in ws (ksplit M ldc
-// floats, ksplit <= SUR_KSPLIT_MAX), bias ignored.
-template <bool TA, bool TB>
-static void sgemm(int M, int N, int K, const float *A, int lda, const float *B, int ldb, float *C,
-                  int ldc, const float *bias, cudaStream_t s, int ksplit = 1,
-                  float *ws = nullptr) {
-  if (ksplit > 1 && ws) {
-    dim3 grid((N + TG_N - 1) / TG_N, (M + TG_M - 1) / TG_M, ksplit);
-    sgemm_kernel<TA, TB><<<grid, 256, 0, s>>>(M, N, K, A, lda, B, ldb, ws, ldc, nullptr);
-    const int64_t mn = (int64_t)M * ldc;
-    ksum_kernel<<<(unsigned)((mn + 255) / 256), 256, 0, s>>>(mn, ksplit, ws, C);
-    return;
-  }
-  dim3 grid((N + TG_N - 1) / TG_N, (M + TG_M - 1) / TG_M, 1);
-  sgemm_kernel<TA, TB><<<grid, 256, 0, s>>>(M, N, K, A, lda, B, ldb, C, ldc, bias);
-}
-
-static __global__ void tanh_kernel(int64_t n, float *h) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) h[i] = tanhf(h[i]);
-}
-
-// dZ = dH * (1 - H^2) in place
-static __global__ void tanh_bwd_kernel(int64_t n, const float *h, float *dh) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) dh[i] *= 1.f - h[i] * h[i];
-}
-
-// dY = 2 (Y - T) / n, and the per-block partial sums of (Y - T)^2.
-static __global__ void mse_kernel(int64_t cnt, int n, const float *y, const float *t, float *dy,
-                                  float *part) {
-  __shared__ float red[256];
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  float e2 = 0;
-  if (i < cnt) {
-    const float e = y[i] - t[i];
-    dy[i] = 2.f * e / (float)n;
-    e2 = e * e;
-  }
-  red[threadIdx.x] = e2;
-  __syncthreads();
-  for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-    if ((int)threadIdx.x < o) red[threadIdx.x] += red[threadIdx.x + o];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) part[blockIdx.x] = red[0];
-}
-
-// db[o] = sum over the batch of dZ[:, o]: block (32 columns) x (8 row
-// lanes), coalesced over the columns.
-static __global__ void colsum_kernel(int n, int cols, const float *dz, float *db) {
-  const int o = blockIdx.x * 32 + (threadIdx.x & 31), r0 = threadIdx.x >> 5;
-  float sacc = 0;
-  if (o < cols)
-    for (int i = r0; i < n; i += 8) sacc += dz[(size_t)i * cols + o];
-  __shared__ float red[8][32];
-  red[r0][threadIdx.x & 31] = sacc;
-  __syncthreads();
-  if (r0 == 0 && o < cols) {
-    float t = 0;
-    for (int j = 0; j < 8; j++) t += red[j][threadIdx.x];
-    db[o] = t;
-  }
-}
-
-static __global__ void adam_kernel(int64_t n, float *p, const float *g, float *m, float *v,
-                                   float lr, float b1, float b2, float c1, float c2, float eps) {
-  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const float gi = g[i];
-  const float mi = b1 * m[i] + (1 - b1) * gi;
-  const float vi = b2 * v[i] + (1 - b2) * gi * gi;
-  m[i] = mi;
-  v[i] = vi;
-  p[i] -= lr * (mi / c1) / (sqrtf(vi / c2) + eps);
-}
-
-// Gather a minibatch: rows idx[i] of X (standardised here) and T.
-static __global__ void gather_kernel(int n, int nout, const int *idx, const float *X,
-                                     const float *T, const float *xm, const float *xs, float *xb,
-                                     float *tb) {
-  const int i = blockIdx.x;
-  if (i >= n) return;
-  const int64_t r = idx[i];
-  for (int c = threadIdx.x; c < SUR_NF; c += blockDim.x)
-    xb[(size_t)i * SUR_NF + c] = (X[r * SUR_NF + c] - xm[c]) / xs[c];
-  for (int c = threadIdx.x; c < nout; c += blockDim.x) tb[(size_t)i * nout + c] = T[r * nout + c];
 }
 
 // ------------------------------------------------------ BF16 inference --
@@ -425,11 +262,11 @@ struct jsc_surrogate {
   int trained, packed;
   // training scratch
   int max_batch;
-  float *d_h[5];            // activations per layer, [max_batch][width]
-  float *d_dh[2];           // two ping-pong gradient buffers [max_batch][SUR_W]
-  float *d_xb, *d_tb, *d_part;
-  float *d_ksum;            // split-K partial products of the weight gradients
-  int *d_idx;               // [max_batch] (gradient checks)
+  float *d_wt[4];           // transposed weights [in][out]
+  float *d_h[4];            // inputs of the layers [max_batch][in]
+  float *d_dz[4];           // gradients of their outputs [max_batch][out]
+  float *d_err, *d_tb, *d_part;
+  float *d_ws;              // partial weight gradients [TR_KSPLIT_MAX][weights]
   int *d_perm;              // [n_train] per-epoch permutation
   float *d_X, *d_T;         // device copy of the training set
   int64_t n_train;
@@ -443,15 +280,16 @@ extern "C" int jsc_surrogate_param_count(const jsc_surrogate *s) {
 }
 
 static void free_train(jsc_surrogate *s) {
-  for (int i = 0; i < 5; i++) cudaFree(s->d_h[i]), s->d_h[i] = nullptr;
-  for (int i = 0; i < 2; i++) cudaFree(s->d_dh[i]), s->d_dh[i] = nullptr;
-  // d_xb is the first activation buffer d_h[0], freed above
+  for (int l = 0; l < 4; l++) {
+    cudaFree(s->d_h[l]);
+    cudaFree(s->d_dz[l]);
+    s->d_h[l] = s->d_dz[l] = nullptr;
+  }
+  cudaFree(s->d_err);
   cudaFree(s->d_tb);
   cudaFree(s->d_part);
-  cudaFree(s->d_ksum);
-  cudaFree(s->d_idx);
-  s->d_xb = s->d_tb = s->d_part = s->d_ksum = nullptr;
-  s->d_idx = nullptr;
+  cudaFree(s->d_ws);
+  s->d_err = s->d_tb = s->d_part = s->d_ws = nullptr;
   s->max_batch = 0;
 }
 
@@ -465,6 +303,7 @@ extern "C" void jsc_surrogate_destroy(jsc_surrogate *s) {
       cudaFree(s->d_m[l][j]);
       cudaFree(s->d_v[l][j]);
     }
+  for (int l = 0; l < 4; l++) cudaFree(s->d_wt[l]);
   cudaFree(s->d_image);
   cudaFree(s->d_tc_image);
   cudaFree(s->d_tc_status);
@@ -600,72 +439,102 @@ extern "C" int jsc_surrogate_set_params(jsc_surrogate *s, const float *in) {
 }
 
 static int ensure_train(jsc_surrogate *s, int batch) {
-  if (s->max_batch >= batch) return JSC_OK;
-  free_train(s);
   int st = JSC_OK;
-  const int width[5] = {SUR_NF, SUR_W, SUR_W, SUR_W, s->nout};
-  for (int i = 0; i < 5 && !st; i++) st = jsc_dmalloc(&s->d_h[i], (size_t)batch * width[i]);
-  for (int i = 0; i < 2 && !st; i++) st = jsc_dmalloc(&s->d_dh[i], (size_t)batch * SUR_W);
+  for (int l = 0; l < 4 && !st; l++)
+    if (!s->d_wt[l]) st = jsc_dmalloc(&s->d_wt[l], (size_t)s->in[l] * s->out[l]);
+  if (st || s->max_batch >= batch) return st;
+  free_train(s);
+  size_t nw = 0;
+  for (int l = 0; l < 4 && !st; l++) {
+    st = jsc_dmalloc(&s->d_h[l], (size_t)batch * s->in[l]);
+    st = st ? st : jsc_dmalloc(&s->d_dz[l], (size_t)batch * s->out[l]);
+    nw += (size_t)s->in[l] * s->out[l];
+  }
+  st = st ? st : jsc_dmalloc(&s->d_err, (size_t)batch * s->nout);
   st = st ? st : jsc_dmalloc(&s->d_tb, (size_t)batch * s->nout);
   st = st ? st : jsc_dmalloc(&s->d_part, (size_t)(batch * SUR_NOUT_MAX + 255) / 256 + 1);
-  st = st ? st : jsc_dmalloc(&s->d_idx, (size_t)batch);
-  st = st ? st : jsc_dmalloc(&s->d_ksum, (size_t)SUR_KSPLIT_MAX * SUR_W *
-                                             (SUR_NOUT_MAX > SUR_W ? SUR_NOUT_MAX : SUR_W));
+  st = st ? st : jsc_dmalloc(&s->d_ws, TR_KSPLIT_MAX * nw);
   if (st) {
     free_train(s);
     return st;
   }
-  s->d_xb = s->d_h[0];
   s->max_batch = batch;
   return JSC_OK;
 }
 
-// Forward and backward over one standardised minibatch already in d_h[0] /
-// d_tb; gradients into d_g, returns the loss (mean over the batch of the
-// squared error summed over outputs).
-static int forward_backward(jsc_surrogate *s, int n, cudaStream_t st, float *loss) {
+static TrainNet train_net(const jsc_surrogate *s) {
+  TrainNet net;
+  net.nout = s->nout;
+  net.off[0] = 0;
   for (int l = 0; l < 4; l++) {
-    sgemm<false, true>(n, s->out[l], s->in[l], s->d_h[l], s->in[l], s->d_p[l][0], s->in[l],
-                       s->d_h[l + 1], s->out[l], s->d_p[l][1], st);
-    if (l < 3) {
-      const int64_t cnt = (int64_t)n * s->out[l];
-      tanh_kernel<<<(unsigned)((cnt + 255) / 256), 256, 0, st>>>(cnt, s->d_h[l + 1]);
-    }
+    net.in[l] = s->in[l];
+    net.out[l] = s->out[l];
+    net.w[l] = s->d_p[l][0];
+    net.b[l] = s->d_p[l][1];
+    net.wt[l] = s->d_wt[l];
+    net.gw[l] = s->d_g[l][0];
+    net.gb[l] = s->d_g[l][1];
+    net.mw[l] = s->d_m[l][0];
+    net.mb[l] = s->d_m[l][1];
+    net.vw[l] = s->d_v[l][0];
+    net.vb[l] = s->d_v[l][1];
+    net.off[l + 1] = net.off[l] + s->in[l] * s->out[l];
   }
-  const int64_t cnt = (int64_t)n * s->nout;
-  const int nblk = (int)((cnt + 255) / 256);
-  float *dy = s->d_dh[0];
-  mse_kernel<<<nblk, 256, 0, st>>>(cnt, n, s->d_h[4], s->d_tb, dy, s->d_part);
-  float *dcur = dy, *dnext = s->d_dh[1];
-  for (int l = 3; l >= 0; l--) {
-    // dW = dZ^T H_l, db = colsum(dZ)
-    const int tiles = ((s->out[l] + TG_M - 1) / TG_M) * ((s->in[l] + TG_N - 1) / TG_N);
-    int ksplit = 296 / tiles;  // about two blocks per SM
-    if (ksplit > n / 64) ksplit = n / 64 > 0 ? n / 64 : 1;
-    if (ksplit > SUR_KSPLIT_MAX) ksplit = SUR_KSPLIT_MAX;
-    sgemm<true, false>(s->out[l], s->in[l], n, dcur, s->out[l], s->d_h[l], s->in[l],
-                       s->d_g[l][0], s->in[l], nullptr, st, ksplit > 1 ? ksplit : 1, s->d_ksum);
-    colsum_kernel<<<(s->out[l] + 31) / 32, 256, 0, st>>>(n, s->out[l], dcur, s->d_g[l][1]);
-    if (l > 0) {
-      // dH_l = dZ W_l, then dZ_{l-1} = dH_l (1 - H_l^2)
-      sgemm<false, false>(n, s->in[l], s->out[l], dcur, s->out[l], s->d_p[l][0], s->in[l], dnext,
-                          s->in[l], nullptr, st);
-      const int64_t c2 = (int64_t)n * s->in[l];
-      tanh_bwd_kernel<<<(unsigned)((c2 + 255) / 256), 256, 0, st>>>(c2, s->d_h[l], dnext);
-      float *tmp = dcur;
-      dcur = dnext;
-      dnext = tmp;
-    }
+  return net;
+}
+
+static int train_begin(const TrainNet &net) {
+  train_transpose_kernel<<<(net.off[4] + TR_THREADS - 1) / TR_THREADS, TR_THREADS>>>(net);
+  JSC_LAUNCH_CHECK();
+  JSC_CUDA_TRY(cudaFuncSetAttribute(train_rows_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    TR_ROWS_SHMEM));
+  return JSC_OK;
+}
+
+// Forward, backward and update of one minibatch (samples idx of x and t, or
+// the first n as they are).  loss: mean over the batch of the squared error
+// summed over outputs, read back when asked for.
+static int train_step(jsc_surrogate *s, const TrainNet &net, int n, const int *idx, const float *x,
+                      const float *t, const float *xm, const float *xs, const TrainAdam &adam,
+                      float *loss) {
+  TrainBatch b;
+  b.n = n;
+  b.idx = idx;
+  b.x = x;
+  b.t = t;
+  b.xm = xm;
+  b.xs = xs;
+  for (int l = 0; l < 4; l++) {
+    b.h[l] = s->d_h[l];
+    b.dz[l] = s->d_dz[l];
   }
+  b.err = s->d_err;
+  train_rows_kernel<<<(n + TR_ROWS - 1) / TR_ROWS, TR_THREADS, TR_ROWS_SHMEM>>>(net, b);
+  JSC_LAUNCH_CHECK();
+  // 64 slices of the samples, none below 64 of them
+  int nz = n / 64 > 0 ? n / 64 : 1;
+  if (nz > TR_KSPLIT_MAX) nz = TR_KSPLIT_MAX;
+  const int kchunk = (n + nz - 1) / nz;
+  int ncol = 0;
+  for (int l = 0; l < 4; l++) ncol += (net.out[l] + 31) / 32;
+  train_weights_kernel<<<ncol + nz * TR_TILES, TR_THREADS>>>(net, b, ncol, kchunk, s->d_ws);
+  JSC_LAUNCH_CHECK();
+  const int np = net.off[4] + 3 * SUR_W + net.nout;
+  train_update_kernel<<<(np + TR_THREADS - 1) / TR_THREADS, TR_THREADS>>>(net, adam, nz, s->d_ws);
   JSC_LAUNCH_CHECK();
   if (loss) {
+    const int64_t cnt = (int64_t)n * s->nout;
+    const int nblk = (int)((cnt + TR_THREADS - 1) / TR_THREADS);
+    train_loss_kernel<<<nblk, TR_THREADS>>>(cnt, s->d_err, s->d_part);
+    JSC_LAUNCH_CHECK();
     float *h = (float *)malloc(nblk * sizeof(float));
     if (!h) return JSC_ERR_NOMEM;
-    JSC_CUDA_TRY(cudaMemcpyAsync(h, s->d_part, nblk * sizeof(float), cudaMemcpyDeviceToHost, st));
-    JSC_CUDA_TRY(cudaStreamSynchronize(st));
+    const cudaError_t e =
+        cudaMemcpy(h, s->d_part, nblk * sizeof(float), cudaMemcpyDeviceToHost);
     double acc = 0;
-    for (int i = 0; i < nblk; i++) acc += h[i];
+    for (int i = 0; i < nblk && e == cudaSuccess; i++) acc += h[i];
     free(h);
+    JSC_CUDA_TRY(e);
     *loss = (float)(acc / n);
   }
   return JSC_OK;
@@ -679,7 +548,10 @@ extern "C" int jsc_surrogate_loss_grad(jsc_surrogate *s, const float *x, const f
   if (st) return st;
   JSC_CUDA_TRY(cudaMemcpy(s->d_h[0], x, (size_t)n * SUR_NF * sizeof(float), cudaMemcpyHostToDevice));
   JSC_CUDA_TRY(cudaMemcpy(s->d_tb, t, (size_t)n * s->nout * sizeof(float), cudaMemcpyHostToDevice));
-  if ((st = forward_backward(s, n, 0, loss))) return st;
+  const TrainNet net = train_net(s);
+  const TrainAdam none = {};
+  if ((st = train_begin(net))) return st;
+  if ((st = train_step(s, net, n, nullptr, s->d_h[0], s->d_tb, nullptr, nullptr, none, loss))) return st;
   JSC_CUDA_TRY(cudaDeviceSynchronize());
   if (grads) {
     size_t o = 0;
@@ -768,6 +640,8 @@ extern "C" int jsc_surrogate_train(jsc_surrogate *s, const float *X, const doubl
     st = JSC_ERR_CUDA;
   int *perm = (int *)malloc((size_t)n * sizeof(int));
   if (!perm) st = st ? st : JSC_ERR_NOMEM;
+  const TrainNet net = train_net(s);
+  if (!st) st = train_begin(net);
   uint64_t rs = seed;
   const float b1 = 0.9f, b2 = 0.999f;
   for (int ep = 0; ep < epochs && !st; ep++) {
@@ -788,24 +662,23 @@ extern "C" int jsc_surrogate_train(jsc_surrogate *s, const float *X, const doubl
       break;
     }
     for (int64_t b0 = 0; b0 + batch <= n && !st; b0 += batch) {
-      gather_kernel<<<batch, 32>>>(batch, nd, s->d_perm + b0, s->d_X, s->d_T, d_xm, d_xs,
-                                   s->d_h[0], s->d_tb);
       const bool last = b0 + 2 * batch > n;
       float l = 0;
-      st = forward_backward(s, batch, 0, last ? &l : nullptr);
+      s->adam_t++;
+      TrainAdam a;
+      a.on = 1;
+      a.lr = lr_ep;
+      a.b1 = b1;
+      a.b2 = b2;
+      a.c1 = 1 - powf(b1, (float)s->adam_t);
+      a.c2 = 1 - powf(b2, (float)s->adam_t);
+      a.eps = 1e-8f;
+      st = train_step(s, net, batch, s->d_perm + b0, s->d_X, s->d_T, d_xm, d_xs, a,
+                      last ? &l : nullptr);
       if (last) {
         ep_loss += l;
         ep_n++;
       }
-      s->adam_t++;
-      const float c1 = 1 - powf(b1, (float)s->adam_t), c2 = 1 - powf(b2, (float)s->adam_t);
-      for (int l2 = 0; l2 < 4 && !st; l2++)
-        for (int j = 0; j < 2; j++) {
-          const int64_t cnt = j ? s->out[l2] : (int64_t)s->out[l2] * s->in[l2];
-          adam_kernel<<<(unsigned)((cnt + 255) / 256), 256>>>(cnt, s->d_p[l2][j], s->d_g[l2][j],
-                                                              s->d_m[l2][j], s->d_v[l2][j], lr_ep,
-                                                              b1, b2, c1, c2, 1e-8f);
-        }
     }
     if (!st) {
       cudaError_t e = cudaDeviceSynchronize();

@@ -223,3 +223,29 @@ def test_gas_variants_on_irregular_tables(workdir, kind):
     for k in want:
         np.testing.assert_array_equal(four[k], want[k])
         np.testing.assert_array_equal(one[k], want[k])
+
+
+@pytest.mark.parametrize("n,nd", [(1, 1), (31, 5), (32, 16), (33, 3), (64, 64), (129, 33), (1000, 16), (4159, 7)])
+def test_training_gradients_at_tile_edges(n, nd):
+    """Gradients of one minibatch against the FP64 restatement at batches
+    around the row tiles (32), the slices (64) and their remainders, and
+    output widths that are no multiple of four.  Bounds as in the gradient
+    check of the surrogate's tests: FP32 sums of n products, relative to the
+    largest gradient."""
+    from jscat import api
+    from oracle import mlp_ref
+    rng = np.random.default_rng(n * 100 + nd)
+    s = api.Surrogate(nd=nd, seed=3)
+    try:
+        p = s.get_params()
+        p = (p + rng.normal(0, 0.05, p.shape)).astype(np.float32)
+        s.set_params(p)
+        x = rng.normal(0, 1, (n, 8)).astype(np.float32)
+        t = rng.normal(0, 1, (n, nd)).astype(np.float32)
+        loss, g = s.loss_grad(x, t)
+        ref_loss, ref_g = mlp_ref.loss_and_grads(s.layers(p.astype(np.float64)), x, t)
+        assert abs(loss - ref_loss) <= 1e-4 * abs(ref_loss)
+        flat = np.concatenate([np.concatenate([gw.ravel(), gb]) for gw, gb in ref_g])
+        assert np.max(np.abs(g - flat)) <= 2e-4 * np.max(np.abs(flat))
+    finally:
+        s.close()
