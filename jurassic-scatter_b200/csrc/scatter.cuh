@@ -319,23 +319,32 @@ static __global__ void __launch_bounds__(JSC_INT1_THREADS, 4) sp_integral_kernel
     const int row = tid * JSC_INT1_SL, m = even ? JSC_NPHI_SCA / 2 : JSC_NPHI_SCA;
     int lo = 0, n = 0;
     double s = 0;
-    for (int iq = 0; iq < m; iq++) {
-      double c = c1 * cph[iq] + c0;
-      if (!even) c += c2 * sin(2. * (0.5 + iq) * M_PI / 180.);
-      const double alpha2 = acos(fmin(fmax(c, -1.0), 1.0));
-      // locate(alpha, nalpha, alpha2) from the interval before
-      int l = lo;
-      while (l < na - 2 && !(alf[l + 1] > alpha2)) l++;
-      while (l > 0 && alf[l] > alpha2) l--;
-      if (l != lo) {
-        ss[row + lo] += s;
-        sn[row + lo] += (unsigned char)n;
-        s = 0;
-        n = 0;
-        lo = l;
+    // three azimuths at a time: their acos run in parallel and share constants
+    static_assert(JSC_NPHI_SCA / 2 % 3 == 0, "azimuths");
+    for (int iq = 0; iq < m; iq += 3) {
+      double al[3];
+#pragma unroll
+      for (int q = 0; q < 3; q++) al[q] = c1 * cph[iq + q] + c0;
+      if (!even)
+        for (int q = 0; q < 3; q++) al[q] += c2 * sin(2. * (0.5 + (iq + q)) * M_PI / 180.);
+#pragma unroll
+      for (int q = 0; q < 3; q++) al[q] = acos(fmin(fmax(al[q], -1.0), 1.0));
+#pragma unroll
+      for (int q = 0; q < 3; q++) {
+        // locate(alpha, nalpha, alpha2) from the interval before
+        int l = lo;
+        while (l < na - 2 && !(alf[l + 1] > al[q])) l++;
+        while (l > 0 && alf[l] > al[q]) l--;
+        if (l != lo) {
+          ss[row + lo] += s;
+          sn[row + lo] += (unsigned char)n;
+          s = 0;
+          n = 0;
+          lo = l;
+        }
+        s += al[q] - alf[l];
+        n++;
       }
-      s += alpha2 - alf[l];
-      n++;
     }
     ss[row + lo] += s;
     sn[row + lo] += (unsigned char)n;
