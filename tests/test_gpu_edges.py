@@ -249,3 +249,57 @@ def test_training_gradients_at_tile_edges(n, nd):
         assert np.max(np.abs(g - flat)) <= 2e-4 * np.max(np.abs(flat))
     finally:
         s.close()
+
+
+def _mie_numpy(x, m):
+    """Q_ext, Q_sca and phase function of spheres (Bohren and Huffman 1983,
+    appendix A, whose downward recurrence starts 15 orders above the larger
+    of the last order and |x m|), all orders of all spheres at once."""
+    nstop = (x + 4 * x ** 0.3333 + 2).astype(int)
+    nmx = (np.maximum(x + 4 * x ** 0.3333 + 2, np.abs(x * m)) + 15).astype(int)
+    d = np.zeros((nmx.max() + 1, len(x)), complex)
+    for n in range(nmx.max(), 1, -1):
+        d[n - 1] = np.where(n <= nmx, n / (x * m) - 1 / (d[n] + n / (x * m)), 0)
+    mu = np.cos(np.radians(np.arange(181.0)))[:, None]
+    p0, p1 = np.zeros((181, 1)), np.ones((181, 1))
+    s1, s2 = np.zeros((181, len(x)), complex), np.zeros((181, len(x)), complex)
+    psi0, psi1, chi0, chi1, q = np.cos(x), np.sin(x), -np.sin(x), np.cos(x), np.zeros(len(x))
+    for n in range(1, int(nstop.max()) + 1):
+        use = n <= nstop
+        with np.errstate(all="ignore"):
+            psi, chi = (2 * n - 1) * psi1 / x - psi0, (2 * n - 1) * chi1 / x - chi0
+            xi, xi1 = psi - 1j * chi, psi1 - 1j * chi1
+            a = ((d[n] / m + n / x) * psi - psi1) / ((d[n] / m + n / x) * xi - xi1)
+            b = ((d[n] * m + n / x) * psi - psi1) / ((d[n] * m + n / x) * xi - xi1)
+        a, b = np.where(use, a, 0), np.where(use, b, 0)
+        psi0, psi1 = psi1, np.where(use, psi, psi1)
+        chi0, chi1 = chi1, np.where(use, chi, chi1)
+        f, t = (2 * n + 1) / (n * (n + 1)), n * mu * p1 - (n + 1) * p0
+        s1, s2 = s1 + f * (a * p1 + b * t), s2 + f * (a * t + b * p1)
+        q += (2 * n + 1) * (np.abs(a) ** 2 + np.abs(b) ** 2)
+        p0, p1 = p1, ((2 * n + 1) * mu * p1 - (n + 1) * p0) / n
+    qs = 2 / x ** 2 * q
+    return 4 / x ** 2 * s1[0].real, qs, 2 / (x * x * qs) * (np.abs(s1) ** 2 + np.abs(s2) ** 2)
+
+
+@pytest.mark.parametrize("nr,ni", [(1.31, 0.0), (1.45, 1e-3), (2.5, 1.2)])
+def test_mie_series_at_its_ends(nr, ni):
+    """The Mie kernel's series against numpy from one order to some hundred
+    and at odd and even last orders, without and with absorption.  1e-10 of
+    the phase function's largest value: the recurrences lose about as many
+    bits as they have hundreds of orders, from 2e-16."""
+    import ctypes as C
+    from jscat import lib as L
+    lib = L.load()
+    lib.jsc_mie_eval.restype = C.c_int
+    x = np.concatenate([np.logspace(-3, 0, 9), np.arange(1.0, 12.0, 0.5), [63.2, 64.8, 127.1, 300.3, 701.0]])
+    n = len(x)
+    out = np.empty((n, 183))
+    arr = [np.ascontiguousarray(v, dtype=np.float64) for v in (x, np.full(n, nr), np.full(n, ni))]
+    dp = C.POINTER(C.c_double)
+    assert lib.jsc_mie_eval(0, n, *[a.ctypes.data_as(dp) for a in arr], out.ctypes.data_as(dp)) == 0
+    qe, qs, ph = _mie_numpy(x, np.full(n, nr + 1j * ni))
+    assert max_rel(out[:, 1], qs) <= 1e-10
+    big = x > 0.05          # extinction of a tiny sphere cancels to its last bits
+    assert max_rel(out[big, 0], qe[big]) <= 1e-10
+    assert np.max(np.abs(out[:, 2:] - ph.T) / ph.T.max(axis=1, keepdims=True)) <= 1e-10
