@@ -911,7 +911,7 @@ static int list_scattering_points(jsc_batch *b, cudaStream_t s) {
   sa.status = b->d_status;
   sa.n_listed = nullptr;
   sa.sp_idx = nullptr;
-  sp_count_kernel<<<(nr + 127) / 128, 128, 0, s>>>(sa);
+  sp_count_kernel<<<(nr + 3) / 4, 128, 0, s>>>(sa);
   JSC_LAUNCH_CHECK();
   if ((st = launch_scan(b, b->d_nsp, nr, b->d_sp_off, s))) return st;
   JSC_CUDA_TRY(cudaMemcpyAsync(b->h_total, b->d_sp_off + nr, sizeof(int64_t),
@@ -924,7 +924,7 @@ static int list_scattering_points(jsc_batch *b, cudaStream_t s) {
   sa.sp = b->d_sp;
   sa.sp_atm = b->d_sp_atm;
   sa.sp_idx = b->d_sp_idx;
-  sp_list_kernel<<<(nr + 127) / 128, 128, 0, s>>>(sa);
+  sp_list_kernel<<<(nr + 3) / 4, 128, 0, s>>>(sa);
   JSC_LAUNCH_CHECK();
   return JSC_OK;
 }
@@ -1134,12 +1134,12 @@ static int fixed_sources(jsc_batch *b, cudaStream_t s) {
   sa.status = b->d_status;
   sa.n_listed = b->d_sp_listed;
   sa.sp_idx = b->d_sp_idx;
-  sp_count_kernel<<<(nr + 127) / 128, 128, 0, s>>>(sa);
+  sp_count_kernel<<<(nr + 3) / 4, 128, 0, s>>>(sa);
   JSC_LAUNCH_CHECK();
   if ((st = launch_scan(b, b->d_nsp, nr, b->d_sp_off, s))) return st;
   sp_listed_init_kernel<<<1, 1, 0, s>>>(b->d_sp_off + nr, b->fx_max_sp, b->d_sp_listed);
   JSC_LAUNCH_CHECK();
-  sp_list_kernel<<<(nr + 127) / 128, 128, 0, s>>>(sa);
+  sp_list_kernel<<<(nr + 3) / 4, 128, 0, s>>>(sa);
   JSC_LAUNCH_CHECK();
   if ((st = copy_profiles(b, b->child, s))) return st;
   if ((st = copy_profiles(b, b->sun_child, s))) return st;
