@@ -534,7 +534,8 @@ static __global__ void __launch_bounds__(128) tangent_kernel(ExpandArgs A) {
 // steps.  Bound by instruction issue; with the crossings in the lane of
 // their segment, every function inlined and the tangent point in lane 0 the
 // warps waited for instructions (9.9 of 17 cycles an issue, 11.7 lanes
-// active), 9.6 ms for 232,000 pencils, now 3.2.
+// active), 9.6 ms for 232,000 pencils, 3.28 after that, 3.03 since the last lane
+// no longer converts its following point by itself.
 template <bool EDGES>
 __global__ void __launch_bounds__(128, 6) expand_kernel(const __grid_constant__ ExpandArgs A) {
   const int r = (int)(((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
@@ -658,28 +659,28 @@ __global__ void __launch_bounds__(128, 6) expand_kernel(const __grid_constant__ 
   __syncwarp();  // the geometry written above, for every lane
   const double *go = A.geo + base * 4;
   double carry[3] = {0, 0, 0};  // position of the point before the 32
+  // Position of output point i.  The next 32 are converted ahead, so that the
+  // last lane has its following point without a conversion of its own.
+  auto position = [&](int i) {
+    return i < o ? cart_of(go[(size_t)i * 4], go[(size_t)i * 4 + 1], go[(size_t)i * 4 + 2])
+                 : Vec3{{0, 0, 0}};
+  };
+  Vec3 xq = position(lane);
 #pragma unroll 1
   for (int i0 = 0; i0 < o; i0 += 32) {
     const int i = i0 + lane;
-    double xp[3], xn[3], z = 0;
-    Vec3 xc = {{0, 0, 0}};
-    if (i < o) {
-      z = go[(size_t)i * 4];
-      xc = cart_of(z, go[(size_t)i * 4 + 1], go[(size_t)i * 4 + 2]);
-    }
+    double xp[3], xn[3];
+    const Vec3 xc = xq;
+    xq = position(i + 32);
     for (int c = 0; c < 3; c++) {
       const double up = __shfl_up_sync(full, xc.v[c], 1);
-      const double dn = __shfl_down_sync(full, xc.v[c], 1);
       xp[c] = lane == 0 ? carry[c] : up;
-      xn[c] = dn;
+      // lane 0 hands the first of the next 32 to lane 31
+      xn[c] = __shfl_sync(full, lane == 0 ? xq.v[c] : xc.v[c], (lane + 1) & 31);
       carry[c] = __shfl_sync(full, xc.v[c], 31);
     }
-    if (lane == 31 && i + 1 < o) {
-      const Vec3 x = cart_of(go[(size_t)(i + 1) * 4], go[(size_t)(i + 1) * 4 + 1],
-                             go[(size_t)(i + 1) * 4 + 2]);
-      for (int c = 0; c < 3; c++) xn[c] = x.v[c];
-    }
     if (i < o) {
+      const double z = go[(size_t)i * 4];
       // chord step (src/lineofsight.c:300-330)
       double ds = 0;
       if (o > 1) {
