@@ -566,6 +566,60 @@ extern "C" int jsc_surrogate_loss_grad(jsc_surrogate *s, const float *x, const f
   return JSC_OK;
 }
 
+// Training set to the device: features as they are, the logarithms of the
+// sources standardised; the standardisations and the envelope of the features.
+static int standardise(jsc_surrogate *s, const float *X, const double *src, int64_t n) {
+  const int nd = s->nout;
+  const int64_t cnt = n * nd;
+  const int nblk = (int)(n < TR_STAT_BLOCKS ? n : TR_STAT_BLOCKS);
+  double fx[TR_STATS][SUR_NF], fy[TR_STATS * SUR_NOUT_MAX];
+  double *y = nullptr;  // logarithms, then the statistics' parts and sums
+  int st = jsc_dmalloc(&y, (size_t)cnt + (size_t)(nblk + 1) * TR_STATS * SUR_NOUT_MAX);
+  if (st) return st;
+  double *part = y + cnt, *sum = part + (size_t)nblk * TR_STATS * SUR_NOUT_MAX;
+  auto stats = [&](int nc, double *out) {  // parts to host sums
+    train_stats_sum_kernel<<<1, TR_STATS * SUR_NOUT_MAX>>>(nblk, nc, part, sum);
+    return cudaGetLastError() ||
+           cudaMemcpy(out, sum, (size_t)TR_STATS * nc * sizeof(double), cudaMemcpyDeviceToHost);
+  };
+  bool bad = cudaMemcpy(s->d_X, X, (size_t)n * SUR_NF * sizeof(float), cudaMemcpyHostToDevice);
+  if (!bad) {
+    train_stats_kernel<float, false><<<nblk, TR_THREADS>>>(n, SUR_NF, s->d_X, part);
+    bad = stats(SUR_NF, fx[0]);
+  }
+  bad = bad || cudaMemcpy(y, src, (size_t)cnt * sizeof(double), cudaMemcpyHostToDevice);
+  if (!bad) {
+    train_stats_kernel<double, true><<<nblk, TR_THREADS>>>(n, nd, y, part);
+    bad = stats(nd, fy);
+  }
+  if (!bad) {
+    for (int c = 0; c < SUR_NF; c++) {
+      const double m = fx[0][c] / n, var = fx[1][c] / n - m * m;
+      const float lo = (float)fx[2][c], hi = (float)fx[3][c], w = 0.02f * (hi - lo);
+      s->xm[c] = (float)m;
+      s->xs[c] = var > 1e-12 ? (float)sqrt(var) : 1.f;
+      s->lo[c] = lo - w;
+      s->hi[c] = hi + w;
+    }
+    for (int d = 0; d < nd; d++) {
+      const double m = fy[d] / n, var = fy[nd + d] / n - m * m;
+      fy[d] = m;
+      s->h_ym[d] = (float)m;
+      s->h_ys[d] = var > 1e-12 ? (float)sqrt(var) : 1.f;
+    }
+    bad = cudaMemcpy(sum, fy, nd * sizeof(double), cudaMemcpyHostToDevice) ||
+          cudaMemcpy(s->d_ym, s->h_ym, nd * sizeof(float), cudaMemcpyHostToDevice) ||
+          cudaMemcpy(s->d_ys, s->h_ys, nd * sizeof(float), cudaMemcpyHostToDevice);
+  }
+  if (!bad) {
+    train_targets_kernel<<<(unsigned)((cnt + TR_THREADS - 1) / TR_THREADS), TR_THREADS>>>(
+        cnt, nd, y, sum, s->d_ys, s->d_T);
+    bad = cudaGetLastError() || cudaDeviceSynchronize();
+  }
+  cudaFree(y);
+  return bad ? JSC_ERR_CUDA : JSC_OK;
+}
+
 extern "C" int jsc_surrogate_train(jsc_surrogate *s, const float *X, const double *src,
                                    int64_t n, int epochs, int batch, float lr, uint64_t seed,
                                    float *loss_per_epoch) {
@@ -576,44 +630,6 @@ extern "C" int jsc_surrogate_train(jsc_surrogate *s, const float *X, const doubl
   JSC_CUDA_TRY(cudaSetDevice(s->device));
   const int nd = s->nout;
   // Standardisation and envelope from the training set.
-  double sum[SUR_NF] = {0}, sum2[SUR_NF] = {0};
-  float lo[SUR_NF], hi[SUR_NF];
-  for (int c = 0; c < SUR_NF; c++) {
-    lo[c] = INFINITY;
-    hi[c] = -INFINITY;
-  }
-  for (int64_t i = 0; i < n; i++)
-    for (int c = 0; c < SUR_NF; c++) {
-      const float v = X[i * SUR_NF + c];
-      sum[c] += v;
-      sum2[c] += (double)v * v;
-      if (v < lo[c]) lo[c] = v;
-      if (v > hi[c]) hi[c] = v;
-    }
-  for (int c = 0; c < SUR_NF; c++) {
-    const double m = sum[c] / n, var = sum2[c] / n - m * m;
-    s->xm[c] = (float)m;
-    s->xs[c] = var > 1e-12 ? (float)sqrt(var) : 1.f;
-    const float w = 0.02f * (hi[c] - lo[c]);
-    s->lo[c] = lo[c] - w;
-    s->hi[c] = hi[c] + w;
-  }
-  float *T = (float *)malloc((size_t)n * nd * sizeof(float));
-  if (!T) return JSC_ERR_NOMEM;
-  for (int d = 0; d < nd; d++) {
-    double m = 0, m2 = 0;
-    for (int64_t i = 0; i < n; i++) {
-      const double y = log(fmax(src[i * nd + d], 1e-300));
-      m += y;
-      m2 += y * y;
-    }
-    m /= n;
-    const double var = m2 / n - m * m;
-    s->h_ym[d] = (float)m;
-    s->h_ys[d] = var > 1e-12 ? (float)sqrt(var) : 1.f;
-    for (int64_t i = 0; i < n; i++)
-      T[i * nd + d] = (float)((log(fmax(src[i * nd + d], 1e-300)) - m) / s->h_ys[d]);
-  }
   int st = JSC_OK;
   cudaFree(s->d_X);
   cudaFree(s->d_T);
@@ -623,12 +639,7 @@ extern "C" int jsc_surrogate_train(jsc_surrogate *s, const float *X, const doubl
   st = st ? st : jsc_dmalloc(&s->d_X, (size_t)n * SUR_NF);
   st = st ? st : jsc_dmalloc(&s->d_T, (size_t)n * nd);
   st = st ? st : jsc_dmalloc(&s->d_perm, (size_t)n);
-  if (!st && (cudaMemcpy(s->d_X, X, (size_t)n * SUR_NF * sizeof(float), cudaMemcpyHostToDevice) ||
-              cudaMemcpy(s->d_T, T, (size_t)n * nd * sizeof(float), cudaMemcpyHostToDevice) ||
-              cudaMemcpy(s->d_ym, s->h_ym, nd * sizeof(float), cudaMemcpyHostToDevice) ||
-              cudaMemcpy(s->d_ys, s->h_ys, nd * sizeof(float), cudaMemcpyHostToDevice)))
-    st = JSC_ERR_CUDA;
-  free(T);
+  st = st ? st : standardise(s, X, src, n);
   if (st) return st;
   s->n_train = n;
   if ((st = ensure_train(s, batch))) return st;

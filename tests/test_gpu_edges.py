@@ -251,6 +251,36 @@ def test_training_gradients_at_tile_edges(n, nd):
         s.close()
 
 
+@pytest.mark.parametrize("n,nd", [(16, 1), (297, 3), (1000, 16), (4099, 64)])
+def test_training_set_standardisation(n, nd):
+    """Loss of the untrained network on the whole training set, whose targets
+    are the standardised logarithms: against numpy in 64 bits, at sample
+    counts below, at and past the rows of the statistics' blocks.  Tolerance:
+    three sums of 128 products in FP32 (3 x 128 x 2^-24)."""
+    from jscat import api
+    rng = np.random.default_rng(n)
+    x = (rng.normal(size=(n, 8)) * 10.0 ** np.arange(-3, 5)).astype(np.float32)
+    x[:, 3] = 7.25                                 # a feature without spread
+    src = np.exp(rng.normal(size=(n, nd)) - 30.0)
+    src[0, 0] = 0.0                                # bounded below
+    sur = api.Surrogate(nd, seed=3)
+    got = sur.train(x, src, epochs=1, batch=n, lr=0.0)
+    par = sur.get_params().astype(np.float64)
+    sur.close()
+    h = x.astype(np.float64)
+    sd = h.std(0)
+    h = (h - h.mean(0)) / np.where(sd * sd > 1e-12, sd, 1.0)
+    y = np.log(np.maximum(src, 1e-300))
+    y = (y - y.mean(0)) / y.std(0)
+    o = 0
+    for k, (a, b) in enumerate(((8, 128), (128, 128), (128, 128), (128, nd))):
+        h = h @ par[o:o + a * b].reshape(b, a).T + par[o + a * b:o + a * b + b]
+        o += a * b + b
+        h = np.tanh(h) if k < 3 else h
+    want = ((h - y) ** 2).sum() / n
+    assert abs(got[0] - want) <= 3 * 128 * 2.0 ** -24 * want
+
+
 def _mie_numpy(x, m):
     """Q_ext, Q_sca and phase function of spheres (Bohren and Huffman 1983,
     appendix A, whose downward recurrence starts 15 orders above the larger
