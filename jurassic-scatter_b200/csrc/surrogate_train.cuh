@@ -1,4 +1,4 @@
-// Training step of the surrogate in three launches (FP32, no contraction):
+// Training step of the surrogate in three launches (FP32):
 //
 //   train_rows_kernel    a block per 32 samples: minibatch gather, forward,
 //                        loss gradient and the gradients of every layer's
@@ -11,8 +11,9 @@
 // train_targets_kernel standardise the training set.
 //
 // Every sum runs in the order of a plain product (the inner index upwards,
-// slices of the samples in order, bias sums over eight interleaved rows), so
-// training is deterministic and does not depend on the tiling.
+// slices of the samples in order, bias sums over eight interleaved rows; the
+// products of the contractions are fused into their sums), so training is
+// deterministic and does not depend on the tiling.
 #pragma once
 #include <math.h>
 #include <stdint.h>
@@ -99,17 +100,18 @@ __device__ __forceinline__ void rows_product(const float *a, const float *B, int
 #pragma unroll
         for (int i = 0; i < 4; i++)
 #pragma unroll
-          for (int j = 0; j < 4; j++) acc[i][j] += as[i] * bs[j];
+          for (int j = 0; j < 4; j++) acc[i][j] = fmaf(as[i], bs[j], acc[i][j]);
       }
     }
   }
   __syncthreads();  // a and the tiles may be rewritten
 }
 
-// Bound by the FP32 pipes (two instructions a product): 51 us of a step of
-// 4096 samples on 128 SMs, 30 us at their full rate.  The step took 330 us
-// in 35 launches, most of it products of 64 x 64 tiles of which each layer
-// fills a few blocks and bias sums in one to four blocks; now 87 us in three.
+// Bound by the latency of its shared-memory operands, eight warps on each of
+// 128 SMs: 43 us of a step of 4096 samples, 15 us at the full FP32 rate; with
+// a multiplication and an addition per product it took 51.  The step took 330
+// us in 35 launches, most of it products of 64 x 64 tiles of which each layer
+// fills a few blocks and bias sums in one to four blocks; now 75 us in three.
 static __global__ void __launch_bounds__(TR_THREADS) train_rows_kernel(TrainNet net, TrainBatch b) {
   extern __shared__ __align__(16) float tr_sh[];
   float *ht[4];                                    // inputs of the layers, [in][TR_LD]
@@ -258,8 +260,8 @@ train_weights_kernel(TrainNet net, TrainBatch b, int ncol, int kchunk, float *ws
       const int o = threadIdx.x >> 2, i = (threadIdx.x & 3) * 2;
       for (int k = 0; k < m; k++) {
         const float a = as[k][o];
-        acc[0][0] += a * bs[k][i];
-        acc[0][1] += a * bs[k][i + 1];
+        acc[0][0] = fmaf(a, bs[k][i], acc[0][0]);
+        acc[0][1] = fmaf(a, bs[k][i + 1], acc[0][1]);
       }
     } else if (ty * 4 < no) {
 #pragma unroll 4
@@ -270,7 +272,7 @@ train_weights_kernel(TrainNet net, TrainBatch b, int ncol, int kchunk, float *ws
 #pragma unroll
         for (int i = 0; i < 4; i++)
 #pragma unroll
-          for (int j = 0; j < 4; j++) acc[i][j] += aa[i] * bb[j];
+          for (int j = 0; j < 4; j++) acc[i][j] = fmaf(aa[i], bb[j], acc[i][j]);
       }
     }
   }
@@ -366,7 +368,7 @@ static __global__ void __launch_bounds__(TR_THREADS) train_loss_kernel(int64_t c
 // and rows of a block's slice, so loads are contiguous; sums in FP64 in a
 // fixed order.  Bound by the read and write, 10 us for 65536 samples x 16
 // channels (sums over the blocks 20 us, targets 5); with two passes of logarithms on the host a training of 8
-// epochs on that set took 39 ms, now 22.
+// epochs on that set took 39 ms, with this 22.
 template <typename T, bool LOG>
 static __global__ void __launch_bounds__(TR_THREADS)
 train_stats_kernel(int64_t n, int nc, T *v, double *part) {
