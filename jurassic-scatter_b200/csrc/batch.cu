@@ -1001,8 +1001,10 @@ static const int64_t kScatterChunk3 = 16;
 // Polar weights of the layers' phase functions for the source integrals.
 static int polar_weights(jsc_batch *b, cudaStream_t s) {
   const int nd = b->cfg.nd;
-  JSC_CUDA_TRY(cudaFuncSetAttribute(sp_integral_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    JSC_INT1_SHMEM));
+  JSC_CUDA_TRY(cudaFuncSetAttribute(sp_integral_kernel<8>,
+                                    cudaFuncAttributeMaxDynamicSharedMemorySize, JSC_INT1_SHMEM));
+  JSC_CUDA_TRY(cudaFuncSetAttribute(sp_integral_kernel<16>,
+                                    cudaFuncAttributeMaxDynamicSharedMemorySize, JSC_INT1_SHMEM));
   if (b->aero_nl < 1) return JSC_OK;
   sp_weights_kernel<<<dim3(nd, b->aero_nl), JSC_INT1_THREADS, 0, s>>>(
       nd, b->d_phase, b->d_wt, b->d_wt + (size_t)b->aero_nl * JSC_NTH_SCA * nd);
@@ -1098,7 +1100,7 @@ static int plain_sources(jsc_batch *b, const double *sp, const int *sp_atm, int6
     ia.wt = b->d_wt;
     ia.wsum = b->d_wt + (size_t)b->aero_nl * JSC_NTH_SCA * nd;
     ia.src = src + c0 * nd;
-    sp_integral_kernel<<<n, JSC_INT1_THREADS, JSC_INT1_SHMEM, s>>>(ia);
+    sp_integral_launch(ia, n, s);
     JSC_LAUNCH_CHECK();
     if ((st = sun_sources(b, pa.sp, pa.sp_atm, n, src + c0 * nd, s))) return st;
   }
@@ -1180,7 +1182,7 @@ static int fixed_sources(jsc_batch *b, cudaStream_t s) {
     ia.wt = b->d_wt;
     ia.wsum = b->d_wt + (size_t)b->aero_nl * JSC_NTH_SCA * nd;
     ia.src = b->d_src + c0 * nd;
-    sp_integral_kernel<<<chunk, JSC_INT1_THREADS, JSC_INT1_SHMEM, s>>>(ia);
+    sp_integral_launch(ia, chunk, s);
     JSC_LAUNCH_CHECK();
     if ((st = sun_sources(b, pa.sp, pa.sp_atm, chunk, b->d_src + c0 * nd, s, n_total, c0)))
       return st;

@@ -225,9 +225,9 @@ static __global__ void sp_spawn_kernel(SpawnArgs A) {
 
 #define JSC_INT_THREADS 256    // sp_integral3_kernel
 #define JSC_INT_CH 16          // channels per pass over the directions
-#define JSC_INT1_THREADS 192   // sp_integral_kernel: a thread per polar step, 12 groups of 16
+#define JSC_INT1_THREADS 192   // sp_integral_kernel: a thread per polar step, 12 groups of 16 (20 of 8)
 #define JSC_INT1_SL 29         // odd row stride of the interval sums (28 pencils, 27 intervals)
-static_assert(JSC_INT1_THREADS >= JSC_NTH_SCA && JSC_INT1_THREADS % JSC_INT_CH == 0, "block shape");
+static_assert(JSC_INT1_THREADS >= JSC_NTH_SCA, "block shape");
 static_assert(JSC_INT1_SL >= JSC_NALPHA_REF, "interval sums");
 
 // Polar weights sin(theta2) phase(theta2) of layer blockIdx.y and channel
@@ -282,17 +282,26 @@ struct IntegralArgs {
 // 32,400 directions.  The zenith has no component across the plane of the
 // zenith and the line of sight, so alpha is even in the azimuth and half of
 // it suffices (all of it should the component exceed rounding).
-// Bound by the FP64 acos of 16,200 directions a point.  Evaluating every
+// A direction and its opposite share one acos, which leaves 8100 a point.
+// Bound by instruction issue at 24 warps an SM (four blocks of 56 KB shared
+// memory; at three blocks, with an acos for every direction and passes of 16
+// channels only, 1.52 and 11.2 ms in the two cases below).  Evaluating every
 // channel in every direction took 9.0 ms for 11,600 points of 16 channels
-// and 61.8 ms for a depth-2 batch of 12 rays, this form 1.7 and 12.6.
+// and 61.8 ms for a depth-2 batch of 12 rays and 8 channels, this form 1.03
+// and 8.0.
 #define JSC_INT1_SHMEM (JSC_NTH_SCA * JSC_INT1_SL * 9)
 
-static __global__ void __launch_bounds__(JSC_INT1_THREADS, 4) sp_integral_kernel(IntegralArgs A) {
+template <int CH>
+__global__ void __launch_bounds__(JSC_INT1_THREADS, 4) sp_integral_kernel(IntegralArgs A) {
   extern __shared__ double ss[];  // [180][JSC_INT1_SL] sums of alpha - alpha[lo]
   unsigned char *sn =             // [180][JSC_INT1_SL] directions (at most 180)
       reinterpret_cast<unsigned char *>(ss + JSC_NTH_SCA * JSC_INT1_SL);
-  __shared__ double rd[JSC_NALPHA_REF][JSC_INT_CH], slp[JSC_NALPHA_REF][JSC_INT_CH];
-  __shared__ double cph[JSC_NPHI_SCA], alf[JSC_NALPHA_MAX];
+  // radiances and slopes of the pencils; before, the azimuths' cosines (with
+  // an array of their own only three blocks fit an SM)
+  __shared__ double rd[JSC_NALPHA_REF][CH], slp[JSC_NALPHA_REF][CH];
+  static_assert(JSC_NALPHA_REF * CH >= JSC_NPHI_SCA, "azimuths");
+  double *cph = &rd[0][0];
+  __shared__ double alf[JSC_NALPHA_MAX];
   __shared__ double red[JSC_INT1_THREADS];
   const int k = blockIdx.x;
   if (k >= live_points(A.n_total, A.first, A.n_pts)) return;
@@ -320,50 +329,75 @@ static __global__ void __launch_bounds__(JSC_INT1_THREADS, 4) sp_integral_kernel
   }
   const bool even = fabs(ax) <= 1e-14;
   __syncthreads();
-  if (tid < JSC_NTH_SCA) {
-    const double th = (0.5 + tid) * M_PI / 180.;
-    const double st = sin(th), ct = cos(th);
-    const double c1 = st * ay, c0 = ct * az, c2 = st * ax;
-    const int row = tid * JSC_INT1_SL, m = even ? JSC_NPHI_SCA / 2 : JSC_NPHI_SCA;
-    int lo = 0, n = 0;
-    double s = 0;
-    // three azimuths at a time: their acos run in parallel and share constants
-    static_assert(JSC_NPHI_SCA / 2 % 3 == 0, "azimuths");
-    for (int iq = 0; iq < m; iq += 3) {
+  // Polar step of this thread; the lanes 2 j and 2 j + 1 hold steps that are
+  // opposite, th and pi - th.
+  const int pol = tid & 1 ? JSC_NTH_SCA - 1 - (tid >> 1) : tid >> 1;
+  const double th = (0.5 + pol) * M_PI / 180.;
+  const double st = sin(th), ct = cos(th);
+  const double c1 = st * ay, c0 = ct * az, c2 = st * ax;
+  const int row = pol * JSC_INT1_SL;
+  // directions in the interval lo of the pencils, and the sum of their alpha
+  struct Run {
+    int lo, n;
+    double s;
+  };
+  auto store = [&](const Run &r) {
+    ss[row + r.lo] += r.s;
+    sn[row + r.lo] += (unsigned char)r.n;
+  };
+  auto add = [&](Run &r, double al) {
+    // locate(alpha, nalpha, alpha2) from the interval before
+    int l = r.lo;
+    while (l < na - 2 && !(alf[l + 1] > al)) l++;
+    while (l > 0 && alf[l] > al) l--;
+    if (l != r.lo) {
+      store(r);
+      r = Run{l, 0, 0};
+    }
+    r.s += al - alf[l];
+    r.n++;
+  };
+  const bool own = tid < JSC_NTH_SCA;
+  Run fwd = {0, 0, 0};
+  // three azimuths at a time: their acos run in parallel and share constants
+  static_assert(JSC_NPHI_SCA / 4 % 3 == 0 && JSC_NTH_SCA % 2 == 0, "azimuths");
+  if (even) {
+    // a direction's opposite lies in the other lane's polar step, at the
+    // azimuth pi - phi, with pi - alpha: one acos for the two
+    Run bwd = {0, 0, 0};
+    for (int iq = 0; iq < JSC_NPHI_SCA / 4; iq += 3) {
       double al[3];
 #pragma unroll
-      for (int q = 0; q < 3; q++) al[q] = c1 * cph[iq + q] + c0;
-      if (!even)
-        for (int q = 0; q < 3; q++) al[q] += c2 * sin(2. * (0.5 + (iq + q)) * M_PI / 180.);
-#pragma unroll
-      for (int q = 0; q < 3; q++) al[q] = acos(fmin(fmax(al[q], -1.0), 1.0));
+      for (int q = 0; q < 3; q++) al[q] = acos(fmin(fmax(c1 * cph[iq + q] + c0, -1.0), 1.0));
 #pragma unroll
       for (int q = 0; q < 3; q++) {
-        // locate(alpha, nalpha, alpha2) from the interval before
-        int l = lo;
-        while (l < na - 2 && !(alf[l + 1] > al[q])) l++;
-        while (l > 0 && alf[l] > al[q]) l--;
-        if (l != lo) {
-          ss[row + lo] += s;
-          sn[row + lo] += (unsigned char)n;
-          s = 0;
-          n = 0;
-          lo = l;
+        const double opp = M_PI - __shfl_xor_sync(0xffffffffu, al[q], 1);
+        if (own) {
+          add(fwd, al[q]);
+          add(bwd, opp);
         }
-        s += al[q] - alf[l];
-        n++;
       }
     }
-    ss[row + lo] += s;
-    sn[row + lo] += (unsigned char)n;
+    if (own) store(bwd);
+  } else if (own) {
+    for (int iq = 0; iq < JSC_NPHI_SCA; iq += 3) {
+      double al[3];
+#pragma unroll
+      for (int q = 0; q < 3; q++)
+        al[q] = c1 * cph[iq + q] + c0 + c2 * sin(2. * (0.5 + (iq + q)) * M_PI / 180.);
+#pragma unroll
+      for (int q = 0; q < 3; q++) al[q] = acos(fmin(fmax(al[q], -1.0), 1.0));
+      for (int q = 0; q < 3; q++) add(fwd, al[q]);
+    }
   }
-  const int c = tid & (JSC_INT_CH - 1), grp = tid / JSC_INT_CH;
-  constexpr int NG = JSC_INT1_THREADS / JSC_INT_CH, PER = JSC_NTH_SCA / NG;
-  static_assert(PER * NG == JSC_NTH_SCA, "polar steps per group");
-  for (int ch0 = 0; ch0 < nd; ch0 += JSC_INT_CH) {
+  if (own) store(fwd);
+  const int c = tid & (CH - 1), grp = tid / CH;
+  constexpr int NG = CH == 8 ? 20 : 12, PER = JSC_NTH_SCA / NG;
+  static_assert(PER * NG == JSC_NTH_SCA && NG * CH <= JSC_INT1_THREADS, "polar steps per group");
+  for (int ch0 = 0; ch0 < nd; ch0 += CH) {
     __syncthreads();
-    for (int i = tid; i < na * JSC_INT_CH; i += JSC_INT1_THREADS) {
-      const int lo = i / JSC_INT_CH, cc = i - lo * JSC_INT_CH;
+    for (int i = tid; i < na * CH; i += JSC_INT1_THREADS) {
+      const int lo = i / CH, cc = i - lo * CH;
       if (ch0 + cc < nd) {
         const double *r = A.rad + ((size_t)k * na + lo) * nd + ch0 + cc;
         rd[lo][cc] = r[0];
@@ -373,7 +407,7 @@ static __global__ void __launch_bounds__(JSC_INT1_THREADS, 4) sp_integral_kernel
     __syncthreads();
     double acc = 0;
     const int id = ch0 + c;
-    if (id < nd) {
+    if (id < nd && grp < NG) {
       double v[PER];  // polar steps grp, grp + NG, ... of this channel
 #pragma unroll
       for (int j = 0; j < PER; j++) v[j] = 0;
@@ -391,12 +425,21 @@ static __global__ void __launch_bounds__(JSC_INT1_THREADS, 4) sp_integral_kernel
     }
     red[tid] = acc;
     __syncthreads();
-    if (tid < JSC_INT_CH && id < nd) {
+    if (tid < CH && id < nd) {
       double t = 0;
-      for (int g = 0; g < NG; g++) t += red[g * JSC_INT_CH + c];
+      for (int g = 0; g < NG; g++) t += red[g * CH + c];
       A.src[(size_t)k * nd + id] = (even ? 2 * t : t) / A.wsum[(size_t)il * nd + id];
     }
   }
+}
+
+// Channels per pass: a pass of 8 takes 9 polar steps a thread, one of 16
+// takes 15, so 8 where that is less in all (up to 8 channels, and 17 to 24).
+static inline void sp_integral_launch(const IntegralArgs &ia, int blocks, cudaStream_t s) {
+  if ((ia.nd + 7) / 8 * 9 < (ia.nd + 15) / 16 * 15)
+    sp_integral_kernel<8><<<blocks, JSC_INT1_THREADS, JSC_INT1_SHMEM, s>>>(ia);
+  else
+    sp_integral_kernel<16><<<blocks, JSC_INT1_THREADS, JSC_INT1_SHMEM, s>>>(ia);
 }
 
 // ------------------------------------------------------------------ sun --

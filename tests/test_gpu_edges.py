@@ -161,6 +161,41 @@ def test_source_integral_against_port(workdir, nd, nalpha, layer):
     assert max_rel(got["tau"], ref["tau"]) <= 1e-9
 
 
+@pytest.mark.parametrize("nd", [7, 9, 17, 24, 25, 33])
+def test_source_integral_channel_passes(workdir, nd):
+    """Channel counts around the passes of 8 and 16: channels repeated from a
+    run of 16, whose radiances are compared with the C restatement above.
+    The passes add the same 180 polar steps of one sign in other groups:
+    180 x 2 x 2^-53."""
+    from jscat import api, synth, structs as S
+    g = np.load(os.path.join(GOLDEN, "aero_sulfate16.npz"))
+    full = S.AeroT.from_buffer_copy(g["aero"].tobytes())
+    all_nus = [float(v) for v in g["nus"]]
+    kw, atm, _ = _limb_inputs(workdir, np.arange(0.0, 121.0))
+    base = synth.write_tables(workdir, kw["emitters"], all_nus, 20261203)
+    geom = synth.limb_geometry([17.3, 12.1])
+    inp = synth.batch_from([atm], np.zeros(2, np.int32), geom)
+
+    def run(ch):
+        aero = S.AeroT.from_buffer_copy(bytes(full))
+        for il in range(full.nl):
+            for j, i in enumerate(ch):
+                aero.beta_e[il][j] = full.beta_e[il][i]
+                aero.beta_s[il][j] = full.beta_s[il][i]
+                aero.beta_a[il][j] = full.beta_a[il][i]
+                for a in range(181):
+                    aero.p[il][j][a] = full.p[il][i][a]
+        kw.update(nus=[all_nus[i] for i in ch], tblbase=base, sca_n=1, sca_mult=1, hydz=0.0,
+                  ctm_co2=0, ctm_h2o=0)
+        return api.formod_batch(S.make_ctl(**kw), inp, aero=aero, nalpha=20)
+
+    want, got = run(range(16)), run([i % 16 for i in range(nd)])
+    for k in ("rad", "tau"):
+        ref = want[k][:, [i % 16 for i in range(nd)]]
+        assert np.all(np.isfinite(ref)) and np.any(ref > 0)
+        assert max_rel(got[k], ref) <= 2 * 180 * 2.0 ** -53
+
+
 @pytest.mark.parametrize("ng,nd,n", [(1, 1, 1), (2, 3, 7), (3, 2, 8), (5, 4, 9), (8, 2, 33), (9, 2, 17), (16, 1, 8),
                                      (17, 2, 9), (25, 1, 5)])
 def test_window_variants_against_others(workdir, ng, nd, n):
