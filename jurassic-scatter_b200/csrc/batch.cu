@@ -221,7 +221,7 @@ extern "C" int jsc_batch_create(jsc_model *m, const ctl_t *ctl, int max_atm,
   if (b->ip == 1) {
     st = st ? st : jsc_dmalloc(&b->d_lev, 8 * (size_t)max_levels);
     st = st ? st : jsc_dmalloc(&b->d_qs, (size_t)(ctl->ng + ctl->nw) * max_levels);
-    st = st ? st : jsc_dmalloc(&b->d_mcount, 1);
+    st = st ? st : jsc_dmalloc(&b->d_mcount, 2);
   }
   b->scan_tiles = (max_rays + JSC_SCAN_TILE - 1) / JSC_SCAN_TILE + 1;
   st = st ? st : jsc_dmalloc(&b->d_scan, (size_t)b->scan_tiles + 1);
@@ -633,10 +633,13 @@ static int ray_warps(int ng) {
 }
 // Default launch variants: four lanes per ray up to kGasNarrow warps of one
 // lane per ray, one lane above; the ray-tile kernel for table grids with an
-// interval of no width and for tables above 4 GB.  The line: 1664 warps 1.09
-// ms with four lanes and 1.14 with one, 2016 warps 1.44 and 1.40 (limb rays,
-// 16 channels; with nadir rays between them, whose lanes then idle, it lies at
-// about 3500).
+// interval of no width and for tables above 4 GB.  One lane per ray takes as
+// long as its longest line of sight until the SMs are full, four lanes as
+// long as all points together, so short rays count by their length: the warps
+// are those of rays as long as the longest (by number where the host does not
+// know the lengths).  Four lanes / one lane, 16 x 4 or 8 x 2 channels x
+// emitters: limb rays 1850 warps 1.46 / 1.50 ms, 2220 1.79 / 1.64; limb and
+// nadir rays in turn 1500 1.14 / 1.37, 2007 1.47 / 1.53, 2509 1.79 / 1.66.
 static const int kEgaDefault = 21;
 static const int kEgaWide = 22;
 static const int kEgaNoWidths = 17;
@@ -647,7 +650,8 @@ static const int64_t kGasNarrow = 2048;
 static int run_variant(const jsc_batch *b) {
   int v = b->ega_variant;
   if (v < 0 || v >= kNumEgaVariants) {
-    const int64_t warps = ((int64_t)b->n_rays + 31) / 32 * b->cfg.nd * (b->cfg.ng > 0 ? b->cfg.ng : 1);
+    const int64_t rays = b->np_longest > 0 && !b->fixed ? b->n_points / b->np_longest : b->n_rays;
+    const int64_t warps = (rays + 31) / 32 * b->cfg.nd * (b->cfg.ng > 0 ? b->cfg.ng : 1);
     v = warps <= kGasNarrow ? kEgaDefault : kEgaWide;
   }
   return gas_variant(v) && !b->m->dv.grid_dt ? kEgaNoWidths : v;
@@ -1628,7 +1632,7 @@ static int los_profile(jsc_batch *b, bool refine, cudaStream_t s) {
     xa.M.cap = b->mcap;
     xa.M.first = nr;
     xa.max_seg = b->max_seg;
-    JSC_CUDA_TRY(cudaMemsetAsync(b->d_mcount, 0, sizeof(unsigned), s));
+    JSC_CUDA_TRY(cudaMemsetAsync(b->d_mcount, 0, 2 * sizeof(unsigned), s));
     if (b->d_live) {
       // rays the queue leaves alone keep no LOS and no surface; a persistent
       // grid pulls the others
@@ -1651,13 +1655,15 @@ static int los_profile(jsc_batch *b, bool refine, cudaStream_t s) {
     if ((st = launch_scan(b, b->d_nlos, nr, b->d_los_off, s))) return st;
     if (b->fixed) {
       *b->h_total = 0;
+      b->np_longest = 0;
       break;
     }
     unsigned *taken = (unsigned *)(b->h_total + 1);
     JSC_CUDA_TRY(cudaMemcpyAsync(b->h_total, b->d_los_off + nr, sizeof(int64_t),
                                  cudaMemcpyDeviceToHost, s));
-    JSC_CUDA_TRY(cudaMemcpyAsync(taken, b->d_mcount, sizeof(unsigned), cudaMemcpyDeviceToHost, s));
+    JSC_CUDA_TRY(cudaMemcpyAsync(taken, b->d_mcount, 2 * sizeof(unsigned), cudaMemcpyDeviceToHost, s));
     JSC_CUDA_TRY(cudaStreamSynchronize(s));
+    b->np_longest = (int)taken[1];
     if ((int64_t)*taken + nr <= b->mcap) break;
     // The pool was too small: the counts of the march are complete all the
     // same, so the next pass fits.
@@ -1692,6 +1698,7 @@ static int los_profile(jsc_batch *b, bool refine, cudaStream_t s) {
 static int los_geo(jsc_batch *b, bool refine, cudaStream_t s) {
   const jsc_model *m = b->m;
   const int nr = b->n_rays;
+  b->np_longest = 0;
   RayArgs ra;
   fill_ray_args(b, ra);
   if (m->n_grid == 1) {

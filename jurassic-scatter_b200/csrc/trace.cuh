@@ -25,7 +25,7 @@
 struct MarchPool {
   double *pts;      // [cap][JSC_CHUNK][JSC_CHUNK_REC]
   int *next;        // [cap] following chunk of the same ray, -1: none
-  unsigned *count;  // chunks taken beyond the first of each ray
+  unsigned *count;  // [2] chunks taken beyond the first of each ray; points of the longest ray
   int cap, first;   // chunks of the pool; chunks 0 .. first-1 are the rays' first ones
 };
 
@@ -280,6 +280,7 @@ __device__ __forceinline__ void march_one(const RayArgs &A, const MarchPool &M, 
   if (role == 0) {
     A.nlos[r] = np;
     A.tsurf[r] = tsurf;
+    if ((unsigned)np > *(volatile unsigned *)(M.count + 1)) atomicMax(M.count + 1, (unsigned)np);
     if (np == 0) {
       A.tp[r] = in.vpz;
       A.tp[A.n_rays + r] = in.vplon;

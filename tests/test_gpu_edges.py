@@ -218,6 +218,36 @@ def test_window_variants_against_others(workdir, ng, nd, n):
         np.testing.assert_array_equal(one[k], want[k])
 
 
+@pytest.mark.parametrize("n,variant", [(900, 21), (1500, 21), (3000, 22)])
+def test_default_variant_by_points(workdir, n, variant):
+    """Limb and nadir rays in turn on both sides of the rule: rays count by
+    their length against the longest, and either side gives the bits of the
+    other."""
+    from jscat import api, synth, structs as S
+    emitters, nus = synth.CFG1_EMITTERS[:2], synth.CFG1_NU[::2]
+    base = synth.write_tables(workdir, emitters, nus, 20261203)
+    atm = synth.atmosphere(emitters, np.random.default_rng(1), t_sigma=0.0)
+    a, c = (synth.limb_geometry(np.linspace(5.0, 60.0, n)), synth.nadir_geometry(np.linspace(0.0, 60.0, n)))
+    geom = {k: np.where(np.arange(n) % 2 == 1, c[k], a[k]) for k in a}
+    ctl = S.make_ctl(emitters, nus, base, hydz=0.0)
+    inp = synth.batch_from([atm], np.zeros(n, np.int32), geom)
+    m = api.Model(ctl)
+    b = api.Batch(m, ctl, 1, len(inp["z"]), n)
+    try:
+        b.upload(inp)
+        b.run()
+        got = b.download()
+        points, longest = int(got["nlos"].sum()), int(got["nlos"].max())
+        warps = (points // longest + 31) // 32 * len(nus) * 2
+        assert (warps <= 2048) == (variant == 21)
+        assert b.variant()["variant"] == variant
+    finally:
+        b.close()
+    want = api.formod_batch(ctl, inp, model=m, variant=43 - variant)
+    for k in ("rad", "tau", "nlos"):
+        np.testing.assert_array_equal(got[k], want[k])
+
+
 @pytest.mark.parametrize("kind", ["uneven", "ties", "shifted", "grids", "short"])
 def test_gas_variants_on_irregular_tables(workdir, kind):
     """The default kernels' rules on tables (evenly spaced columns, strictly
