@@ -19,6 +19,7 @@
 // per task: Q_ext, Q_sca and the normalised phase function at NTHETA angles.
 #include <math.h>
 #include <stdint.h>
+#include <string.h>
 
 #include <vector>
 
@@ -56,20 +57,19 @@ constexpr int kHalf = (NTHETA + 1) / 2;   // angles 0..90 degrees
 constexpr int kThreads = 128;
 static_assert(kHalf < kThreads, "a thread per angle and one for Q_sca");
 
-// What a task keeps per order n.
-struct MieTerm {
-  cplx d;           // D_n
-  double psi, chi;
-  cplx a, b;        // (2 n + 1) / (n (n + 1)) times a_n, b_n
-  double c1, c2;    // (2 n + 1) / n, (n + 1) / n
-  double q;         // (2 n + 1) (|a_n|^2 + |b_n|^2)
-};
+// What a task keeps per order n: D_n, then (2 n + 1) / (n (n + 1)) a_n in its
+// place; psi_n and chi_n, then the same of b_n; and (2 n + 1) (|a_n|^2 +
+// |b_n|^2).
+constexpr int kTerm = 5;                  // doubles per order
+constexpr int kSharedOrders = 5000;       // most orders kept in shared memory (200 KB)
+constexpr int kScratchTasks = 1184;       // tasks per launch above that: 8 blocks an SM
 
 struct MieArgs {
-  int n;
+  int n, cap;                 // tasks; orders 0 .. cap - 1 of the largest
+  const int *task;            // [n] the tasks, long ones first
   const double *x, *nr, *ni;  // [n] size parameter, refractive index
-  const int64_t *doff;        // [n + 1] first term of each task
-  MieTerm *term;
+  const cplx *c;              // [cap] (2 n + 1) / n, (n + 1) / n
+  double *term;               // [blocks][kTerm * cap] where shared memory is too small
   double *out;                // [n][2 + NTHETA]: Q_ext, Q_sca, phase
   unsigned *status;
 };
@@ -77,9 +77,18 @@ struct MieArgs {
 // Bound by the serial recurrences (one complex quotient an order).  With a
 // warp per task that ran the upward recurrence, both coefficients and three
 // angles a lane in one loop: 916 us for an ice cloud of 1360 tasks (up to 830
-// orders), now 199 us.
+// orders), now 146 us.  The orders lie in shared memory (33 KB a block there),
+// long tasks start first: in device memory, allocated for the call and 88 bytes
+// an order, the kernel took 199 us and the allocation 0.6 ms more than before.
+// SHARED false: more than kSharedOrders.
+template <bool SHARED>
 __global__ void __launch_bounds__(kThreads) mie_kernel(MieArgs A) {
-  const int task = blockIdx.x, tid = threadIdx.x;
+  extern __shared__ __align__(16) double mie_sh[];
+  const int task = A.task[blockIdx.x], tid = threadIdx.x;
+  double *base = SHARED ? mie_sh : A.term + (size_t)blockIdx.x * kTerm * A.cap;
+  cplx *td = reinterpret_cast<cplx *>(base);                         // D_n, a_n
+  cplx *tr = reinterpret_cast<cplx *>(base) + A.cap;                 // psi_n and chi_n, b_n
+  double *tq = base + 4 * (size_t)A.cap;
   const double x = A.x[task];
   const cplx m = cmake(A.nr[task], A.ni[task]);
   const cplx y = cmul(cmake(x, 0.0), m);
@@ -87,9 +96,8 @@ __global__ void __launch_bounds__(kThreads) mie_kernel(MieArgs A) {
   const int nstop = (int)xstop;
   const double ymod = cabs_(y);
   const int nmx = (int)((xstop > ymod ? xstop : ymod) + 15);
-  MieTerm *term = A.term + A.doff[task];
-  if (nmx + 1 > A.doff[task + 1] - A.doff[task] || nstop >= nmx) {
-    if (tid == 0) atomicOr(A.status, 1u);  // the host sized the scratch otherwise
+  if (nstop + 1 > A.cap || nstop >= nmx) {
+    if (tid == 0) atomicOr(A.status, 1u);  // the host counted otherwise
     return;
   }
   if (tid == 0) {
@@ -98,19 +106,17 @@ __global__ void __launch_bounds__(kThreads) mie_kernel(MieArgs A) {
     for (int k = nmx; k >= 2; k--) {
       const cplx q = cscale(ry, (double)k);
       d = csub(q, cdiv(cmake(1.0, 0.0), cadd(d, q)));
-      if (k - 1 <= nstop) term[k - 1].d = d;
+      if (k - 1 <= nstop) td[k - 1] = d;
     }
   } else if (tid == 32) {
     double psi0 = cos(x), psi1 = sin(x), chi0 = -sin(x), chi1 = cos(x);
     const double rx = 1.0 / x;
-    term[0].psi = psi1;
-    term[0].chi = chi1;
+    tr[0] = cmake(psi1, chi1);
     for (int n = 1; n <= nstop; n++) {
       const double f = 2.0 * n - 1.0;
       const double psi = div_known(f * psi1, x, rx) - psi0;
       const double chi = div_known(f * chi1, x, rx) - chi0;
-      term[n].psi = psi;
-      term[n].chi = chi;
+      tr[n] = cmake(psi, chi);
       psi0 = psi1;
       psi1 = psi;
       chi0 = chi1;
@@ -118,27 +124,36 @@ __global__ void __launch_bounds__(kThreads) mie_kernel(MieArgs A) {
     }
   }
   __syncthreads();
-  for (int n = 1 + tid; n <= nstop; n += kThreads) {
-    MieTerm &t = term[n];
-    const double rn = (double)n, psi1 = term[n - 1].psi;
-    const cplx xi = cmake(t.psi, -t.chi), xi1 = cmake(psi1, -term[n - 1].chi);
-    const cplx ga = cadd(cdiv(t.d, m), cmake(rn / x, 0.0));
-    const cplx an = cdiv(csub(cscale(ga, t.psi), cmake(psi1, 0.0)), csub(cmul(ga, xi), xi1));
-    const cplx gb = cadd(cmul(m, t.d), cmake(rn / x, 0.0));
-    const cplx bn = cdiv(csub(cscale(gb, t.psi), cmake(psi1, 0.0)), csub(cmul(gb, xi), xi1));
-    const double fn = (2.0 * rn + 1.0) / (rn * (rn + 1.0));
-    t.a = cscale(an, fn);
-    t.b = cscale(bn, fn);
-    t.c1 = (2.0 * rn + 1.0) / rn;
-    t.c2 = (rn + 1.0) / rn;
-    t.q = (2.0 * rn + 1.0) * (an.re * an.re + an.im * an.im + bn.re * bn.re + bn.im * bn.im);
+  // from the top, so that the order below a chunk is still psi and chi
+  for (int n0 = (nstop - 1) / kThreads * kThreads; n0 >= 0; n0 -= kThreads) {
+    const int n = n0 + 1 + tid;
+    cplx an, bn;
+    double q = 0;
+    if (n <= nstop) {
+      const double rn = (double)n, psi = tr[n].re, psi1 = tr[n - 1].re;
+      const cplx xi = cmake(psi, -tr[n].im), xi1 = cmake(psi1, -tr[n - 1].im), d = td[n];
+      const cplx ga = cadd(cdiv(d, m), cmake(rn / x, 0.0));
+      an = cdiv(csub(cscale(ga, psi), cmake(psi1, 0.0)), csub(cmul(ga, xi), xi1));
+      const cplx gb = cadd(cmul(m, d), cmake(rn / x, 0.0));
+      bn = cdiv(csub(cscale(gb, psi), cmake(psi1, 0.0)), csub(cmul(gb, xi), xi1));
+      q = (2.0 * rn + 1.0) * (an.re * an.re + an.im * an.im + bn.re * bn.re + bn.im * bn.im);
+      const double fn = (2.0 * rn + 1.0) / (rn * (rn + 1.0));
+      an = cscale(an, fn);
+      bn = cscale(bn, fn);
+    }
+    __syncthreads();
+    if (n <= nstop) {
+      td[n] = an;
+      tr[n] = bn;
+      tq[n] = q;
+    }
   }
   __syncthreads();
   __shared__ double qs_s;
   if (tid == kHalf) {
     double q = 0.0;
 #pragma unroll 8
-    for (int n = 1; n <= nstop; n++) q += term[n].q;
+    for (int n = 1; n <= nstop; n++) q += tq[n];
     qs_s = (2.0 / (x * x)) * q;
   }
   // Sums of a_n p, b_n t, a_n t and b_n p over the odd and the even orders:
@@ -151,9 +166,8 @@ __global__ void __launch_bounds__(kThreads) mie_kernel(MieArgs A) {
     const double mu = cos((double)tid * (0.5 * M_PI / (double)(kHalf - 1)));
     double p = 1.0, pprev = 0.0;
     auto order = [&](int n, cplx &sap, cplx &sbt, cplx &sat, cplx &sbp) {
-      const MieTerm &t = term[n];
-      const cplx a = t.a, b = t.b;
-      const double rn = (double)n, c1 = t.c1, c2 = t.c2;
+      const cplx a = td[n], b = tr[n], c = A.c[n];
+      const double rn = (double)n, c1 = c.re, c2 = c.im;
       const double tau = __fma_rn(rn * mu, p, -((rn + 1.0) * pprev));
       sap.re = __fma_rn(a.re, p, sap.re);
       sap.im = __fma_rn(a.im, p, sap.im);
@@ -214,19 +228,36 @@ extern "C" int jsc_mie_eval(int device, int n, const double *x, const double *nr
       return JSC_ERR_CUDA;
     }
   }
-  std::vector<int64_t> off((size_t)n + 1, 0);
+  int cap = 0;
+  std::vector<int> orders((size_t)n);
   for (int i = 0; i < n; i++) {
     const int64_t s = mie_slots(x[i], nr[i], ni[i]);
     if (!(x[i] > 0) || s > 10000 + 3) {
       jsc_set_error(JSC_ERR_ARG, "Mie: size parameter %g needs more than 10000 terms", x[i]);
       return JSC_ERR_ARG;
     }
-    off[i + 1] = off[i] + s;
+    orders[i] = (int)(x[i] + 4.0 * pow(x[i], 0.3333) + 2.0) + 3;  // and slack, as mie_slots
+    if (orders[i] > cap) cap = orders[i];
   }
-  double *dx = nullptr, *dnr = nullptr, *dni = nullptr, *dout = nullptr;
-  int64_t *doff = nullptr;
-  MieTerm *dterm = nullptr;
-  unsigned *dst = nullptr;
+  // one buffer: x, nr, ni, the factors of the orders, the tasks by length
+  // (64 classes, long ones first); then the status word and the output
+  const size_t nin = 3 * (size_t)n + 2 * (size_t)cap + ((size_t)n + 1) / 2;
+  const size_t nout = 1 + (size_t)n * (2 + NTHETA);
+  std::vector<double> in(nin, 0.0);
+  memcpy(in.data(), x, n * sizeof(double));
+  memcpy(in.data() + n, nr, n * sizeof(double));
+  memcpy(in.data() + 2 * (size_t)n, ni, n * sizeof(double));
+  double *c = in.data() + 3 * (size_t)n;
+  for (int k = 1; k < cap; k++) {
+    c[2 * k] = (2.0 * k + 1.0) / k;
+    c[2 * k + 1] = (k + 1.0) / k;
+  }
+  int *task = reinterpret_cast<int *>(c + 2 * (size_t)cap), first[65] = {0};
+  auto cls = [&](int i) { return 63 - (int)((int64_t)orders[i] * 63 / cap); };
+  for (int i = 0; i < n; i++) first[cls(i) + 1]++;
+  for (int k = 0; k < 64; k++) first[k + 1] += first[k];
+  for (int i = 0; i < n; i++) task[first[cls(i)]++] = i;
+  double *d = nullptr, *dterm = nullptr;
   int st = JSC_OK;
   auto fail = [&](cudaError_t e, const char *what) {
     if (e != cudaSuccess && !st) {
@@ -234,47 +265,48 @@ extern "C" int jsc_mie_eval(int device, int n, const double *x, const double *nr
       st = JSC_ERR_CUDA;
     }
   };
-  fail(cudaMalloc(&dx, 3 * (size_t)n * sizeof(double)), "cudaMalloc");
-  fail(cudaMalloc(&dout, (size_t)n * (2 + NTHETA) * sizeof(double)), "cudaMalloc");
-  fail(cudaMalloc(&doff, ((size_t)n + 1) * sizeof(int64_t)), "cudaMalloc");
-  fail(cudaMalloc(&dterm, (size_t)off[n] * sizeof(MieTerm)), "cudaMalloc");
-  fail(cudaMalloc(&dst, sizeof(unsigned)), "cudaMalloc");
+  const bool shared = cap <= kSharedOrders;
+  const size_t sh = shared ? sizeof(double) * kTerm * cap : 0;
+  fail(cudaMalloc(&d, (nin + nout + 1) * sizeof(double)), "cudaMalloc");
+  if (!shared) fail(cudaMalloc(&dterm, sizeof(double) * kTerm * cap * (size_t)(n < kScratchTasks ? n : kScratchTasks)), "cudaMalloc");
+  if (sh > 48 * 1024)
+    fail(cudaFuncSetAttribute(mie_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh),
+         "shared memory");
   if (!st) {
-    dnr = dx + n;
-    dni = dx + 2 * (size_t)n;
-    fail(cudaMemcpy(dx, x, n * sizeof(double), cudaMemcpyHostToDevice), "copy");
-    fail(cudaMemcpy(dnr, nr, n * sizeof(double), cudaMemcpyHostToDevice), "copy");
-    fail(cudaMemcpy(dni, ni, n * sizeof(double), cudaMemcpyHostToDevice), "copy");
-    fail(cudaMemcpy(doff, off.data(), ((size_t)n + 1) * sizeof(int64_t), cudaMemcpyHostToDevice),
-         "copy");
-    fail(cudaMemset(dst, 0, sizeof(unsigned)), "memset");
-  }
-  if (!st) {
+    double *dc = d + ((3 * (size_t)n + 1) & ~(size_t)1);  // 16-byte aligned, as in the copies below
+    double *dt = dc + 2 * (size_t)cap, *dres = dt + ((size_t)n + 1) / 2;
+    fail(cudaMemcpy(d, in.data(), 3 * (size_t)n * sizeof(double), cudaMemcpyHostToDevice), "copy");
+    fail(cudaMemcpy(dc, c, (nin - 3 * (size_t)n) * sizeof(double), cudaMemcpyHostToDevice), "copy");
+    fail(cudaMemset(dres, 0, sizeof(double)), "memset");
     MieArgs a;
     a.n = n;
-    a.x = dx;
-    a.nr = dnr;
-    a.ni = dni;
-    a.doff = doff;
+    a.cap = cap;
+    a.task = reinterpret_cast<const int *>(dt);
+    a.x = d;
+    a.nr = d + n;
+    a.ni = d + 2 * (size_t)n;
+    a.c = reinterpret_cast<const cplx *>(dc);
     a.term = dterm;
-    a.out = dout;
-    a.status = dst;
-    mie_kernel<<<(unsigned)n, kThreads>>>(a);
-    jsc_count_launch();
-    fail(cudaGetLastError(), "mie_kernel launch");
+    a.out = dres + 1;
+    a.status = reinterpret_cast<unsigned *>(dres);
+    const int step = shared || n < kScratchTasks ? n : kScratchTasks;
+    for (int o = 0; o < n && !st; o += step, a.task += step) {
+      const unsigned blocks = (unsigned)(n - o < step ? n - o : step);
+      if (shared) mie_kernel<true><<<blocks, kThreads, sh>>>(a);
+      else mie_kernel<false><<<blocks, kThreads>>>(a);
+      jsc_count_launch();
+      fail(cudaGetLastError(), "mie_kernel launch");
+    }
     unsigned hs = 0;
-    fail(cudaMemcpy(&hs, dst, sizeof(unsigned), cudaMemcpyDeviceToHost), "mie_kernel");
+    if (!st) fail(cudaMemcpy(&hs, dres, sizeof(unsigned), cudaMemcpyDeviceToHost), "mie_kernel");
     if (!st && hs) {
       jsc_set_error(JSC_ERR_ARG, "Mie: recurrence scratch too small");
       st = JSC_ERR_ARG;
     }
-    fail(cudaMemcpy(out, dout, (size_t)n * (2 + NTHETA) * sizeof(double), cudaMemcpyDeviceToHost),
-         "copy back");
+    if (!st)
+      fail(cudaMemcpy(out, dres + 1, (nout - 1) * sizeof(double), cudaMemcpyDeviceToHost), "copy back");
   }
-  cudaFree(dx);
-  cudaFree(dout);
-  cudaFree(doff);
+  cudaFree(d);
   cudaFree(dterm);
-  cudaFree(dst);
   return st;
 }

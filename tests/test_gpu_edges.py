@@ -398,3 +398,27 @@ def test_mie_series_at_its_ends(nr, ni):
     big = x > 0.05          # extinction of a tiny sphere cancels to its last bits
     assert max_rel(out[big, 0], qe[big]) <= 1e-10
     assert np.max(np.abs(out[:, 2:] - ph.T) / ph.T.max(axis=1, keepdims=True)) <= 1e-10
+
+
+@pytest.mark.parametrize("n", [3, 1300])
+def test_mie_series_beyond_shared_memory(n):
+    """Size parameters whose orders fit shared memory, alone and in a call
+    with one whose orders do not (all tasks then keep them in device memory,
+    in several launches from 1185 tasks on): the same operations, the same
+    bits."""
+    import ctypes as C
+    from jscat import lib as L
+    lib = L.load()
+    lib.jsc_mie_eval.restype = C.c_int
+    dp = C.POINTER(C.c_double)
+
+    def run(x):
+        out = np.empty((len(x), 183))
+        arr = [np.ascontiguousarray(v) for v in (x, np.full(len(x), 1.33), np.full(len(x), 1e-4))]
+        assert lib.jsc_mie_eval(0, len(x), *[a.ctypes.data_as(dp) for a in arr], out.ctypes.data_as(dp)) == 0
+        return out
+
+    x = np.random.default_rng(n).uniform(0.1, 400.0, n)
+    want, got = run(x), run(np.append(x, 5400.0))
+    assert np.all(np.isfinite(got))
+    np.testing.assert_array_equal(got[:n], want)
