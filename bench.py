@@ -158,16 +158,18 @@ def make_workload(n_rays, seed_offset=0):
 TRAFFIC_PER_EGA = {17: ((6.198689e9 + 0.141950e9) / 1.853620866e9, "8def761b6c704d73")}
 # Sources per kernel family: a thread per (ray, channel) (variants 0-8), a
 # lane per (ray, channel, emitter) (9-13), lanes over a tile of 32 rays
-# (14-20).
+# (14-20), gas transmittance with segment and transfer passes (21-22).
 KERNEL_SOURCES = {
     "thread": ["ega_kernel.cuh", "device_common.cuh"],
     "lane": ["ega_lane.cuh", "device_common.cuh"],
     "ray": ["ega_lane.cuh", "device_common.cuh"],
+    "gas": ["ega_gas.cuh", "device_math.cuh", "ega_lane.cuh", "device_common.cuh"],
 }
 
 
 def kernel_family(variant):
-    return "thread" if variant < 9 else ("lane" if variant < 14 else "ray")
+    return ("thread" if variant < 9 else "lane" if variant < 14 else
+            "ray" if variant < 21 else "gas")
 
 
 def kernel_sources_sha(family):
@@ -352,7 +354,7 @@ def scattering_bench(args, local, torch, oracle_sample=True):
                          "mma_sync_path": {"ms_per_step": sur_ms_mma, "inference_ms": inf_ms_mma}},
            "training": {"samples": int(len(X)), "epochs": args.sca_epochs, "seconds": train_s,
                         "final_loss": float(losses[-1]),
-                        "kernels": "hand-written FP32 SGEMM forward/backward, Adam"}}
+                        "kernels": "hand-written FP32 forward/backward, weight gradients, Adam (three launches a step)"}}
     if oracle_sample:
         try:
             from oracle import refrun
