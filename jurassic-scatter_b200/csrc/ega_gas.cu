@@ -1,14 +1,19 @@
 // Launchers of the gas transmittance, the segment pass and the transfer pass.
 #include "ega_gas.cuh"
 
-// A warp per emitter; the register budget follows the block size.
+// A warp per emitter; the register budget follows the block size.  Up to four
+// emitters 72 registers (28 warps an SM, no spills) beat 64 (32 warps): 43.5
+// against 44.6 ms for the pencils of depth-2 scattering, 2.75 against 2.83 ms
+// for 5000 rays x 16 channels x 4 emitters; 80 (24 warps) only do while the
+// rays fill less than the chip, and with eight emitters 64 stay best (71.6 ms
+// against 75.3 with 80 and 75.8 with 48).
 template <bool DIG>
 static void gas_launch(const GasArgs &ga, cudaStream_t s) {
   const int nw = ga.e.m.ng > 0 ? ga.e.m.ng : 1;
   const unsigned blocks = (unsigned)(((int64_t)ga.e.n_rays + 31) / 32 * ga.e.m.nd);
   const size_t sh = gas_shmem(nw, 32, nw <= 8 ? 4 : 2);
-  if (nw <= 2) ega_gas_kernel<DIG, 4, 64, 16><<<blocks, 32 * nw, sh, s>>>(ga);
-  else if (nw <= 4) ega_gas_kernel<DIG, 4, 128, 8><<<blocks, 32 * nw, sh, s>>>(ga);
+  if (nw <= 2) ega_gas_kernel<DIG, 4, 64, 14><<<blocks, 32 * nw, sh, s>>>(ga);
+  else if (nw <= 4) ega_gas_kernel<DIG, 4, 128, 7><<<blocks, 32 * nw, sh, s>>>(ga);
   else if (nw <= 8) ega_gas_kernel<DIG, 4, 256, 4><<<blocks, 32 * nw, sh, s>>>(ga);
   else ega_gas_kernel<DIG, 2, 1024, 1><<<blocks, 32 * nw, sh, s>>>(ga);
 }
