@@ -221,7 +221,7 @@ extern "C" int jsc_batch_create(jsc_model *m, const ctl_t *ctl, int max_atm,
   if (b->ip == 1) {
     st = st ? st : jsc_dmalloc(&b->d_lev, 8 * (size_t)max_levels);
     st = st ? st : jsc_dmalloc(&b->d_qs, (size_t)(ctl->ng + ctl->nw) * max_levels);
-    st = st ? st : jsc_dmalloc(&b->d_mcount, 2);
+    st = st ? st : jsc_dmalloc(&b->d_mcount, 3);
   }
   b->scan_tiles = (max_rays + JSC_SCAN_TILE - 1) / JSC_SCAN_TILE + 1;
   st = st ? st : jsc_dmalloc(&b->d_scan, (size_t)b->scan_tiles + 1);
@@ -791,9 +791,9 @@ static __global__ void round_live_kernel(const unsigned long long *n_listed, int
 static int batch_run(jsc_batch *b, cudaStream_t s);
 static int run_hydro(jsc_batch *b, cudaStream_t s);
 
-// Fixed-capacity runs: rays whose line of sight did not fit (the storing
-// pass flagged them) keep only the points inside the buffer, so that no
-// later kernel reads past it.
+// Fixed-capacity runs (IP 2/3; IP 1: march_fit_kernel): rays whose line of
+// sight did not fit (the storing pass flagged them) keep only the points
+// inside the buffer, so that no later kernel reads past it.
 static __global__ void clamp_los_kernel(int *nlos, const int64_t *off, int n, int64_t cap) {
   const int r = blockIdx.x * blockDim.x + threadIdx.x;
   if (r >= n) return;
@@ -1578,7 +1578,8 @@ static int fixed_unsupported() {
 
 // Lines of sight of a run in one-dimensional atmospheres (trace.cuh): march,
 // prefix sum of the counts (with the layer edges), records.  One read-back
-// of the total sizes the LOS buffers (none in a fixed-capacity run).
+// of the total sizes the LOS buffers; a fixed-capacity run has none, and cuts
+// its rays to the buffers by the prefix sum of the marched counts.
 static int los_profile(jsc_batch *b, bool refine, cudaStream_t s) {
   const jsc_model *m = b->m;
   const int nr = b->n_rays;
@@ -1586,6 +1587,7 @@ static int los_profile(jsc_batch *b, bool refine, cudaStream_t s) {
   RayArgs ra;
   fill_ray_args(b, ra);
   ra.nlos = refine ? b->d_nlos_b : b->d_nlos;
+  ra.los_off = refine ? b->d_los_off_b : b->d_los_off;
   ExpandArgs xa;
   memset(&xa, 0, sizeof(xa));
   xa.n_rays = nr;
@@ -1604,6 +1606,7 @@ static int los_profile(jsc_batch *b, bool refine, cudaStream_t s) {
   xa.nlos_b = ra.nlos;
   xa.nlos = b->d_nlos;
   xa.off = b->d_los_off;
+  xa.raw = b->fixed ? ra.los_off : nullptr;
   xa.tp = b->d_tp;
   xa.status = b->d_status;
   if (refine) {
@@ -1631,8 +1634,8 @@ static int los_profile(jsc_batch *b, bool refine, cudaStream_t s) {
     xa.M.count = b->d_mcount;
     xa.M.cap = b->mcap;
     xa.M.first = nr;
-    xa.max_seg = b->max_seg;
-    JSC_CUDA_TRY(cudaMemsetAsync(b->d_mcount, 0, 2 * sizeof(unsigned), s));
+    xa.max_seg = xa.max_count = b->max_seg;
+    JSC_CUDA_TRY(cudaMemsetAsync(b->d_mcount, 0, 3 * sizeof(unsigned), s));
     if (b->d_live) {
       // rays the queue leaves alone keep no LOS and no surface; a persistent
       // grid pulls the others
@@ -1648,11 +1651,16 @@ static int los_profile(jsc_batch *b, bool refine, cudaStream_t s) {
       march_kernel<1><<<(unsigned)((nr + 127) / 128), 128, 0, s>>>(ra, xa.M);
     }
     JSC_LAUNCH_CHECK();
+    if (b->fixed) {
+      if ((st = launch_scan(b, ra.nlos, nr, (int64_t *)ra.los_off, s))) return st;
+      march_fit_kernel<<<(unsigned)((nr + 127) / 128), 128, 0, s>>>(ra, xa.M, b->max_seg);
+      JSC_LAUNCH_CHECK();
+    }
     if (refine) {
       edge_count_kernel<<<g32, 128, 0, s>>>(xa);
       JSC_LAUNCH_CHECK();
     }
-    if ((st = launch_scan(b, b->d_nlos, nr, b->d_los_off, s))) return st;
+    if ((refine || !b->fixed) && (st = launch_scan(b, b->d_nlos, nr, b->d_los_off, s))) return st;
     if (b->fixed) {
       *b->h_total = 0;
       b->np_longest = 0;
@@ -1860,7 +1868,7 @@ static int batch_run(jsc_batch *b, cudaStream_t s) {
     const int st = b->ip == 1 ? los_profile(b, refine, s) : los_geo(b, refine, s);
     if (st) return st;
   }
-  if (b->fixed) {
+  if (b->fixed && b->ip != 1) {
     clamp_los_kernel<<<(nr + 127) / 128, 128, 0, s>>>(b->d_nlos, b->d_los_off, nr, b->max_seg);
     JSC_LAUNCH_CHECK();
   }

@@ -356,6 +356,15 @@ static __global__ void psurf_kernel(int n, int per_level, const int *atm_off, co
   jsc_geo2cart(0, lon[l], lat[l], psurf + 3 * (size_t)i);
 }
 
+// Record of a point that belongs to no line of sight: a state that passes
+// over all points can evaluate, indices inside their tables.
+__device__ __forceinline__ void null_record(double *rec, int W) {
+  for (int i = 0; i < W; i++) rec[i] = 0;
+  rec[REC_T] = 250;
+  rec[REC_PLK] = (double)planck_index(250.0);
+  rec[REC_AI] = -999.0;
+}
+
 // One LOS point: geometry, state, raw step.  Written by the storing pass.
 template <bool STORE>
 __device__ __forceinline__ void emit_point(const RayArgs &A, const Profile &a,

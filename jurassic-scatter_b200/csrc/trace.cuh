@@ -5,6 +5,7 @@
 //   march_kernel     the march: per ray the number of points, the surface
 //                    temperature and, per point, its position, step and
 //                    smoothed step, in chunks of 32 points
+//   march_fit_kernel fixed-capacity runs: the rays cut to the capacity
 //   edge_count_kernel  points that the aerosol/cloud layer edges add
 //                    (src/lineofsight.c:193-372), a warp per ray
 //   expand_kernel    the LOS records (state, columns, table brackets, layer
@@ -25,7 +26,8 @@
 struct MarchPool {
   double *pts;      // [cap][JSC_CHUNK][JSC_CHUNK_REC]
   int *next;        // [cap] following chunk of the same ray, -1: none
-  unsigned *count;  // [2] chunks taken beyond the first of each ray; points of the longest ray
+  unsigned *count;  // [3] chunks taken beyond the first of each ray; points of the longest ray;
+                    // chunks taken by march_fit_kernel
   int cap, first;   // chunks of the pool; chunks 0 .. first-1 are the rays' first ones
 };
 
@@ -85,11 +87,12 @@ __device__ __forceinline__ int level_guess(double zf, double zs, int n, double z
 // middle of the step, and that displaced along each axis), and each lane
 // looks up one.  LANES 1: a thread per ray looks them up one after another.
 // ENDS: store nothing, report the last two points in *end (the solar
-// direction search).  Returns the number of points.
-template <int LANES, bool ENDS>
+// direction search).  FIT: store the first `limit` points only.  Returns the
+// number of points.
+template <int LANES, bool ENDS, bool FIT = false>
 __device__ __forceinline__ int march_ray(const RayArgs &A, const MarchPool &M, int ai, int r,
                                          const RayIn &in, unsigned gmask, int role, RayEnd *end,
-                                         double *tsurf) {
+                                         double *tsurf, int limit = 0) {
   const int lo = A.atm_off[ai], n = A.atm_off[ai + 1] - lo;
   const double *__restrict__ lev = A.lev + 8 * (size_t)lo;
   const double *__restrict__ zl = A.z + lo;
@@ -134,7 +137,7 @@ __device__ __forceinline__ int march_ray(const RayArgs &A, const MarchPool &M, i
     }
     const double norm = radius_of(x), z = norm - JSC_RE;
     double *rec = nullptr;
-    if (!ENDS) {
+    if (!ENDS && (!FIT || np < limit)) {
       if ((np & (JSC_CHUNK - 1)) == 0 && np > 0 && chunk >= 0) {  // the next chunk
         int id = 0;
         if (role == 0) {
@@ -281,11 +284,9 @@ __device__ __forceinline__ void march_one(const RayArgs &A, const MarchPool &M, 
     A.nlos[r] = np;
     A.tsurf[r] = tsurf;
     if ((unsigned)np > *(volatile unsigned *)(M.count + 1)) atomicMax(M.count + 1, (unsigned)np);
-    if (np == 0) {
-      A.tp[r] = in.vpz;
-      A.tp[A.n_rays + r] = in.vplon;
-      A.tp[2 * A.n_rays + r] = in.vplat;
-    }
+    A.tp[r] = in.vpz;  // where no tangent point is found
+    A.tp[A.n_rays + r] = in.vplon;
+    A.tp[2 * A.n_rays + r] = in.vplat;
   }
 }
 
@@ -314,6 +315,34 @@ static __global__ void __launch_bounds__(128) march_queue_kernel(RayArgs A, Marc
     if (r0 >= n) break;
     if (r0 + lane < n) march_one<1>(A, M, r0 + lane, 0u, 0);
   }
+}
+
+// Fixed-capacity runs, a thread per ray, after the prefix sum A.los_off of
+// the marched counts A.nlos: a ray that reaches past the max_seg points of
+// the LOS buffers keeps the points inside them and no surface, and the run
+// reports it.  The pool holds every chain inside the buffers, but the march
+// takes chunks as it goes, so rays past their end may have taken those of rays
+// before: where the pool ran out, the rays inside march once more, up to that
+// end and on a counter of their own (first chunks and at most one per 32
+// points of the buffers: the pool's size).  The chains of the others are not
+// read again.
+static __global__ void __launch_bounds__(128) march_fit_kernel(RayArgs A, MarchPool M,
+                                                               int64_t max_seg) {
+  const int r = blockIdx.x * blockDim.x + threadIdx.x;
+  if (r >= A.n_rays) return;
+  const int np = A.nlos[r];
+  const int64_t room = max_seg - A.los_off[r];
+  if (np > room) {
+    atomicOr(A.status, JSC_DEV_ERR_NLOS);
+    A.nlos[r] = room > 0 ? (int)room : 0;
+    A.tsurf[r] = -999;
+  }
+  if (np == 0 || room <= 0 || (int64_t)M.count[0] + M.first <= M.cap) return;
+  const RayIn in = {A.obsz[r], A.obslon[r], A.obslat[r], A.vpz[r], A.vplon[r], A.vplat[r]};
+  double tsurf;
+  M.count += 2;
+  march_ray<1, false, true>(A, M, A.ray_atm[r], r, in, 0u, 0, nullptr, &tsurf,
+                            room < np ? (int)room : np);
 }
 
 // ------------------------------------------------------ aerosol layers --
@@ -353,8 +382,9 @@ struct ExpandArgs {
   const int *nlos_b;               // points of the march
   int *nlos;                       // points with the layer edges
   const int64_t *off;
+  const int64_t *raw;              // prefix sum of the marched counts (fixed-capacity runs), or null
   double *geo, *pts, *tp;
-  int64_t max_seg;
+  int64_t max_seg, max_count;      // points of the buffers; most points of a ray
   EdgeSet E;
   int nl;                          // aerosol/cloud layers
   double transs;
@@ -386,11 +416,30 @@ static __global__ void __launch_bounds__(128) edge_count_kernel(ExpandArgs A) {
   }
   o = __reduce_add_sync(0xffffffffu, o);
   if (lane) return;
-  if (o > NLOS || o > A.max_seg) {
+  if (o > NLOS || o > A.max_count) {
     atomicOr(A.status, JSC_DEV_ERR_NLOS);
     o = 0;
   }
   A.nlos[r] = o;
+}
+
+// Ray r reaches past the LOS buffers: it has no tangent point.
+__device__ __forceinline__ bool past_buffers(const ExpandArgs &A, int r) {
+  return A.raw && A.raw[r + 1] > A.max_seg;
+}
+
+// The records of ray r from point `keep` on (of n, the first at base) are not
+// written: the ray keeps the points before, and passes over all points find
+// null records.
+static __device__ __noinline__ void cut_ray(const ExpandArgs &A, int r, int lane, int64_t base,
+                                               int keep, int n) {
+  __syncwarp();  // every lane has read nlos
+  if (lane == 0) {
+    atomicOr(A.status, JSC_DEV_ERR_NLOS);
+    A.nlos[r] = keep;
+  }
+  for (int64_t i = base + keep + lane; i < base + n && i < A.max_seg; i += 32)
+    null_record(A.pts + i * A.W, A.W);
 }
 
 // Geography to position and back as calls: they are used at several places
@@ -498,7 +547,7 @@ static __global__ void __launch_bounds__(128) tangent_kernel(ExpandArgs A) {
   const int r = blockIdx.x * blockDim.x + threadIdx.x;
   if (r >= A.n_rays) return;
   const int np = A.nlos_b[r];
-  if (np == 0) return;
+  if (np == 0 || past_buffers(A, r)) return;
   const int m = (int)A.tp[r];
   double g0[3], g1[3], g2[3], tp[3];
   if (m <= 0 || m >= np - 1) {
@@ -537,8 +586,10 @@ static __global__ void __launch_bounds__(128) tangent_kernel(ExpandArgs A) {
 // warps waited for instructions (9.9 of 17 cycles an issue, 11.7 lanes
 // active), 9.6 ms for 232,000 pencils, 3.28 after that, 3.03 since the last lane
 // no longer converts its following point by itself.
+// A ray whose records do not fit (a fixed-capacity run, EDGES; without edges
+// march_fit_kernel has cut it) has none.
 template <bool EDGES>
-__global__ void __launch_bounds__(128, 6) expand_kernel(const __grid_constant__ ExpandArgs A) {
+__global__ void __launch_bounds__(128, EDGES ? 6 : 8) expand_kernel(const __grid_constant__ ExpandArgs A) {
   const int r = (int)(((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
   const int lane = threadIdx.x & 31;
   const unsigned full = 0xffffffffu;
@@ -547,18 +598,17 @@ __global__ void __launch_bounds__(128, 6) expand_kernel(const __grid_constant__ 
   if (nb == 0) return;
   const int ai = A.ray_atm[r], lo = A.atm_off[ai], nlev = A.atm_off[ai + 1] - lo;
   const int64_t base = A.off[r];
-  const int nmax = EDGES ? A.nlos[r] : nb;
+  // points to write; none where they do not fit
+  const int nmax = !EDGES ? nb : base + A.nlos[r] <= A.max_seg ? A.nlos[r] : -1;
   // lowest marched point: the first NaN, else the first smallest altitude
   double zlow = 0;
   int mlow = INT_MAX, mnan = INT_MAX;
   double prev[3] = {0, 0, 0};  // geometry of the point before the chunk
   int chunk = r, o = 0;
   for (int c0 = 0; c0 < nb; c0 += JSC_CHUNK) {
-    if (chunk < 0) {  // the march ran out of chunks
-      if (lane == 0) {
-        atomicOr(A.status, JSC_DEV_ERR_NLOS);
-        A.tp[r] = 0;
-      }
+    if (chunk < 0) {  // no chunk: cannot be where the pool holds the run
+      cut_ray(A, r, lane, base, EDGES ? 0 : c0, A.nlos[r]);
+      if (lane == 0) A.tp[r] = 0;
       return;
     }
     const int ip = c0 + lane;
@@ -602,15 +652,8 @@ __global__ void __launch_bounds__(128, 6) expand_kernel(const __grid_constant__ 
         if (lane >= d) incl += v;
       }
       const int total = __shfl_sync(full, incl, 31);
-      if (o + total > nmax || base + o + total > A.max_seg) {
-        if (lane == 0) {
-          atomicOr(A.status, JSC_DEV_ERR_NLOS);
-          A.tp[r] = 0;
-        }
-        return;
-      }
 #pragma unroll 1
-      for (int s0 = 0; s0 < total; s0 += 32) {
+      for (int s0 = 0; s0 < total && o + total <= nmax; s0 += 32) {
         // output point s of the chunk: the k-th crossing before marched point
         // src, or (k = its crossings) that point
         const int s = s0 + lane;
@@ -655,8 +698,12 @@ __global__ void __launch_bounds__(128, 6) expand_kernel(const __grid_constant__ 
     }
   }
   mnan = __reduce_min_sync(full, mnan);
-  if (lane == 0) A.tp[r] = (double)(mnan != INT_MAX ? mnan : mlow);
+  if (lane == 0 && !past_buffers(A, r)) A.tp[r] = (double)(mnan != INT_MAX ? mnan : mlow);
   if (!EDGES) return;
+  if (o != nmax) {
+    cut_ray(A, r, lane, base, 0, A.nlos[r]);
+    return;
+  }
   __syncwarp();  // the geometry written above, for every lane
   const double *go = A.geo + base * 4;
   double carry[3] = {0, 0, 0};  // position of the point before the 32

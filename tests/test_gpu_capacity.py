@@ -1,0 +1,170 @@
+"""Fixed-capacity batches whose lines of sight exceed the capacity given at
+their creation: the run reports it, the rays inside the buffers keep their
+results, the others are cut, and the next request that fits is unaffected."""
+import os
+
+import numpy as np
+import pytest
+
+from conftest import GOLDEN
+
+pytestmark = pytest.mark.gpu
+
+NLOS_STATUS = 5   # JSC_ERR_NLOS
+KEYS = ("rad", "tau", "tpz", "tplon", "tplat", "nlos")
+
+
+def _rays(n, seed=5):
+    from jscat import synth
+    rng = np.random.default_rng(seed)
+    a, b = synth.limb_geometry(rng.uniform(6.0, 50.0, n)), synth.nadir_geometry(rng.uniform(0.0, 60.0, n))
+    odd = np.arange(n) % 3 == 1
+    geom = {k: np.where(odd, b[k], a[k]) for k in a}
+    geom["vpz"][4::13] = 130.0    # rays that miss the atmosphere
+    return geom
+
+
+def _case(workdir, nd, n, aero=False, **kw):
+    from jscat import synth, structs as S
+    rng = np.random.default_rng(3)
+    atms = [synth.atmosphere(synth.CFG0_EMITTERS, rng, t_sigma=1.0) for _ in range(2)]
+    base = synth.write_tables(workdir, synth.CFG0_EMITTERS, synth.CFG0_NU, 20261203)
+    layers = None
+    if aero:
+        layers = S.AeroT.from_buffer_copy(np.load(os.path.join(GOLDEN, "aero_ice8.npz"))["aero"].tobytes())
+        kw = dict(dict(sca_n=1, sca_mult=0), **kw)
+    ctl = S.make_ctl(synth.CFG0_EMITTERS, synth.CFG0_NU[:nd], base, hydz=0.0, **kw)
+    geom = _rays(n)
+    return ctl, synth.batch_from(atms, np.arange(n) % 2, geom), layers
+
+
+def _missing(inp, rays):
+    """The same request with some of its rays above the atmosphere."""
+    out = {k: np.array(v) for k, v in inp.items()}
+    out["vpz"][rays] = 130.0
+    return out
+
+
+def _overflowing(ctl, inp, layers, model, cap, variant=-1):
+    """Outputs of a fixed run that has to report the capacity, then those of
+    the same batch on rays that fit."""
+    from jscat import api, lib as L
+    n, nd = len(inp["ray_atm"]), ctl.nd
+    b = api.Batch(model, ctl, len(inp["atm_off"]) - 1, len(inp["z"]), n, max_seg=cap)
+    out = {k: np.full((n, nd) if k in ("rad", "tau") else n, -7, np.int32 if k == "nlos" else float) for k in KEYS}
+    try:
+        if layers is not None:
+            b.set_aero(layers)
+        b.set_variant(variant)
+        L.check(L.load().jsc_batch_set_fixed(b.h, 1), "jsc_batch_set_fixed")
+        b.upload(inp)
+        b.run()
+        with pytest.raises(L.JscError) as e:
+            b.download(out=out)
+        assert e.value.status == NLOS_STATUS
+        first = int(np.argmin(out["nlos"] == api.formod_batch(ctl, inp, model=model, aero=layers)["nlos"]))
+        fits = _missing(inp, np.arange(n) >= max(first, 1) // 2 + 1)
+        b.upload(fits)
+        b.run()
+        again = b.download()
+        want = api.formod_batch(ctl, fits, model=model, aero=layers)
+        for k in KEYS:
+            np.testing.assert_array_equal(again[k], want[k])
+    finally:
+        b.close()
+    return out
+
+
+def _cut_chains(points, n, cap, nd):
+    """The march has to run out of chunks of 32 points: more of them than the
+    pool holds (a chunk of 1284 bytes per ray and per 32 points of the
+    capacity, or the continuum array if that is larger)."""
+    pool = max((n + cap // 32 + 1) * 1284 // 8 + 1, cap * nd) * 8 // 1284
+    return np.sum((points + 31) // 32) > pool
+
+
+@pytest.mark.parametrize("nd,n,variant,part", [(1, 64, -1, 0.3), (2, 64, 21, 0.3), (2, 64, 22, 0.4), (2, 200, 6, 0.02),
+                                               (1, 33, -1, 0.97), (4, 40, 21, 0.9), (2, 20000, -1, 0.5)])
+def test_clear_air_past_capacity(workdir, nd, n, variant, part):
+    """Rays inside the capacity keep the bits of an ordinary run, the one
+    across its end keeps its points inside, later ones none; where the
+    capacity is a fraction of the points the march's pool runs out as well
+    (a thread per ray above 16384 rays)."""
+    from jscat import api
+    ctl, inp, _ = _case(workdir, nd, n)
+    m = api.Model(ctl)
+    full = api.formod_batch(ctl, inp, model=m)
+    end = np.cumsum(full["nlos"])
+    cap = int(part * end[-1])
+    cut = int(np.argmax(end > cap))
+    if part <= 0.5:
+        assert _cut_chains(full["nlos"], n, cap, nd)
+    out = _overflowing(ctl, inp, None, m, cap, variant)
+    for k in KEYS:
+        np.testing.assert_array_equal(out[k][:cut], full[k][:cut])
+    assert out["nlos"][cut] == cap - (end[cut] - full["nlos"][cut])
+    assert np.all(out["nlos"][cut + 1:] == 0)
+    for k, v in (("tpz", "vpz"), ("tplon", "vplon"), ("tplat", "vplat")):
+        np.testing.assert_array_equal(out[k][cut:], inp[v][cut:])
+
+
+@pytest.mark.parametrize("mult,nd,n,variant,part", [(0, 1, 48, -1, 0.3), (0, 2, 48, 22, 0.3), (0, 4, 30, -1, 0.9),
+                                                    (1, 2, 9, -1, 0.6), (1, 4, 5, 22, 0.9)])
+def test_layers_past_capacity(workdir, mult, nd, n, variant, part):
+    """The same with layer edges between the points and single scattering:
+    the ray across the end of the buffers keeps nothing."""
+    from jscat import api
+    ctl, inp, layers = _case(workdir, nd, n, True, sca_mult=mult)
+    m = api.Model(ctl)
+    full = api.formod_batch(ctl, inp, model=m, aero=layers)
+    end = np.cumsum(full["nlos"])
+    cap = int(part * end[-1])
+    cut = int(np.argmax(end > cap))
+    clear, _, _ = _case(workdir, nd, n)
+    marched = api.formod_batch(clear, inp, model=m)["nlos"]
+    assert np.all(np.cumsum(marched)[:cut] <= cap)
+    if part <= 0.3:
+        assert _cut_chains(marched, n, cap, nd)
+    out = _overflowing(ctl, inp, layers, m, cap, variant)
+    for k in KEYS:
+        np.testing.assert_array_equal(out[k][:cut], full[k][:cut])
+    assert np.all(out["nlos"][cut:] == 0)
+    past = np.cumsum(marched) > cap
+    for k, v in (("tpz", "vpz"), ("tplon", "vplon"), ("tplat", "vplat")):
+        np.testing.assert_array_equal(out[k][~past], full[k][~past])
+        np.testing.assert_array_equal(out[k][past], inp[v][past])
+
+
+@pytest.mark.parametrize("layers", [False, True])
+def test_graph_past_capacity(workdir, layers):
+    """A captured graph: a replay past the capacity reports it, the replay
+    after it gives the bits of an ordinary run."""
+    import torch
+    from jscat import api, lib as L
+    n = 64
+    ctl, inp, aero = _case(workdir, 2, n, layers)
+    m = api.Model(ctl)
+    full = api.formod_batch(ctl, inp, model=m, aero=aero)
+    end = np.cumsum(full["nlos"])
+    cap = int(0.4 * end[-1])
+    cut = int(np.argmax(end > cap))
+    fits = _missing(inp, np.arange(n) >= cut)
+    want = api.formod_batch(ctl, fits, model=m, aero=aero)
+    stream = torch.cuda.Stream()
+    pin = lambda a: torch.from_numpy(np.ascontiguousarray(a)).pin_memory().numpy()   # noqa: E731
+    gb = api.GraphBatch(m, ctl, fits, stream.cuda_stream, pin, max_seg=cap, aero=aero)
+    try:
+        for _ in range(2):
+            gb.launch(inp)
+            stream.synchronize()
+            with pytest.raises(L.JscError) as e:
+                gb.status()
+            assert e.value.status == NLOS_STATUS
+            np.testing.assert_array_equal(gb.out["rad"][:cut], full["rad"][:cut])
+            gb.launch(fits)
+            stream.synchronize()
+            gb.status()
+            for k in KEYS:
+                np.testing.assert_array_equal(gb.out[k], want[k])
+    finally:
+        gb.close()
