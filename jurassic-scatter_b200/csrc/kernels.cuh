@@ -365,6 +365,33 @@ __device__ __forceinline__ void null_record(double *rec, int W) {
   rec[REC_AI] = -999.0;
 }
 
+// The records of a run's lines of sight, as far as cut_ray needs them.
+struct Lines {
+  unsigned *status;
+  int *nlos;
+  double *pts;
+  int W;
+  int64_t max_seg;
+};
+
+template <typename Args>
+__device__ __forceinline__ Lines lines_of(const Args &A) {
+  return Lines{A.status, A.nlos, A.pts, A.W, A.max_seg};
+}
+
+// The records of ray r (n, the first at base) are not written: the ray keeps no
+// point, and passes over all points find null records.  By `lanes` lanes that
+// have read nlos.
+static __device__ __noinline__ void cut_ray(Lines L, int r, int lane, int lanes, int64_t base,
+                                            int n) {
+  if (lane == 0) {
+    atomicOr(L.status, JSC_DEV_ERR_NLOS);
+    L.nlos[r] = 0;
+  }
+  for (int64_t i = base + lane; i < base + n && i < L.max_seg; i += lanes)
+    null_record(L.pts + i * L.W, L.W);
+}
+
 // One LOS point: geometry, state, raw step.  Written by the storing pass.
 template <bool STORE>
 __device__ __forceinline__ void emit_point(const RayArgs &A, const Profile &a,
@@ -822,8 +849,7 @@ __device__ __forceinline__ Profile refine_profile(const RefineArgs &A, int r) {
 // the point, then the point) places them in the order the serial pass
 // writes them, the raw records are copied with coalesced loads, then lanes
 // take 32 refined points at a time for refine_point, with the neighbours'
-// Cartesian positions passed by shuffles.  Same outputs as the serial pass,
-// including its overflow status.
+// Cartesian positions passed by shuffles.
 template <int IP = 1>
 __global__ void __launch_bounds__(128, 8) refine_store_kernel(RefineArgs A) {
   const int r = (int)(((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
@@ -835,8 +861,15 @@ __global__ void __launch_bounds__(128, 8) refine_store_kernel(RefineArgs A) {
   const Profile a = refine_profile(A, r);
   const double *gb = A.geo_b + A.off_b[r] * 4, *pb = A.pts_b + A.off_b[r] * A.W;
   const int64_t base = A.off[r];
+  // points to write; a ray that does not fit the buffers (a fixed-capacity
+  // run) has none
   const int nmax = A.nlos[r];
   const int W = A.W;
+  if (base + nmax > A.max_seg) {
+    __syncwarp();  // every lane has read nlos
+    cut_ray(lines_of(A), r, lane, 32, base, nmax);
+    return;
+  }
   int o = 0;
   for (int c0 = 0; c0 < nb; c0 += 32) {
     const int ip = c0 + lane;
@@ -862,10 +895,7 @@ __global__ void __launch_bounds__(128, 8) refine_store_kernel(RefineArgs A) {
       if (lane >= d) incl += v;
     }
     const int total = __shfl_sync(full, incl, 31);
-    if (o + total > nmax || base + o + total > A.max_seg) {
-      if (lane == 0) atomicOr(A.status, JSC_DEV_ERR_NLOS);
-      return;
-    }
+    if (o + total > nmax) return;  // the counting pass found too many (nmax 0)
     int slot = o + incl - cnt;  // first output slot of this lane
     if (ip < nb) {
       if (win)
@@ -896,10 +926,6 @@ __global__ void __launch_bounds__(128, 8) refine_store_kernel(RefineArgs A) {
       if (e < ne) A.pts[(base + sl) * W + (e - pp * W)] = pb[(size_t)c0 * W + e];
     }
     o += total;
-  }
-  if (o > NLOS) {
-    if (lane == 0) atomicOr(A.status, JSC_DEV_ERR_NLOS);
-    return;
   }
   __syncwarp();  // the points written above, for every lane
   const double *go = A.geo + base * 4;

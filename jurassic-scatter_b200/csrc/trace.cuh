@@ -428,20 +428,6 @@ __device__ __forceinline__ bool past_buffers(const ExpandArgs &A, int r) {
   return A.raw && A.raw[r + 1] > A.max_seg;
 }
 
-// The records of ray r from point `keep` on (of n, the first at base) are not
-// written: the ray keeps the points before, and passes over all points find
-// null records.
-static __device__ __noinline__ void cut_ray(const ExpandArgs &A, int r, int lane, int64_t base,
-                                               int keep, int n) {
-  __syncwarp();  // every lane has read nlos
-  if (lane == 0) {
-    atomicOr(A.status, JSC_DEV_ERR_NLOS);
-    A.nlos[r] = keep;
-  }
-  for (int64_t i = base + keep + lane; i < base + n && i < A.max_seg; i += 32)
-    null_record(A.pts + i * A.W, A.W);
-}
-
 // Geography to position and back as calls: they are used at several places
 // of the kernels below, whose instructions would not stay in the
 // instruction cache if each were inlined.
@@ -541,13 +527,17 @@ __device__ inline double marched_point(const MarchPool &M, int r, int ip, double
   return rec[3];
 }
 
-// Tangent point of each ray, a thread per ray, from its marched points
+// Tangent point of each ray, a thread per ray, from its marched points;
+// rays without records are cut.
 // (src/lineofsight.c:411-452); tp[r] holds the number of the lowest one.
 static __global__ void __launch_bounds__(128) tangent_kernel(ExpandArgs A) {
   const int r = blockIdx.x * blockDim.x + threadIdx.x;
   if (r >= A.n_rays) return;
   const int np = A.nlos_b[r];
-  if (np == 0 || past_buffers(A, r)) return;
+  if (np == 0) return;
+  if (A.off[r] + A.nlos[r] > A.max_seg)  // expand_kernel<true> has written nothing
+    cut_ray(lines_of(A), r, 0, 1, A.off[r], A.nlos[r]);
+  if (past_buffers(A, r)) return;
   const int m = (int)A.tp[r];
   double g0[3], g1[3], g2[3], tp[3];
   if (m <= 0 || m >= np - 1) {
@@ -586,8 +576,8 @@ static __global__ void __launch_bounds__(128) tangent_kernel(ExpandArgs A) {
 // warps waited for instructions (9.9 of 17 cycles an issue, 11.7 lanes
 // active), 9.6 ms for 232,000 pencils, 3.28 after that, 3.03 since the last lane
 // no longer converts its following point by itself.
-// A ray whose records do not fit (a fixed-capacity run, EDGES; without edges
-// march_fit_kernel has cut it) has none.
+// A ray whose records do not fit (a fixed-capacity run, EDGES) gets none, and
+// tangent_kernel cuts it; without edges march_fit_kernel has.
 template <bool EDGES>
 __global__ void __launch_bounds__(128, EDGES ? 6 : 8) expand_kernel(const __grid_constant__ ExpandArgs A) {
   const int r = (int)(((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
@@ -606,9 +596,11 @@ __global__ void __launch_bounds__(128, EDGES ? 6 : 8) expand_kernel(const __grid
   double prev[3] = {0, 0, 0};  // geometry of the point before the chunk
   int chunk = r, o = 0;
   for (int c0 = 0; c0 < nb; c0 += JSC_CHUNK) {
-    if (chunk < 0) {  // no chunk: cannot be where the pool holds the run
-      cut_ray(A, r, lane, base, EDGES ? 0 : c0, A.nlos[r]);
-      if (lane == 0) A.tp[r] = 0;
+    if (chunk < 0) {  // cannot be: the pool holds the chains of a run's last march
+      if (lane == 0) {
+        atomicOr(A.status, JSC_DEV_ERR_NLOS);
+        A.nlos[r] = 0;
+      }
       return;
     }
     const int ip = c0 + lane;
@@ -700,10 +692,7 @@ __global__ void __launch_bounds__(128, EDGES ? 6 : 8) expand_kernel(const __grid
   mnan = __reduce_min_sync(full, mnan);
   if (lane == 0 && !past_buffers(A, r)) A.tp[r] = (double)(mnan != INT_MAX ? mnan : mlow);
   if (!EDGES) return;
-  if (o != nmax) {
-    cut_ray(A, r, lane, base, 0, A.nlos[r]);
-    return;
-  }
+  if (o != nmax) return;
   __syncwarp();  // the geometry written above, for every lane
   const double *go = A.geo + base * 4;
   double carry[3] = {0, 0, 0};  // position of the point before the 32

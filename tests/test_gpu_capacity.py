@@ -168,3 +168,30 @@ def test_graph_past_capacity(workdir, layers):
                 np.testing.assert_array_equal(gb.out[k], want[k])
     finally:
         gb.close()
+
+
+@pytest.mark.parametrize("ip,mult", [(2, None), (2, 0), (3, 0)])
+def test_horizontally_varying_past_capacity(workdir, ip, mult):
+    """IP 2 and 3, without and with layers, whose edges are a pass over the
+    stored points: the ray across the end keeps its points inside in clear
+    air and nothing with layers."""
+    from jscat import api, synth, structs as S
+    ctlkw, atm, geom = synth.curtain_case(workdir)
+    geom = {k: v[::4] for k, v in geom.items()}
+    n, layers = len(geom["obsz"]), None
+    kw = dict(ctlkw, nus=ctlkw["nus"][:2], ip=ip, **(dict(cz=1.5, cx=900.0) if ip == 3 else {}))
+    if mult is not None:
+        layers = S.AeroT.from_buffer_copy(np.load(os.path.join(GOLDEN, "aero_ice8.npz"))["aero"].tobytes())
+        kw.update(sca_n=1, sca_mult=mult)
+    atms = [{k: v[..., 121 * i:121 * i + 121] for k, v in atm.items()} for i in range(5)] if ip == 2 else [atm]
+    ctl, inp = S.make_ctl(**kw), synth.batch_from(atms, np.zeros(n, np.int32), geom)
+    m = api.Model(ctl)
+    full = api.formod_batch(ctl, inp, model=m, aero=layers)
+    end = np.cumsum(full["nlos"])
+    cap = int(0.6 * end[-1])
+    cut = int(np.argmax(end > cap))
+    out = _overflowing(ctl, inp, layers, m, cap)
+    for k in KEYS:
+        np.testing.assert_array_equal(out[k][:cut], full[k][:cut])
+    assert out["nlos"][cut] == (cap - (end[cut] - full["nlos"][cut]) if mult is None else 0)
+    assert np.all(out["nlos"][cut + 1:] == 0)
