@@ -79,6 +79,7 @@ extern "C" void jsc_batch_destroy(jsc_batch *b) {
   cudaFree(b->d_lev);
   cudaFree(b->d_qs);
   cudaFree(b->d_mcount);
+  cudaFree(b->d_npts);
   cudaFree(b->d_ray_atm);
   cudaFree(b->d_ray);
   cudaFree(b->d_nlos);
@@ -216,6 +217,7 @@ extern "C" int jsc_batch_create(jsc_model *m, const ctl_t *ctl, int max_atm,
   st = st ? st : jsc_dmalloc(&b->d_tau, (size_t)max_rays * ctl->nd);
   st = st ? st : jsc_dmalloc(&b->d_status, 1);
   st = st ? st : jsc_dmalloc(&b->d_counters, 2);
+  st = st ? st : jsc_dmalloc(&b->d_npts, 1);
   if (!st) st = batch_alloc_los(b, max_seg > 0 ? max_seg : (int64_t)max_rays * 512);
   st = st ? st : batch_alloc_ctm(b, b->max_seg);
   if (b->ip == 1) {
@@ -799,6 +801,12 @@ static __global__ void clamp_los_kernel(int *nlos, const int64_t *off, int n, in
   if (r >= n) return;
   const int64_t room = cap - off[r];
   if (room < nlos[r]) nlos[r] = room > 0 ? (int)room : 0;
+}
+
+// LOS points of a fixed-capacity run inside the buffers, for the pass over all
+// (point, channel) pairs.
+static __global__ void live_records_kernel(const int64_t *total, int64_t cap, int64_t *live) {
+  *live = *total < cap ? *total : cap;
 }
 
 // OR a child batch's device status into its parent's.
@@ -1932,8 +1940,12 @@ static int batch_run(jsc_batch *b, cudaStream_t s) {
     ca.pts = b->d_pts;
     ca.beta = b->d_ctm;
     ca.src = b->d_srcp;
-    ca.n_live = b->fixed ? b->d_los_off + nr : nullptr;
+    ca.n_live = b->fixed ? b->d_npts : nullptr;
     ev_record(b, JSC_T_CTM, 0, s);
+    if (b->fixed) {
+      live_records_kernel<<<1, 1, 0, s>>>(b->d_los_off + nr, b->max_seg, b->d_npts);
+      JSC_LAUNCH_CHECK();
+    }
     jsc_ctm_src_launch(ca, s);
     JSC_LAUNCH_CHECK();
     ev_record(b, JSC_T_CTM, 1, s);

@@ -189,6 +189,7 @@ struct jsc_batch {
   double *d_ctm, *d_srcp;   // [ctm_seg][nd]: continuum extinction, Planck source
   int64_t ctm_seg;
   int64_t n_points;         // LOS points of the current run
+  int64_t *d_npts;          // [1] of them inside the buffers (fixed-capacity runs)
   int np_longest;           // of its longest ray (before layer edges); 0: not known
   double *d_tsurf;          // [max_rays]
   double *d_tp;             // [3][max_rays]

@@ -136,6 +136,25 @@ def test_layers_past_capacity(workdir, mult, nd, n, variant, part):
 
 
 @pytest.mark.parametrize("layers", [False, True])
+@pytest.mark.parametrize("variant", [9, 13, 14, 17])
+def test_continuum_pass_past_capacity(workdir, layers, variant):
+    """The lane and ray-tile variants, whose pass over all (point, channel)
+    pairs takes their number from the device: not more than the buffers
+    hold."""
+    from jscat import api
+    n = 24
+    ctl, inp, aero = _case(workdir, 4, n, layers)
+    m = api.Model(ctl)
+    full = api.formod_batch(ctl, inp, model=m, aero=aero)
+    end = np.cumsum(full["nlos"])
+    cap = int(0.5 * end[-1])
+    cut = int(np.argmax(end > cap))
+    out = _overflowing(ctl, inp, aero, m, cap, variant)
+    for k in KEYS:
+        np.testing.assert_array_equal(out[k][:cut], full[k][:cut])
+
+
+@pytest.mark.parametrize("layers", [False, True])
 def test_graph_past_capacity(workdir, layers):
     """A captured graph: a replay past the capacity reports it, the replay
     after it gives the bits of an ordinary run."""
