@@ -1642,7 +1642,8 @@ static int los_profile(jsc_batch *b, bool refine, cudaStream_t s) {
     xa.M.count = b->d_mcount;
     xa.M.cap = b->mcap;
     xa.M.first = nr;
-    xa.max_seg = xa.max_count = b->max_seg;
+    xa.max_seg = b->max_seg;
+    xa.max_count = b->fixed ? b->max_seg : INT64_MAX;  // else the buffers grow
     JSC_CUDA_TRY(cudaMemsetAsync(b->d_mcount, 0, 3 * sizeof(unsigned), s));
     if (b->d_live) {
       // rays the queue leaves alone keep no LOS and no surface; a persistent
@@ -1815,7 +1816,7 @@ static int los_geo(jsc_batch *b, bool refine, cudaStream_t s) {
     fa.status = b->d_status;
     fa.geo = b->d_geo;
     fa.pts = b->d_pts;
-    fa.max_seg = b->max_seg;
+    fa.max_seg = b->fixed ? b->max_seg : INT64_MAX;  // most points of a ray: else the buffers grow
     refine_count_kernel<<<(nr + 127) / 128, 128, 0, s>>>(fa);
     JSC_LAUNCH_CHECK();
     {

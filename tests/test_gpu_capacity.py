@@ -214,3 +214,44 @@ def test_horizontally_varying_past_capacity(workdir, ip, mult):
         np.testing.assert_array_equal(out[k][:cut], full[k][:cut])
     assert out["nlos"][cut] == (cap - (end[cut] - full["nlos"][cut]) if mult is None else 0)
     assert np.all(out["nlos"][cut + 1:] == 0)
+
+
+@pytest.mark.parametrize("ip,n,cap", [(1, 1, 1), (1, 17, 1), (1, 17, 200), (2, 5, 1), (3, 3, 100)])
+def test_buffers_grow_with_layers(workdir, ip, n, cap):
+    """Ordinary runs whose rays, each by itself, have more points with the
+    layer edges than the batch starts with room for: the buffers grow, as
+    they do in clear air."""
+    from jscat import api, synth, structs as S
+    ctlkw, atm, geom = synth.curtain_case(workdir)
+    geom = {k: v[:n] for k, v in geom.items()}
+    layers = S.AeroT.from_buffer_copy(np.load(os.path.join(GOLDEN, "aero_ice8.npz"))["aero"].tobytes())
+    kw = dict(ctlkw, sca_n=1, sca_mult=0, ip=ip, **(dict(cz=1.5, cx=900.0) if ip == 3 else {}))
+    cols = [{k: v[..., 121 * i:121 * i + 121] for k, v in atm.items()} for i in range(5)]
+    atms = [atm] if ip == 3 else cols
+    ctl, inp = S.make_ctl(**kw), synth.batch_from(atms, np.zeros(n, np.int32), geom)
+    m = api.Model(ctl)
+
+    def run(max_seg):
+        b = api.Batch(m, ctl, len(atms), len(inp["z"]), n, max_seg=max_seg)
+        try:
+            b.set_aero(layers)
+            b.upload(inp)
+            b.run()
+            return b.download()
+        finally:
+            b.close()
+
+    want, got = run(4096 * n), run(cap)
+    assert want["nlos"].min() > cap
+    for k in KEYS:
+        np.testing.assert_array_equal(got[k], want[k])
+
+
+def test_one_ray_above_the_default_capacity(workdir):
+    """One pencil whose line of sight, with short steps and a layer, exceeds
+    the 512 points a one-ray batch starts with."""
+    from jscat import api
+    ctl, inp, layers = _case(workdir, 2, 1, True, raydz=0.2, rayds=2.0)
+    out = api.formod_batch(ctl, inp, aero=layers)
+    assert out["nlos"][0] > 512
+    assert np.all(out["rad"] > 0)
