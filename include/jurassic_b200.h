@@ -600,6 +600,11 @@ int jsc_batch_set_wait_budget(jsc_batch *b, unsigned polls);
  * JSC_OK (scan correct), JSC_ERR_WATCHDOG (a wait gave up) or an error. */
 int jsc_scan_selftest(int device, int n, unsigned budget, int stall);
 
+/* Diagnostic: the n-th device allocation that a run or jsc_batch_set_aero
+ * makes for b from now on fails with JSC_ERR_NOMEM (0: none does).  The batch
+ * stays usable: a later call allocates again. */
+int jsc_batch_fail_alloc(jsc_batch *b, int n);
+
 /* Per-(ray, channel) checksum of every emissivity-table index the EGA
  * interpolation selected in the last run, for parity checks against the
  * reference's indices.  Per emitter g, D_g folds d = d*1000003 + v over the

@@ -15,14 +15,36 @@
 static int sca_alpha(double *alpha, int nalpha);
 static int map_status(unsigned st);
 
+// Device memory of a batch; fails on request (jsc_batch_fail_alloc).
+template <typename T>
+static int batch_dmalloc(jsc_batch *b, T **p, size_t n) {
+  if (b->fail_alloc > 0 && --b->fail_alloc == 0) {
+    *p = nullptr;
+    jsc_set_error(JSC_ERR_NOMEM, "allocation of %zu bytes refused on request", n * sizeof(T));
+    return JSC_ERR_NOMEM;
+  }
+  return jsc_dmalloc(p, n);
+}
+
+extern "C" int jsc_batch_fail_alloc(jsc_batch *b, int n) {
+  if (!b || n < 0) return JSC_ERR_ARG;
+  b->fail_alloc = n;
+  return JSC_OK;
+}
+
+// The sizes below are 0 while their buffers are being replaced, so that a
+// failed allocation leaves a batch without them, not one that writes through
+// them.
+
 // LOS geometry and records of max_seg points.
 static int batch_alloc_los(jsc_batch *b, int64_t max_seg) {
   cudaFree(b->d_geo);
   cudaFree(b->d_pts);
   b->d_geo = b->d_pts = nullptr;
+  b->max_seg = 0;
   int st;
-  if ((st = jsc_dmalloc(&b->d_geo, (size_t)max_seg * 4))) return st;
-  if ((st = jsc_dmalloc(&b->d_pts, (size_t)max_seg * b->W))) return st;
+  if ((st = batch_dmalloc(b, &b->d_geo, (size_t)max_seg * 4))) return st;
+  if ((st = batch_dmalloc(b, &b->d_pts, (size_t)max_seg * b->W))) return st;
   b->max_seg = max_seg;
   return JSC_OK;
 }
@@ -38,6 +60,7 @@ static int batch_alloc_ctm(jsc_batch *b, int64_t pool_seg) {
   b->d_mpts = nullptr;
   b->d_mnext = nullptr;
   b->mcap = 0;
+  b->ctm_seg = 0;
   const size_t chunk = JSC_CHUNK * JSC_CHUNK_REC * sizeof(double);
   size_t n = (size_t)b->max_seg * b->cfg.nd;
   if (b->ip == 1) {
@@ -50,8 +73,8 @@ static int batch_alloc_ctm(jsc_batch *b, int64_t pool_seg) {
     if (n < need) n = need;
   }
   int st;
-  if ((st = jsc_dmalloc(&b->d_ctm, n))) return st;
-  if ((st = jsc_dmalloc(&b->d_srcp, (size_t)b->max_seg * b->cfg.nd))) return st;
+  if ((st = batch_dmalloc(b, &b->d_ctm, n))) return st;
+  if ((st = batch_dmalloc(b, &b->d_srcp, (size_t)b->max_seg * b->cfg.nd))) return st;
   if (b->ip == 1) {
     const size_t cap = n * sizeof(double) / (chunk + sizeof(int));
     b->mcap = cap < INT_MAX ? (int)cap : INT_MAX;
@@ -60,6 +83,19 @@ static int batch_alloc_ctm(jsc_batch *b, int64_t pool_seg) {
   }
   b->ctm_seg = b->max_seg;
   return JSC_OK;
+}
+
+// The LOS buffers of a run, as at the batch's creation where an earlier run
+// lost them to a failed allocation.
+static int batch_ensure_los(jsc_batch *b) {
+  int st;
+  if (b->max_seg > 0 && b->ctm_seg >= b->max_seg) return JSC_OK;
+  if (b->fixed) {
+    jsc_set_error(JSC_ERR_NOMEM, "a failed allocation left the batch without LOS buffers");
+    return JSC_ERR_NOMEM;
+  }
+  if (b->max_seg == 0 && (st = batch_alloc_los(b, b->seg_req))) return st;
+  return batch_alloc_ctm(b, b->max_seg);
 }
 
 extern "C" void jsc_batch_destroy(jsc_batch *b) {
@@ -218,7 +254,8 @@ extern "C" int jsc_batch_create(jsc_model *m, const ctl_t *ctl, int max_atm,
   st = st ? st : jsc_dmalloc(&b->d_status, 1);
   st = st ? st : jsc_dmalloc(&b->d_counters, 2);
   st = st ? st : jsc_dmalloc(&b->d_npts, 1);
-  if (!st) st = batch_alloc_los(b, max_seg > 0 ? max_seg : (int64_t)max_rays * 512);
+  b->seg_req = max_seg > 0 ? max_seg : (int64_t)max_rays * 512;
+  if (!st) st = batch_alloc_los(b, b->seg_req);
   st = st ? st : batch_alloc_ctm(b, b->max_seg);
   if (b->ip == 1) {
     st = st ? st : jsc_dmalloc(&b->d_lev, 8 * (size_t)max_levels);
@@ -361,6 +398,15 @@ extern "C" int jsc_batch_set_aero(jsc_batch *b, const aero_t *aero) {
     if (alti[i] > amax) amax = alti[i];
     if (alti[i] < amin) amin = alti[i];
   }
+  // room that does not depend on the layers
+  int st = JSC_OK;
+  if (!b->d_nlos_b) st = batch_dmalloc(b, &b->d_nlos_b, (size_t)b->max_rays);
+  if (!st && !b->d_los_off_b) st = batch_dmalloc(b, &b->d_los_off_b, (size_t)b->max_rays + 1);
+  if (!st && !b->h_aero && !(b->h_aero = (aero_t *)malloc(sizeof(aero_t)))) st = JSC_ERR_NOMEM;
+  if (st) {
+    free(alti);
+    return st;
+  }
   const size_t nh = 3 * NLMAX + (size_t)jl;
   double *h = (double *)calloc(nh > 0 ? nh : 1, sizeof(double));
   double *beta = (double *)calloc((size_t)3 * (nl > 0 ? nl : 1) * nd, sizeof(double));
@@ -388,21 +434,22 @@ extern "C" int jsc_batch_set_aero(jsc_batch *b, const aero_t *aero) {
   cudaFree(b->d_wt);
   b->d_aero = nullptr;
   b->d_beta = b->d_phase = b->d_wt = nullptr;
-  int st = jsc_dmalloc(&b->d_aero, nh);
-  if (!st) st = jsc_dmalloc(&b->d_beta, (size_t)3 * (nl > 0 ? nl : 1) * nd);
-  if (!st) st = jsc_dmalloc(&b->d_phase, (size_t)(nl > 0 ? nl : 1) * nd * NTHETA);
-  if (!st) st = jsc_dmalloc(&b->d_wt, (size_t)(nl > 0 ? nl : 1) * nd * (JSC_NTH_SCA + 1));
+  st = batch_dmalloc(b, &b->d_aero, nh);
+  if (!st) st = batch_dmalloc(b, &b->d_beta, (size_t)3 * (nl > 0 ? nl : 1) * nd);
+  if (!st) st = batch_dmalloc(b, &b->d_phase, (size_t)(nl > 0 ? nl : 1) * nd * NTHETA);
+  if (!st) st = batch_dmalloc(b, &b->d_wt, (size_t)(nl > 0 ? nl : 1) * nd * (JSC_NTH_SCA + 1));
   if (!st && cudaMemcpy(b->d_aero, h, nh * sizeof(double), cudaMemcpyHostToDevice) != cudaSuccess) st = JSC_ERR_CUDA;
   if (!st && cudaMemcpy(b->d_beta, beta, (size_t)3 * (nl > 0 ? nl : 1) * nd * sizeof(double),
                         cudaMemcpyHostToDevice) != cudaSuccess) st = JSC_ERR_CUDA;
   if (!st && cudaMemcpy(b->d_phase, phase, (size_t)(nl > 0 ? nl : 1) * nd * NTHETA * sizeof(double),
                         cudaMemcpyHostToDevice) != cudaSuccess) st = JSC_ERR_CUDA;
   free(alti); free(h); free(beta); free(phase);
-  if (st) {
+  if (st) {  // no layers then: a run asks for them
+    cudaFree(b->d_aero);
+    b->d_aero = nullptr;
     jsc_set_error(st, "jsc_batch_set_aero: device upload failed");
     return st;
   }
-  if (!b->h_aero && !(b->h_aero = (aero_t *)malloc(sizeof(aero_t)))) return JSC_ERR_NOMEM;
   if (b->h_aero != aero) memcpy(b->h_aero, aero, sizeof(aero_t));
   b->aero_nl = nl;
   b->n_alti = jl;
@@ -411,10 +458,6 @@ extern "C" int jsc_batch_set_aero(jsc_batch *b, const aero_t *aero) {
   // child batches (secondary and solar pencils) see the same layers
   for (jsc_batch *c : {b->child, b->sun_child})
     if (c && (st = jsc_batch_set_aero(c, aero))) return st;
-  if (!b->d_nlos_b) {
-    if ((st = jsc_dmalloc(&b->d_nlos_b, (size_t)b->max_rays))) return st;
-    if ((st = jsc_dmalloc(&b->d_los_off_b, (size_t)b->max_rays + 1))) return st;
-  }
   return JSC_OK;
 }
 
@@ -422,9 +465,10 @@ static int batch_alloc_los_b(jsc_batch *b, int64_t max_seg) {
   cudaFree(b->d_geo_b);
   cudaFree(b->d_pts_b);
   b->d_geo_b = b->d_pts_b = nullptr;
+  b->max_seg_b = 0;
   int st;
-  if ((st = jsc_dmalloc(&b->d_geo_b, (size_t)max_seg * 4))) return st;
-  if ((st = jsc_dmalloc(&b->d_pts_b, (size_t)max_seg * b->W))) return st;
+  if ((st = batch_dmalloc(b, &b->d_geo_b, (size_t)max_seg * 4))) return st;
+  if ((st = batch_dmalloc(b, &b->d_pts_b, (size_t)max_seg * b->W))) return st;
   b->max_seg_b = max_seg;
   return JSC_OK;
 }
@@ -879,9 +923,9 @@ static int reserve_points(jsc_batch *b, int64_t n_sp) {
   b->d_sp_atm = nullptr;
   b->max_sp = 0;
   const int64_t n = n_sp + n_sp / 4 + 256;
-  if ((st = jsc_dmalloc(&b->d_sp, (size_t)n * JSC_SP_REC))) return st;
-  if ((st = jsc_dmalloc(&b->d_sp_atm, (size_t)n))) return st;
-  if ((st = jsc_dmalloc(&b->d_src, (size_t)n * b->cfg.nd))) return st;
+  if ((st = batch_dmalloc(b, &b->d_sp, (size_t)n * JSC_SP_REC))) return st;
+  if ((st = batch_dmalloc(b, &b->d_sp_atm, (size_t)n))) return st;
+  if ((st = batch_dmalloc(b, &b->d_src, (size_t)n * b->cfg.nd))) return st;
   b->max_sp = n;
   return JSC_OK;
 }
@@ -892,19 +936,24 @@ static int reserve_sp_idx(jsc_batch *b) {
   cudaFree(b->d_sp_idx);
   b->d_sp_idx = nullptr;
   b->sp_idx_seg = 0;
-  int st = jsc_dmalloc(&b->d_sp_idx, (size_t)b->max_seg);
+  int st = batch_dmalloc(b, &b->d_sp_idx, (size_t)b->max_seg);
   if (!st) b->sp_idx_seg = b->max_seg;
+  return st;
+}
+
+// Room for the scattering-point counts of the rays and their prefix sum.
+static int reserve_counts(jsc_batch *b) {
+  int st = JSC_OK;
+  if (!b->d_nsp) st = batch_dmalloc(b, &b->d_nsp, (size_t)b->max_rays);
+  if (!st && !b->d_sp_off) st = batch_dmalloc(b, &b->d_sp_off, (size_t)b->max_rays + 1);
   return st;
 }
 
 // Scattering points per ray and their list (src/forwardmodel.c:317-331).
 static int list_scattering_points(jsc_batch *b, cudaStream_t s) {
   const int nr = b->n_rays;
-  int st;
-  if (!b->d_nsp) {
-    if ((st = jsc_dmalloc(&b->d_nsp, (size_t)b->max_rays))) return st;
-    if ((st = jsc_dmalloc(&b->d_sp_off, (size_t)b->max_rays + 1))) return st;
-  }
+  int st = reserve_counts(b);
+  if (st) return st;
   SpArgs sa;
   sa.n_rays = nr;
   sa.W = b->W;
@@ -1225,10 +1274,7 @@ static int prepare_fixed_scattering(jsc_batch *b) {
   b->fx_chunk = chunk;
   b->fx_rounds = (int)((want + chunk - 1) / chunk);
   b->fx_max_sp = (int64_t)b->fx_rounds * chunk;
-  if (!b->d_nsp) {
-    if ((st = jsc_dmalloc(&b->d_nsp, (size_t)b->max_rays))) return st;
-    if ((st = jsc_dmalloc(&b->d_sp_off, (size_t)b->max_rays + 1))) return st;
-  }
+  if ((st = reserve_counts(b))) return st;
   if ((st = reserve_points(b, b->fx_max_sp))) return st;
   if ((st = reserve_sp_idx(b))) return st;
   if (!b->d_sp_listed && (st = jsc_dmalloc(&b->d_sp_listed, 1))) return st;
@@ -1874,7 +1920,9 @@ static int batch_run(jsc_batch *b, cudaStream_t s) {
   }
   ev_record(b, JSC_T_RAYTRACE, 0, s);
   {
-    const int st = b->ip == 1 ? los_profile(b, refine, s) : los_geo(b, refine, s);
+    int st = batch_ensure_los(b);
+    if (st) return st;
+    st = b->ip == 1 ? los_profile(b, refine, s) : los_geo(b, refine, s);
     if (st) return st;
   }
   if (b->fixed && b->ip != 1) {

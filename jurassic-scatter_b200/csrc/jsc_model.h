@@ -188,6 +188,8 @@ struct jsc_batch {
   double *d_pts;            // [max_seg][W]: p t ds qh2o k[nw] u[ng]
   double *d_ctm, *d_srcp;   // [ctm_seg][nd]: continuum extinction, Planck source
   int64_t ctm_seg;
+  int64_t seg_req;          // LOS points asked for at creation
+  int fail_alloc;           // the allocation from now that fails (tests), 0: none
   int64_t n_points;         // LOS points of the current run
   int64_t *d_npts;          // [1] of them inside the buffers (fixed-capacity runs)
   int np_longest;           // of its longest ray (before layer edges); 0: not known

@@ -30,7 +30,7 @@ EXPORTS = [
     "formod_pencil", "formod_fov", "read_shape", "read_tbl", "srcfunc_planck",
     "formod_continua", "intpol_tbl", "intpol_tbl_eps", "intpol_tbl_u", "locate_tbl",
     "jsc_srcfunc_sca", "jsc_batch_scatter_points", "jsc_surrogate_get_scaling",
-    "jsc_batch_set_nalpha_depth", "jsc_batch_set_wait_budget", "jsc_scan_selftest",
+    "jsc_batch_set_nalpha_depth", "jsc_batch_set_wait_budget", "jsc_scan_selftest", "jsc_batch_fail_alloc",
     "jsc_batch_set_fixed_points", "jsc_batch_set_surrogate_depth",
     "jsc_batch_scatter_samples_depth", "jsc_batch_surrogate_stats_depth",
 ]
@@ -154,6 +154,7 @@ def load():
         "jsc_batch_set_nalpha_depth": (i, [vp, i, i]),
         "jsc_batch_set_wait_budget": (i, [vp, C.c_uint]),
         "jsc_scan_selftest": (i, [i, i, C.c_uint, i]),
+        "jsc_batch_fail_alloc": (i, [vp, i]),
         "jsc_batch_set_fixed_points": (i, [vp, C.c_int64]),
         "jsc_batch_set_surrogate_depth": (i, [vp, i, vp, d, i]),
         "jsc_batch_scatter_samples_depth": (i, [vp, i, P(C.c_float), P(d), C.c_int64,

@@ -255,3 +255,78 @@ def test_one_ray_above_the_default_capacity(workdir):
     out = api.formod_batch(ctl, inp, aero=layers)
     assert out["nlos"][0] > 512
     assert np.all(out["rad"] > 0)
+
+
+def _curtain(workdir, ip, n, mult=None):
+    from jscat import synth, structs as S
+    ctlkw, atm, geom = synth.curtain_case(workdir)
+    geom = {k: v[:n] for k, v in geom.items()}
+    kw, layers = dict(ctlkw, ip=ip), None
+    if mult is not None:
+        layers = S.AeroT.from_buffer_copy(np.load(os.path.join(GOLDEN, "aero_ice8.npz"))["aero"].tobytes())
+        kw.update(sca_n=1, sca_mult=mult)
+    atms = [{k: v[..., 121 * i:121 * i + 121] for k, v in atm.items()} for i in range(5)]
+    return S.make_ctl(**kw), synth.batch_from(atms, np.zeros(n, np.int32), geom), layers
+
+
+@pytest.mark.parametrize("ip,mult", [(1, None), (1, 0), (1, 1), (2, None), (2, 0)])
+def test_run_after_a_failed_growth(workdir, ip, mult):
+    """Each allocation of a run whose buffers have to grow fails in turn
+    (an error code on the host, before any use of the memory): the call
+    reports it, and the next one allocates again and gives the results."""
+    from jscat import api, lib as L
+    ctl, inp, layers = _curtain(workdir, ip, 3, mult)
+    m, lib = api.Model(ctl), L.load()
+    want = api.formod_batch(ctl, inp, model=m, aero=layers)
+    failed = 0
+    for k in range(1, 40):
+        b = api.Batch(m, ctl, len(inp["atm_off"]) - 1, len(inp["z"]), 3, max_seg=1)
+        try:
+            if layers is not None:
+                b.set_aero(layers)
+            b.upload(inp)
+            L.check(lib.jsc_batch_fail_alloc(b.h, k))
+            try:
+                b.run()
+            except L.JscError as e:
+                assert e.status == 10   # JSC_ERR_NOMEM
+                failed += 1
+            else:
+                break
+            b.run()
+            got = b.download()
+            for c in KEYS:
+                np.testing.assert_array_equal(got[c], want[c])
+        finally:
+            b.close()
+    assert failed == {(1, None): 6, (1, 0): 6, (1, 1): 12, (2, None): 4, (2, 0): 6}[ip, mult]
+
+
+def test_layers_after_a_failed_allocation(workdir):
+    """jsc_batch_set_aero with each of its allocations failing in turn: no
+    run takes half of the layers, and the next call sets them."""
+    from jscat import api, lib as L
+    ctl, inp, layers = _case(workdir, 2, 5, True)
+    m, lib = api.Model(ctl), L.load()
+    want = api.formod_batch(ctl, inp, model=m, aero=layers)
+    for before in (False, True):
+        for k in range(3 if before else 1, 7):
+            b = api.Batch(m, ctl, 2, len(inp["z"]), 5)
+            try:
+                if before:
+                    b.set_aero(layers)
+                L.check(lib.jsc_batch_fail_alloc(b.h, k - 2 if before else k))
+                with pytest.raises(L.JscError) as e:
+                    b.set_aero(layers)
+                assert e.value.status == 10
+                b.upload(inp)
+                with pytest.raises(L.JscError) as e:
+                    b.run()
+                assert e.value.status == 1   # JSC_ERR_ARG: a run with layers needs them
+                b.set_aero(layers)
+                b.run()
+                got = b.download()
+                for c in KEYS:
+                    np.testing.assert_array_equal(got[c], want[c])
+            finally:
+                b.close()
