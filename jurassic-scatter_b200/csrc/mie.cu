@@ -269,8 +269,10 @@ extern "C" int jsc_mie_eval(int device, int n, const double *x, const double *nr
   const size_t sh = shared ? sizeof(double) * kTerm * cap : 0;
   fail(cudaMalloc(&d, (nin + nout + 1) * sizeof(double)), "cudaMalloc");
   if (!shared) fail(cudaMalloc(&dterm, sizeof(double) * kTerm * cap * (size_t)(n < kScratchTasks ? n : kScratchTasks)), "cudaMalloc");
+  // the largest size always: the attribute is shared by all threads of the process
   if (sh > 48 * 1024)
-    fail(cudaFuncSetAttribute(mie_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sh),
+    fail(cudaFuncSetAttribute(mie_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              kSharedOrders * kTerm * (int)sizeof(double)),
          "shared memory");
   if (!st) {
     double *dc = d + ((3 * (size_t)n + 1) & ~(size_t)1);  // 16-byte aligned, as in the copies below
