@@ -499,8 +499,8 @@ void jsc_batch_set_timing(jsc_batch *b, int on);
 double jsc_batch_kernel_ms(const jsc_batch *b, const char *kernel);
 
 /* Launch autotuner: runs the batch once, then times every launch variant
- * of the EGA/radiative-transfer kernel (threads per block x register
- * budget) on it and keeps the fastest for later runs of this batch.
+ * of the EGA and radiative transfer on it, with all that a run launches for
+ * the variant, and keeps the fastest for later runs of this batch.
  * jsc_batch_variant reports the choice. */
 int jsc_batch_autotune(jsc_batch *b, void *stream);
 int jsc_batch_variant(const jsc_batch *b, int *variant, int *block, int *min_blocks);

@@ -691,6 +691,11 @@ static const int kEgaWide = 22;
 static const int kEgaNoWidths = 17;
 static const int64_t kGasNarrow = 2048;
 
+// Variant v as b's tables allow it.
+static int resolved(const jsc_batch *b, int v) {
+  return gas_variant(v) && !b->m->dv.grid_dt ? kEgaNoWidths : v;
+}
+
 // The variant a run of b launches (-1 resolves to the default for its
 // configuration).
 static int run_variant(const jsc_batch *b) {
@@ -700,7 +705,7 @@ static int run_variant(const jsc_batch *b) {
     const int64_t warps = (rays + 31) / 32 * b->cfg.nd * (b->cfg.ng > 0 ? b->cfg.ng : 1);
     v = warps <= kGasNarrow ? kEgaDefault : kEgaWide;
   }
-  return gas_variant(v) && !b->m->dv.grid_dt ? kEgaNoWidths : v;
+  return resolved(b, v);
 }
 
 static bool lane_variant(int variant) {
@@ -742,12 +747,11 @@ static int launch_gas(jsc_batch *b, const EgaArgs &ea, int lanes, cudaStream_t s
   return JSC_OK;
 }
 
-static int launch_ega(jsc_batch *b, const EgaArgs &ea, int nr, int ndp, int ng, int variant,
+static int launch_ega(jsc_batch *b, const EgaArgs &ea, int nr, int ndp, int ng, int v,
                       cudaStream_t s) {
   const int64_t threads = (int64_t)nr * ndp;
   const unsigned g128 = (unsigned)((threads + 127) / 128);
   const unsigned g256 = (unsigned)((threads + 255) / 256);
-  const int v = gas_variant(variant) && !b->m->dv.grid_dt ? kEgaNoWidths : variant;
   const bool dig = ea.digest != nullptr;  // index digests (every variant has them)
   if (gas_variant(v)) return launch_gas(b, ea, kEgaVariants[v].minb, s);
   if (kEgaVariants[v].ray && ray_warps(ng) && ea.order) {
@@ -1901,6 +1905,45 @@ static int los_geo(jsc_batch *b, bool refine, cudaStream_t s) {
   return JSC_OK;
 }
 
+// Everything that a run launches for a variant (resolved by run_variant): the
+// order of the rays, the continuum pass, the EGA and transfer.
+static int ega_passes(jsc_batch *b, EgaArgs ea, int variant, cudaStream_t s) {
+  if (gas_variant(variant) || (kEgaVariants[variant].ray && ray_warps(b->m->ng))) {
+    const int e = jsc_ray_order(ea.n_rays, b->d_ray_atm, b->d_nlos, b->d_tsurf, b->d_tp, b->d_rkeys,
+                                b->d_rorder, b->d_rtmp, b->rtmp_bytes, s);
+    if (e) {
+      jsc_set_error(JSC_ERR_CUDA, "ray order: %s", cudaGetErrorString((cudaError_t)e));
+      return JSC_ERR_CUDA;
+    }
+    ea.order = b->d_rorder;
+  }
+  if (lane_variant(variant)) {
+    // continuum extinction and Planck source per (LOS point, channel)
+    CtmArgs ca;
+    ca.m = ea.m;
+    ca.cfg = ea.cfg;
+    ca.n_points = b->n_points;
+    ca.W = ea.W;
+    ca.pts = ea.pts;
+    ca.beta = b->d_ctm;
+    ca.src = b->d_srcp;
+    ca.n_live = b->fixed ? b->d_npts : nullptr;
+    ev_record(b, JSC_T_CTM, 0, s);
+    if (b->fixed) {
+      live_records_kernel<<<1, 1, 0, s>>>(b->d_los_off + ea.n_rays, b->max_seg, b->d_npts);
+      JSC_LAUNCH_CHECK();
+    }
+    jsc_ctm_src_launch(ca, s);
+    JSC_LAUNCH_CHECK();
+    ev_record(b, JSC_T_CTM, 1, s);
+  }
+  ev_record(b, JSC_T_EGA, 0, s);
+  const int st = launch_ega(b, ea, ea.n_rays, ea.ndp, b->m->ng, variant, s);
+  if (st) return st;
+  ev_record(b, JSC_T_EGA, 1, s);
+  return JSC_OK;
+}
+
 static int batch_run(jsc_batch *b, cudaStream_t s) {
   const jsc_model *m = b->m;
   const int nr = b->n_rays;
@@ -1969,42 +2012,9 @@ static int batch_run(jsc_batch *b, cudaStream_t s) {
   ea.beta_ctm = b->d_ctm;
   ea.src_pl = b->d_srcp;
   ea.order = nullptr;
-  const int variant = run_variant(b);
-  if (gas_variant(variant) || (kEgaVariants[variant].ray && ray_warps(m->ng))) {
-    int e = jsc_ray_order(nr, b->d_ray_atm, b->d_nlos, b->d_tsurf, b->d_tp, b->d_rkeys,
-                          b->d_rorder, b->d_rtmp, b->rtmp_bytes, s);
-    if (e) {
-      jsc_set_error(JSC_ERR_CUDA, "ray order: %s", cudaGetErrorString((cudaError_t)e));
-      return JSC_ERR_CUDA;
-    }
-    ea.order = b->d_rorder;
-  }
-  if (lane_variant(variant)) {
-    // continuum extinction and Planck source per (LOS point, channel)
-    CtmArgs ca;
-    ca.m = m->dv;
-    ca.cfg = b->cfg;
-    ca.n_points = b->n_points;
-    ca.W = b->W;
-    ca.pts = b->d_pts;
-    ca.beta = b->d_ctm;
-    ca.src = b->d_srcp;
-    ca.n_live = b->fixed ? b->d_npts : nullptr;
-    ev_record(b, JSC_T_CTM, 0, s);
-    if (b->fixed) {
-      live_records_kernel<<<1, 1, 0, s>>>(b->d_los_off + nr, b->max_seg, b->d_npts);
-      JSC_LAUNCH_CHECK();
-    }
-    jsc_ctm_src_launch(ca, s);
-    JSC_LAUNCH_CHECK();
-    ev_record(b, JSC_T_CTM, 1, s);
-  }
   b->last_ega = ea;
-  ev_record(b, JSC_T_EGA, 0, s);
-  int st = launch_ega(b, ea, nr, ndp, m->ng, variant, s);
+  int st = ega_passes(b, ea, run_variant(b), s);
   if (st) return st;
-  JSC_LAUNCH_CHECK();
-  ev_record(b, JSC_T_EGA, 1, s);
   // LOS point total for the work counters.
   JSC_CUDA_TRY(cudaMemcpyAsync(b->d_counters, b->d_los_off + nr, sizeof(int64_t),
                                cudaMemcpyDeviceToDevice, s));
@@ -2088,20 +2098,10 @@ extern "C" int jsc_batch_index_digest(jsc_batch *b, uint64_t *out) {
 extern "C" int jsc_batch_autotune(jsc_batch *b, void *stream) {
   if (!b || b->n_rays < 1) return JSC_ERR_ARG;
   cudaStream_t s = (cudaStream_t)stream;
-  b->ega_variant = kLaneBase;  // a lane variant also fills the continuum arrays
   int st = jsc_batch_run(b, stream);  // LOS records for the timing runs
   if (st) return st;
   EgaArgs ea = b->last_ega;
   ea.digest = nullptr;
-  {
-    int e = jsc_ray_order(b->n_rays, b->d_ray_atm, b->d_nlos, b->d_tsurf, b->d_tp, b->d_rkeys,
-                          b->d_rorder, b->d_rtmp, b->rtmp_bytes, s);
-    if (e) {
-      jsc_set_error(JSC_ERR_CUDA, "ray order: %s", cudaGetErrorString((cudaError_t)e));
-      return JSC_ERR_CUDA;
-    }
-    ea.order = b->d_rorder;
-  }
   cudaEvent_t e0 = nullptr, e1 = nullptr;
   JSC_CUDA_TRY(cudaEventCreate(&e0));
   if (cudaEventCreate(&e1) != cudaSuccess) {
@@ -2113,7 +2113,7 @@ extern "C" int jsc_batch_autotune(jsc_batch *b, void *stream) {
   float best_ms = 1e30f;
   for (int v = 0; v < kNumEgaVariants && !st; v++) {
     cudaError_t e = cudaEventRecord(e0, s);
-    if (e == cudaSuccess) st = launch_ega(b, ea, b->n_rays, ea.ndp, b->m->ng, v, s);
+    if (e == cudaSuccess) st = ega_passes(b, ea, resolved(b, v), s);
     if (!st && e == cudaSuccess) e = cudaEventRecord(e1, s);
     if (!st && e == cudaSuccess) e = cudaEventSynchronize(e1);
     float ms = -1;
