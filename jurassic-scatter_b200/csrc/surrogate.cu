@@ -566,58 +566,54 @@ extern "C" int jsc_surrogate_loss_grad(jsc_surrogate *s, const float *x, const f
   return JSC_OK;
 }
 
+// Sums over the training set of the parts that train_stats_kernel left.
+static int stats_sums(int nblk, int nc, const double *part, double *sum, double *out) {
+  train_stats_sum_kernel<<<1, TR_STATS * SUR_NOUT_MAX>>>(nblk, nc, part, sum);
+  JSC_LAUNCH_CHECK();
+  JSC_CUDA_TRY(cudaMemcpy(out, sum, (size_t)TR_STATS * nc * sizeof(double), cudaMemcpyDeviceToHost));
+  return JSC_OK;
+}
+
 // Training set to the device: features as they are, the logarithms of the
 // sources standardised; the standardisations and the envelope of the features.
-static int standardise(jsc_surrogate *s, const float *X, const double *src, int64_t n) {
+// y: room for the logarithms, then the statistics' parts and sums.
+static int standardise(jsc_surrogate *s, const float *X, const double *src, int64_t n, int nblk,
+                       double *y) {
   const int nd = s->nout;
   const int64_t cnt = n * nd;
-  const int nblk = (int)(n < TR_STAT_BLOCKS ? n : TR_STAT_BLOCKS);
   double fx[TR_STATS][SUR_NF], fy[TR_STATS * SUR_NOUT_MAX];
-  double *y = nullptr;  // logarithms, then the statistics' parts and sums
-  int st = jsc_dmalloc(&y, (size_t)cnt + (size_t)(nblk + 1) * TR_STATS * SUR_NOUT_MAX);
-  if (st) return st;
   double *part = y + cnt, *sum = part + (size_t)nblk * TR_STATS * SUR_NOUT_MAX;
-  auto stats = [&](int nc, double *out) {  // parts to host sums
-    train_stats_sum_kernel<<<1, TR_STATS * SUR_NOUT_MAX>>>(nblk, nc, part, sum);
-    return cudaGetLastError() ||
-           cudaMemcpy(out, sum, (size_t)TR_STATS * nc * sizeof(double), cudaMemcpyDeviceToHost);
-  };
-  bool bad = cudaMemcpy(s->d_X, X, (size_t)n * SUR_NF * sizeof(float), cudaMemcpyHostToDevice);
-  if (!bad) {
-    train_stats_kernel<float, false><<<nblk, TR_THREADS>>>(n, SUR_NF, s->d_X, part);
-    bad = stats(SUR_NF, fx[0]);
+  int st;
+  JSC_CUDA_TRY(cudaMemcpy(s->d_X, X, (size_t)n * SUR_NF * sizeof(float), cudaMemcpyHostToDevice));
+  train_stats_kernel<float, false><<<nblk, TR_THREADS>>>(n, SUR_NF, s->d_X, part);
+  JSC_LAUNCH_CHECK();
+  if ((st = stats_sums(nblk, SUR_NF, part, sum, fx[0]))) return st;
+  JSC_CUDA_TRY(cudaMemcpy(y, src, (size_t)cnt * sizeof(double), cudaMemcpyHostToDevice));
+  train_stats_kernel<double, true><<<nblk, TR_THREADS>>>(n, nd, y, part);
+  JSC_LAUNCH_CHECK();
+  if ((st = stats_sums(nblk, nd, part, sum, fy))) return st;
+  for (int c = 0; c < SUR_NF; c++) {
+    const double m = fx[0][c] / n, var = fx[1][c] / n - m * m;
+    const float lo = (float)fx[2][c], hi = (float)fx[3][c], w = 0.02f * (hi - lo);
+    s->xm[c] = (float)m;
+    s->xs[c] = var > 1e-12 ? (float)sqrt(var) : 1.f;
+    s->lo[c] = lo - w;
+    s->hi[c] = hi + w;
   }
-  bad = bad || cudaMemcpy(y, src, (size_t)cnt * sizeof(double), cudaMemcpyHostToDevice);
-  if (!bad) {
-    train_stats_kernel<double, true><<<nblk, TR_THREADS>>>(n, nd, y, part);
-    bad = stats(nd, fy);
+  for (int d = 0; d < nd; d++) {
+    const double m = fy[d] / n, var = fy[nd + d] / n - m * m;
+    fy[d] = m;
+    s->h_ym[d] = (float)m;
+    s->h_ys[d] = var > 1e-12 ? (float)sqrt(var) : 1.f;
   }
-  if (!bad) {
-    for (int c = 0; c < SUR_NF; c++) {
-      const double m = fx[0][c] / n, var = fx[1][c] / n - m * m;
-      const float lo = (float)fx[2][c], hi = (float)fx[3][c], w = 0.02f * (hi - lo);
-      s->xm[c] = (float)m;
-      s->xs[c] = var > 1e-12 ? (float)sqrt(var) : 1.f;
-      s->lo[c] = lo - w;
-      s->hi[c] = hi + w;
-    }
-    for (int d = 0; d < nd; d++) {
-      const double m = fy[d] / n, var = fy[nd + d] / n - m * m;
-      fy[d] = m;
-      s->h_ym[d] = (float)m;
-      s->h_ys[d] = var > 1e-12 ? (float)sqrt(var) : 1.f;
-    }
-    bad = cudaMemcpy(sum, fy, nd * sizeof(double), cudaMemcpyHostToDevice) ||
-          cudaMemcpy(s->d_ym, s->h_ym, nd * sizeof(float), cudaMemcpyHostToDevice) ||
-          cudaMemcpy(s->d_ys, s->h_ys, nd * sizeof(float), cudaMemcpyHostToDevice);
-  }
-  if (!bad) {
-    train_targets_kernel<<<(unsigned)((cnt + TR_THREADS - 1) / TR_THREADS), TR_THREADS>>>(
-        cnt, nd, y, sum, s->d_ys, s->d_T);
-    bad = cudaGetLastError() || cudaDeviceSynchronize();
-  }
-  cudaFree(y);
-  return bad ? JSC_ERR_CUDA : JSC_OK;
+  JSC_CUDA_TRY(cudaMemcpy(sum, fy, nd * sizeof(double), cudaMemcpyHostToDevice));
+  JSC_CUDA_TRY(cudaMemcpy(s->d_ym, s->h_ym, nd * sizeof(float), cudaMemcpyHostToDevice));
+  JSC_CUDA_TRY(cudaMemcpy(s->d_ys, s->h_ys, nd * sizeof(float), cudaMemcpyHostToDevice));
+  train_targets_kernel<<<(unsigned)((cnt + TR_THREADS - 1) / TR_THREADS), TR_THREADS>>>(
+      cnt, nd, y, sum, s->d_ys, s->d_T);
+  JSC_LAUNCH_CHECK();
+  JSC_CUDA_TRY(cudaDeviceSynchronize());
+  return JSC_OK;
 }
 
 extern "C" int jsc_surrogate_train(jsc_surrogate *s, const float *X, const double *src,
@@ -628,8 +624,11 @@ extern "C" int jsc_surrogate_train(jsc_surrogate *s, const float *X, const doubl
     return JSC_ERR_ARG;
   }
   JSC_CUDA_TRY(cudaSetDevice(s->device));
+  (void)cudaGetLastError();  // launch checks below report this call's errors only
   const int nd = s->nout;
   // Standardisation and envelope from the training set.
+  const int nblk = (int)(n < TR_STAT_BLOCKS ? n : TR_STAT_BLOCKS);
+  double *y = nullptr;
   int st = JSC_OK;
   cudaFree(s->d_X);
   cudaFree(s->d_T);
@@ -639,7 +638,9 @@ extern "C" int jsc_surrogate_train(jsc_surrogate *s, const float *X, const doubl
   st = st ? st : jsc_dmalloc(&s->d_X, (size_t)n * SUR_NF);
   st = st ? st : jsc_dmalloc(&s->d_T, (size_t)n * nd);
   st = st ? st : jsc_dmalloc(&s->d_perm, (size_t)n);
-  st = st ? st : standardise(s, X, src, n);
+  st = st ? st : jsc_dmalloc(&y, (size_t)n * nd + (size_t)(nblk + 1) * TR_STATS * SUR_NOUT_MAX);
+  st = st ? st : standardise(s, X, src, n, nblk, y);
+  cudaFree(y);
   if (st) return st;
   s->n_train = n;
   if ((st = ensure_train(s, batch))) return st;
