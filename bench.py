@@ -942,16 +942,21 @@ def optprop_bench(args, torch, cpu=True):
             from oracle import refrun
             ctlkw = dict(emitters=synth.CFG0_EMITTERS, nus=nus, tblbase="-", sca_n=sca_n,
                          sca_mult=1)
-            ref = refrun.reference_aero(ctlkw, f, os.path.dirname(f), timed=True)
-            ra = S.AeroT.from_buffer_copy(ref["aero"])
-            nl, nd = ra.nl, len(nus)
-            got = np.concatenate([S.arr(aero.beta_e)[:nl, :nd].ravel(),
-                                  S.arr(aero.p)[:nl, :nd].ravel()])
-            want = np.concatenate([S.arr(ra.beta_e)[:nl, :nd].ravel(),
-                                   S.arr(ra.p)[:nl, :nd].ravel()])
-            row["reference_cpu_ms"] = 1e3 * ref["seconds"]
-            row["max_rel_err_vs_reference"] = float(np.max(np.abs(got - want) /
-                                                           np.maximum(np.abs(want), 1e-300)))
+            try:
+                ref = refrun.reference_aero(ctlkw, f, os.path.dirname(f), timed=True)
+            except Exception as exc:  # no reference here: the GPU times stay
+                row["reference_error"] = str(exc)[:300]
+                ref = None
+            if ref is not None:
+                ra = S.AeroT.from_buffer_copy(ref["aero"])
+                nl, nd = ra.nl, len(nus)
+                got = np.concatenate([S.arr(aero.beta_e)[:nl, :nd].ravel(),
+                                      S.arr(aero.p)[:nl, :nd].ravel()])
+                want = np.concatenate([S.arr(ra.beta_e)[:nl, :nd].ravel(),
+                                       S.arr(ra.p)[:nl, :nd].ravel()])
+                row["reference_cpu_ms"] = 1e3 * ref["seconds"]
+                row["max_rel_err_vs_reference"] = float(np.max(np.abs(got - want) /
+                                                               np.maximum(np.abs(want), 1e-300)))
         res.append(row)
     return {"workload": "get_opt_prop of the benchmark's aerosol/cloud layers", "cases": res,
             "timing": "host wall clock around jsc_get_opt_prop (aero_t in host memory)",
