@@ -1088,6 +1088,7 @@ static int plain_sources(jsc_batch *b, const double *sp, const int *sp_atm, int6
   const int64_t per_pt = three_d ? JSC_NDIR3 : na;
   if ((st = ensure_child(b, &b->child, (int)(chunk * per_pt), b->depth - 1))) return st;
   if ((st = ensure_child(b, &b->sun_child, (int)chunk, 0))) return st;
+  b->child->fixed = b->sun_child->fixed = 0;  // an earlier run may have been a fixed one
   if (!b->d_planck_sun) {
     double h[NDMAX];
     for (int id = 0; id < nd; id++) h[id] = planck(JSC_TSUN, b->m->nu[id]);
@@ -1183,6 +1184,7 @@ static int plain_sources(jsc_batch *b, const double *sp, const int *sp_atm, int6
 static int fixed_sources(jsc_batch *b, cudaStream_t s) {
   const int nr = b->n_rays, nd = b->cfg.nd, na = b->nalpha;
   int st;
+  b->child->fixed = b->sun_child->fixed = 1;
   SpArgs sa;
   sa.n_rays = nr;
   sa.W = b->W;
@@ -1579,7 +1581,18 @@ extern "C" int jsc_batch_scatter_points(jsc_batch *b, int n, const double *x, co
   }
   b->n_sp = n;
   if ((st = run_hydro(b, s))) return st;
-  if ((st = plain_sources(b, b->d_sp, b->d_sp_atm, n, b->d_src, s))) return st;
+  // a fixed-capacity batch keeps the children that its runs need: these pencils
+  // get their own
+  jsc_batch *const child = b->child, *const sun_child = b->sun_child;
+  if (b->fixed) b->child = b->sun_child = nullptr;
+  st = plain_sources(b, b->d_sp, b->d_sp_atm, n, b->d_src, s);
+  if (b->fixed) {
+    jsc_batch_destroy(b->child);
+    jsc_batch_destroy(b->sun_child);
+    b->child = child;
+    b->sun_child = sun_child;
+  }
+  if (st) return st;
   unsigned status = 0;
   JSC_CUDA_TRY(cudaMemcpyAsync(src, b->d_src, (size_t)n * b->cfg.nd * sizeof(double),
                                cudaMemcpyDeviceToHost, s));
@@ -1695,7 +1708,7 @@ static int los_profile(jsc_batch *b, bool refine, cudaStream_t s) {
     xa.max_seg = b->max_seg;
     xa.max_count = b->fixed ? b->max_seg : INT64_MAX;  // else the buffers grow
     JSC_CUDA_TRY(cudaMemsetAsync(b->d_mcount, 0, 3 * sizeof(unsigned), s));
-    if (b->d_live) {
+    if (b->fixed && b->d_live) {
       // rays the queue leaves alone keep no LOS and no surface; a persistent
       // grid pulls the others
       JSC_CUDA_TRY(cudaMemsetAsync(ra.nlos, 0, (size_t)nr * sizeof(int), s));

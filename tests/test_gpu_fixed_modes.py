@@ -1,0 +1,105 @@
+"""A single-scattering batch between fixed-capacity and ordinary runs: each
+kind has its own way to run the secondary and solar pencils, and neither may
+take over what the other left."""
+import ctypes as C
+import os
+
+import numpy as np
+import pytest
+
+from conftest import GOLDEN
+
+pytestmark = pytest.mark.gpu
+
+KEYS = ("rad", "tau", "nlos")
+
+
+def _case(workdir, n):
+    from jscat import synth, structs as S
+    layers = S.AeroT.from_buffer_copy(np.load(os.path.join(GOLDEN, "aero_ice8.npz"))["aero"].tobytes())
+    atm = synth.atmosphere(synth.CFG0_EMITTERS, np.random.default_rng(3))
+    base = synth.write_tables(workdir, synth.CFG0_EMITTERS, synth.CFG0_NU, 20261203)
+    ctl = S.make_ctl(synth.CFG0_EMITTERS, synth.CFG0_NU[:2], base, hydz=0.0, sca_n=1, sca_mult=1)
+    geom = synth.limb_geometry(np.linspace(7.0, 10.5, n))
+    geom["time"][:] = 43200.0
+    return ctl, synth.batch_from([atm], np.zeros(n, np.int32), geom), layers
+
+
+def _above(inp, rays):
+    out = {k: np.array(v) for k, v in inp.items()}
+    out["vpz"][rays] = 130.0
+    return out
+
+
+def _run(b, inp):
+    b.upload(inp)
+    b.run()
+    return b.download()
+
+
+def test_ordinary_runs_after_fixed_ones(workdir):
+    """The last fixed run scatters at few points; the ordinary one after it
+    at all of them, and the fixed one after that again."""
+    from jscat import api, lib as L
+    ctl, inp, layers = _case(workdir, 4)
+    m, lib = api.Model(ctl), L.load()
+    few = _above(inp, np.arange(4) > 0)
+    want, wfew = (api.formod_batch(ctl, i, model=m, aero=layers) for i in (inp, few))
+    b = api.Batch(m, ctl, 1, len(inp["z"]), 4)
+    try:
+        b.set_aero(layers)
+        for _ in range(2):
+            L.check(lib.jsc_batch_set_fixed_points(b.h, 400))
+            L.check(lib.jsc_batch_set_fixed(b.h, 1))
+            got = _run(b, few)
+            for k in KEYS:
+                np.testing.assert_array_equal(got[k], wfew[k])
+            L.check(lib.jsc_batch_set_fixed(b.h, 0))
+            got = _run(b, inp)
+            for k in KEYS:
+                np.testing.assert_array_equal(got[k], want[k])
+    finally:
+        b.close()
+        m.close()
+
+
+def test_scatter_points_of_a_fixed_batch(workdir):
+    """jsc_batch_scatter_points on a batch in fixed-capacity mode, with fewer
+    and with more points than a round of its runs holds: the sources of an
+    ordinary batch, and the fixed runs go on."""
+    from jscat import api, synth, lib as L
+    ctl, inp, layers = _case(workdir, 2)
+    m, lib = api.Model(ctl), L.load()
+    few = _above(inp, [1])
+    wfew = api.formod_batch(ctl, few, model=m, aero=layers)
+    dp, ip = C.POINTER(C.c_double), C.POINTER(C.c_int)
+
+    def sources(b, n):
+        x = np.zeros((n, 3))
+        x[:, 0] = synth.RE + 9.0 + 0.01 * np.arange(n)
+        dx = np.tile([0.1, 1.0, 0.2], (n, 1))
+        layer, sec, src = np.zeros(n, np.int32), np.full(n, 43200.0), np.zeros((n, ctl.nd))
+        L.check(lib.jsc_batch_scatter_points(b.h, n, x.ctypes.data_as(dp), dx.ctypes.data_as(dp), layer.ctypes.data_as(ip),
+                                             sec.ctypes.data_as(dp), None, src.ctypes.data_as(dp), None))
+        return src
+
+    b, plain = (api.Batch(m, ctl, 1, len(inp["z"]), 2) for _ in range(2))
+    try:
+        for c in (b, plain):
+            c.set_aero(layers)
+            c.upload(inp)
+        L.check(lib.jsc_batch_set_fixed_points(b.h, 100))
+        L.check(lib.jsc_batch_set_fixed(b.h, 1))
+        for n in (3, 150):
+            got = _run(b, few)
+            for k in KEYS:
+                np.testing.assert_array_equal(got[k], wfew[k])
+            b.upload(inp)
+            np.testing.assert_array_equal(sources(b, n), sources(plain, n))
+        got = _run(b, few)
+        for k in KEYS:
+            np.testing.assert_array_equal(got[k], wfew[k])
+    finally:
+        b.close()
+        plain.close()
+        m.close()
