@@ -840,6 +840,7 @@ static __global__ void round_live_kernel(const unsigned long long *n_listed, int
 
 static int batch_run(jsc_batch *b, cudaStream_t s);
 static int run_hydro(jsc_batch *b, cudaStream_t s);
+static int fixed_unsupported();
 
 // Fixed-capacity runs (IP 2/3; IP 1: march_fit_kernel): rays whose line of
 // sight did not fit (the storing pass flagged them) keep only the points
@@ -1184,6 +1185,9 @@ static int plain_sources(jsc_batch *b, const double *sp, const int *sp_atm, int6
 static int fixed_sources(jsc_batch *b, cudaStream_t s) {
   const int nr = b->n_rays, nd = b->cfg.nd, na = b->nalpha;
   int st;
+  // jsc_batch_set_nalpha drops the pencils' batch
+  for (const jsc_batch *c : {b->child, b->sun_child})
+    if (!c || !c->d_live || !c->d_qhead) return fixed_unsupported();
   b->child->fixed = b->sun_child->fixed = 1;
   SpArgs sa;
   sa.n_rays = nr;

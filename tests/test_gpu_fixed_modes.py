@@ -103,3 +103,29 @@ def test_scatter_points_of_a_fixed_batch(workdir):
         b.close()
         plain.close()
         m.close()
+
+
+def test_pencil_count_after_fixed_mode(workdir):
+    """jsc_batch_set_nalpha drops what the fixed-capacity runs had prepared:
+    the next one says so, until jsc_batch_set_fixed prepares it again."""
+    from jscat import api, lib as L
+    ctl, inp, layers = _case(workdir, 2)
+    m, lib = api.Model(ctl), L.load()
+    want = api.formod_batch(ctl, inp, model=m, aero=layers, nalpha=10)
+    b = api.Batch(m, ctl, 1, len(inp["z"]), 2)
+    try:
+        b.set_aero(layers)
+        L.check(lib.jsc_batch_set_fixed_points(b.h, 200))
+        L.check(lib.jsc_batch_set_fixed(b.h, 1))
+        b.set_nalpha(10)
+        b.upload(inp)
+        with pytest.raises(L.JscError) as e:
+            b.run()
+        assert "jsc_batch_set_fixed" in str(e.value)
+        L.check(lib.jsc_batch_set_fixed(b.h, 1))
+        got = _run(b, inp)
+        for k in KEYS:
+            np.testing.assert_array_equal(got[k], want[k])
+    finally:
+        b.close()
+        m.close()
