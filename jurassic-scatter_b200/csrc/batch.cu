@@ -1854,7 +1854,6 @@ static int los_geo(jsc_batch *b, bool refine, cudaStream_t s) {
     fa.W = b->W;
     fa.n_levels = b->n_levels;
     fa.ig_h2o = m->dv.ig_h2o;
-    fa.ray_atm = b->d_ray_atm;
     fa.atm_off = b->d_atm_off;
     fa.z = b->d_z;
     fa.p = b->d_p;
@@ -1906,7 +1905,6 @@ static int los_geo(jsc_batch *b, bool refine, cudaStream_t s) {
     fa.geo = b->d_geo;
     fa.pts = b->d_pts;
     fa.max_seg = b->max_seg;
-    fa.ip = b->ip;
     fa.n_prof = b->n_atm;
     fa.psurf = b->d_psurf;
     fa.lat = b->d_lat;

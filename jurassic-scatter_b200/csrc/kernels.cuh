@@ -470,6 +470,7 @@ struct RayEnd {
 template <int MODE, int IP = 1>
 __device__ int trace_core(const RayArgs &A, int ai, int r, const RayIn &in, RayEnd *end) {
   constexpr bool STORE = MODE == 1;
+  static_assert(MODE != 2 || IP != 1, "IP 1: march_ray");
   const int lo = A.atm_off[ai];
   Profile a;
   a.n = A.atm_off[ai + 1] - lo;
@@ -712,9 +713,10 @@ __global__ void __launch_bounds__(128, 7) raytrace_kernel(RayArgs A) {
 
 // ------------------------------------------------------ aerosol layers --
 
+// Layer edges in horizontally varying atmospheres (IP 1: trace.cuh).
 struct RefineArgs {
   int n_rays, ng, nw, W, n_levels, ig_h2o;
-  const int *ray_atm, *atm_off;
+  const int *atm_off;
   const double *z, *p, *t, *q, *k;       // atmospheric profiles
   const int *nlos_b;                     // ray-traced LOS (raw records)
   const int64_t *off_b;
@@ -731,17 +733,16 @@ struct RefineArgs {
   const int *grid_nt;
   unsigned *status;
   // IP 2/3: as in RayArgs
-  int ip, n_prof;
+  int n_prof;
   const double *psurf, *lat;
   double cz, cx;
 };
 
 // Point where the segment between raw points ip-1 and ip crosses znew, with
 // the atmospheric state there (intersection_point, src/lineofsight.c:385-407).
-template <int IP = 1>
-__device__ __forceinline__ void refine_cross(const RefineArgs &A, const Profile &a,
-                                             const double *gb, int ip, double znew,
-                                             double *go, double *po) {
+template <int IP>
+__device__ __forceinline__ void refine_cross(const RefineArgs &A, const double *gb, int ip,
+                                             double znew, double *go, double *po) {
   double x1[3], x2[3], zz, lon, lat, p, t;
   const double *g0 = gb + (size_t)(ip - 1) * 4, *g1 = gb + (size_t)ip * 4;
   const double frac = (g0[0] - znew) / (g0[0] - g1[0]);
@@ -752,22 +753,13 @@ __device__ __forceinline__ void refine_cross(const RefineArgs &A, const Profile 
   go[0] = zz;
   go[1] = lon;
   go[2] = lat;
-  if (IP != 1) {
-    double qk[NGMAX + NWMAX];
-    atm_geo<IP>(geo_atm(A), zz, lon, lat, &p, &t, qk);
-    po[REC_P] = p;
-    po[REC_T] = t;
-    po[REC_QH2O] = A.ig_h2o >= 0 ? qk[A.ig_h2o] : 0.0;
-    for (int w = 0; w < A.nw; w++) po[REC_K + w] = qk[A.ng + w];
-    for (int g = 0; g < A.ng; g++) po[REC_K + A.nw + g] = qk[g];
-    return;
-  }
-  const int ipz = atm_full(a, zz, &p, &t);
+  double qk[NGMAX + NWMAX];
+  atm_geo<IP>(geo_atm(A), zz, lon, lat, &p, &t, qk);
   po[REC_P] = p;
   po[REC_T] = t;
-  po[REC_QH2O] = A.ig_h2o >= 0 ? atm_lin(a.q + (size_t)A.ig_h2o * a.stride, a, ipz, zz) : 0.0;
-  for (int w = 0; w < A.nw; w++) po[REC_K + w] = atm_lin(a.k + (size_t)w * a.stride, a, ipz, zz);
-  for (int g = 0; g < A.ng; g++) po[REC_K + A.nw + g] = atm_lin(a.q + (size_t)g * a.stride, a, ipz, zz);
+  po[REC_QH2O] = A.ig_h2o >= 0 ? qk[A.ig_h2o] : 0.0;
+  for (int w = 0; w < A.nw; w++) po[REC_K + w] = qk[A.ng + w];
+  for (int g = 0; g < A.ng; g++) po[REC_K + A.nw + g] = qk[g];
 }
 
 // Chord step length, column densities, (p, T) bracket, Planck index and
@@ -828,21 +820,6 @@ __device__ __forceinline__ void refine_point(const RefineArgs &A, int64_t base, 
   rec[REC_AI] = (double)aeroi;
 }
 
-// Profile of ray r's atmosphere.
-__device__ __forceinline__ Profile refine_profile(const RefineArgs &A, int r) {
-  const int ai = A.ray_atm[r];
-  const int lo = A.atm_off[ai];
-  Profile a;
-  a.n = A.atm_off[ai + 1] - lo;
-  a.stride = A.n_levels;
-  a.z = A.z + lo;
-  a.p = A.p + lo;
-  a.t = A.t + lo;
-  a.q = A.q + lo;
-  a.k = A.k + lo;
-  return a;
-}
-
 // STORE pass of the layer-edge refinement with a warp per ray (the COUNT
 // pass is refine_count_kernel): lanes take 32 raw points at a time, a
 // warp scan of their output counts (crossing points of the segment before
@@ -850,15 +827,15 @@ __device__ __forceinline__ Profile refine_profile(const RefineArgs &A, int r) {
 // writes them, the raw records are copied with coalesced loads, then lanes
 // take 32 refined points at a time for refine_point, with the neighbours'
 // Cartesian positions passed by shuffles.
-template <int IP = 1>
+template <int IP>
 __global__ void __launch_bounds__(128, 8) refine_store_kernel(RefineArgs A) {
+  static_assert(IP == 2 || IP == 3, "IP 1: expand_kernel");
   const int r = (int)(((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
   const int lane = threadIdx.x & 31;
   const unsigned full = 0xffffffffu;
   if (r >= A.n_rays) return;  // whole warps leave together
   const int nb = A.nlos_b[r];
   if (nb == 0) return;
-  const Profile a = refine_profile(A, r);
   const double *gb = A.geo_b + A.off_b[r] * 4, *pb = A.pts_b + A.off_b[r] * A.W;
   const int64_t base = A.off[r];
   // points to write; a ray that does not fit the buffers (a fixed-capacity
@@ -902,11 +879,11 @@ __global__ void __launch_bounds__(128, 8) refine_store_kernel(RefineArgs A) {
         for (int il = 0; il < A.n_alti; il++) {
           const double z1 = A.alti[il], z2 = A.alti[A.n_alti - il - 1];
           if (zp > z1 && zc < z1) {
-            refine_cross<IP>(A, a, gb, ip, z1, A.geo + (base + slot) * 4, A.pts + (base + slot) * W);
+            refine_cross<IP>(A, gb, ip, z1, A.geo + (base + slot) * 4, A.pts + (base + slot) * W);
             slot++;
           }
           if (zp < z2 && zc > z2) {
-            refine_cross<IP>(A, a, gb, ip, z2, A.geo + (base + slot) * 4, A.pts + (base + slot) * W);
+            refine_cross<IP>(A, gb, ip, z2, A.geo + (base + slot) * 4, A.pts + (base + slot) * W);
             slot++;
           }
         }
