@@ -186,7 +186,9 @@ struct jsc_batch {
   int64_t *d_los_off;       // [max_rays+1]
   double *d_geo;            // [max_seg][4]: z lon lat raw-ds
   double *d_pts;            // [max_seg][W]: p t ds qh2o k[nw] u[ng]
-  double *d_ctm, *d_srcp;   // [ctm_seg][nd]: continuum extinction, Planck source
+  // [ctm_seg][nd] each: continuum extinction and Planck source (variants 9-20); gas, then
+  // segment transmittance and segment source (21, 22).  Before them d_ctm is the march pool.
+  double *d_ctm, *d_srcp;
   int64_t ctm_seg;
   int64_t seg_req;          // LOS points asked for at creation
   int fail_alloc;           // the allocation from now that fails (tests), 0: none
