@@ -536,7 +536,10 @@ int jsc_batch_async_status(const jsc_batch *b);
  * jsc_batch_graph_launch re-checks the inputs those arrays hold (profile
  * offsets and ray profiles, as jsc_batch_upload) and replays the graph;
  * synchronise the stream, then read the outputs and
- * jsc_batch_async_status. */
+ * jsc_batch_async_status.  The graph holds the buffers, layers and pencils of
+ * its capture: where jsc_batch_set_aero, jsc_batch_set_nalpha or a run outside
+ * fixed-capacity mode has replaced one, a launch returns JSC_ERR_ARG; capture
+ * again. */
 int jsc_batch_graph_capture(jsc_batch *b, const jsc_batch_input *in,
                             const jsc_batch_output *out, void *stream);
 int jsc_batch_graph_launch(jsc_batch *b, void *stream);

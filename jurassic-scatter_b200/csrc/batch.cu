@@ -2386,6 +2386,29 @@ static int check_input(const jsc_batch *b, const jsc_batch_input *in) {
   return JSC_OK;
 }
 
+// Digest of what the launches of a captured run hold of b and its children
+// besides their inputs: buffers, their sizes, layers, pencils.
+static uint64_t captured_state(const jsc_batch *b) {
+  if (!b) return 0;
+  const void *p[] = {b->d_geo, b->d_pts, b->d_ctm, b->d_srcp, b->d_mnext, b->d_nlos_b, b->d_los_off_b,
+                     b->d_geo_b, b->d_pts_b, b->d_aero, b->d_beta, b->d_phase, b->d_wt, b->d_nsp,
+                     b->d_sp_off, b->d_sp_idx, b->d_sp, b->d_sp_atm, b->d_src, b->d_theta2,
+                     b->d_planck_sun, b->d_live, b->d_digest, b->child, b->sun_child};
+  const int64_t n[] = {b->max_seg, b->max_seg_b, b->mcap, b->max_sp, b->fx_max_sp, b->fx_chunk,
+                       b->fx_rounds, b->aero_nl, b->n_alti, b->nalpha};
+  const double a[] = {b->altimax, b->altimin};
+  const uint64_t c[] = {captured_state(b->child), captured_state(b->sun_child)};
+  uint64_t h = 1469598103934665603ull;  // FNV-1a
+  auto mix = [&h](const void *v, size_t bytes) {
+    for (size_t i = 0; i < bytes; i++) h = (h ^ ((const unsigned char *)v)[i]) * 1099511628211ull;
+  };
+  mix(p, sizeof(p));
+  mix(n, sizeof(n));
+  mix(a, sizeof(a));
+  mix(c, sizeof(c));
+  return h;
+}
+
 extern "C" int jsc_batch_graph_capture(jsc_batch *b, const jsc_batch_input *in,
                                        const jsc_batch_output *out, void *stream) {
   if (!b || !in || !out || !stream || !b->fixed) {
@@ -2436,12 +2459,18 @@ extern "C" int jsc_batch_graph_capture(jsc_batch *b, const jsc_batch_input *in,
   if (g) cudaGraphDestroy(g);
   if (st) return st;
   b->gin = *in;
+  b->graph_state = captured_state(b);
   b->graph_ready = 1;
   return JSC_OK;
 }
 
 extern "C" int jsc_batch_graph_launch(jsc_batch *b, void *stream) {
   if (!b || !b->graph_ready) return JSC_ERR_ARG;
+  if (captured_state(b) != b->graph_state) {
+    jsc_set_error(JSC_ERR_ARG, "jsc_batch_graph_launch: the batch's buffers, layers or pencils are "
+                               "not those of the capture; capture again");
+    return JSC_ERR_ARG;
+  }
   // the graph copies from the captured host arrays: check what they hold now
   int st = check_input(b, &b->gin);
   if (st) return st;

@@ -173,6 +173,7 @@ struct jsc_batch {
   cudaGraphExec_t gexec;
   jsc_batch_input gin;      // host inputs the graph copies from
   int graph_ready, graph_kernels;
+  uint64_t graph_state;     // what the graph holds of the batch (captured_state)
 
   // Pool of the ray march (IP 1), chunks of 32 points (trace.cuh): the memory
   // of d_ctm, which is written after the pool has been read.

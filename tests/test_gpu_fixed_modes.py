@@ -129,3 +129,53 @@ def test_pencil_count_after_fixed_mode(workdir):
     finally:
         b.close()
         m.close()
+
+
+@pytest.mark.parametrize("change", ["layers", "pencils", "growth"])
+def test_graph_of_another_state(workdir, change):
+    """A launch of a graph whose batch has other layers, another number of
+    pencils or other buffers since is refused on the host; a new capture runs
+    with the new state."""
+    import torch
+    from jscat import api, lib as L
+    ctl, inp, layers = _case(workdir, 2)
+    if change != "pencils":
+        ctl.sca_mult = 0
+    m, lib = api.Model(ctl), L.load()
+    few = _above(inp, [0, 1])
+    pin = lambda a: torch.from_numpy(np.ascontiguousarray(a)).pin_memory().numpy()   # noqa: E731
+    stream = torch.cuda.Stream()
+    gb = api.GraphBatch(m, ctl, few if change == "growth" else inp, stream.cuda_stream, pin, aero=layers,
+                        fixed_points=400, max_seg=16 if change == "growth" else 0)
+    nalpha = None
+    try:
+        gb.launch()
+        stream.synchronize()
+        gb.status()
+        if change == "layers":
+            layers = type(layers).from_buffer_copy(bytes(layers))
+            layers.trans[0] = 0.5
+            gb.batch.set_aero(layers)
+        elif change == "pencils":
+            nalpha = 10
+            gb.batch.set_nalpha(nalpha)
+        else:
+            L.check(lib.jsc_batch_set_fixed(gb.batch.h, 0))
+            _run(gb.batch, inp)
+        with pytest.raises(L.JscError) as e:
+            gb.launch()
+        assert e.value.status == 1 and "capture again" in str(e.value)   # JSC_ERR_ARG
+        L.check(lib.jsc_batch_set_fixed(gb.batch.h, 1))
+        bi, bo = gb._keep
+        for k in gb._KEYS:
+            gb.host[k][...] = inp[k]
+        L.check(lib.jsc_batch_graph_capture(gb.batch.h, C.byref(bi), C.byref(bo), stream.cuda_stream))
+        gb.launch()
+        stream.synchronize()
+        gb.status()
+        want = api.formod_batch(ctl, inp, model=m, aero=layers, nalpha=nalpha)
+        for k in KEYS:
+            np.testing.assert_array_equal(gb.out[k], want[k])
+    finally:
+        gb.close()
+        m.close()
