@@ -2327,13 +2327,13 @@ extern "C" int jsc_batch_scatter_samples(jsc_batch *b, float *feat, double *src,
 extern "C" int jsc_batch_set_fixed(jsc_batch *b, int on) {
   if (!b) return JSC_ERR_ARG;
   JSC_CUDA_TRY(cudaSetDevice(b->m->device));
+  b->fixed = 0;  // until all that a fixed run uses is there
   if (on) {
     int st;
     if (b->depth > 0 && (st = prepare_fixed_scattering(b))) return st;
     if (b->ip != 1 && b->cfg.sca_n > 0 && b->max_seg_b < b->max_seg &&
         (st = batch_alloc_los_b(b, b->max_seg)))
       return st;
-
     if (!b->h_status && cudaMallocHost((void **)&b->h_status, sizeof(unsigned)) != cudaSuccess) {
       jsc_set_error(JSC_ERR_NOMEM, "pinned host allocation");
       return JSC_ERR_NOMEM;

@@ -179,3 +179,40 @@ def test_graph_of_another_state(workdir, change):
     finally:
         gb.close()
         m.close()
+
+
+def test_failed_preparation(workdir):
+    """A larger point capacity whose allocations fail in turn: the call
+    reports it and leaves an ordinary batch, not a fixed-capacity one without
+    its buffers; the next call prepares it."""
+    from jscat import api, lib as L
+    ctl, inp, layers = _case(workdir, 2)
+    m, lib = api.Model(ctl), L.load()
+    want = api.formod_batch(ctl, inp, model=m, aero=layers)
+    failed = 0
+    for k in range(1, 20):
+        b = api.Batch(m, ctl, 1, len(inp["z"]), 2)
+        try:
+            b.set_aero(layers)
+            L.check(lib.jsc_batch_set_fixed_points(b.h, 50))
+            L.check(lib.jsc_batch_set_fixed(b.h, 1))
+            L.check(lib.jsc_batch_set_fixed_points(b.h, 1200))
+            L.check(lib.jsc_batch_fail_alloc(b.h, k))
+            st = lib.jsc_batch_set_fixed(b.h, 1)
+            L.check(lib.jsc_batch_fail_alloc(b.h, 0))
+            if st == 0:
+                break
+            assert st == 10   # JSC_ERR_NOMEM
+            failed += 1
+            for _ in range(2):   # as an ordinary batch, then prepared
+                got = _run(b, inp)
+                for c in KEYS:
+                    np.testing.assert_array_equal(got[c], want[c])
+                L.check(lib.jsc_batch_set_fixed(b.h, 1))
+            got = _run(b, inp)
+            for c in KEYS:
+                np.testing.assert_array_equal(got[c], want[c])
+        finally:
+            b.close()
+    assert failed == 3   # point records, their profiles, their sources
+    m.close()
