@@ -3,6 +3,9 @@ and scattering."""
 import numpy as np
 import pytest
 
+from test_gpu_parity import shape_case  # noqa: F401  (the fixture)
+from test_gpu_parity import test_every_launch_variant as _against_reference
+
 pytestmark = pytest.mark.gpu
 
 
@@ -73,3 +76,10 @@ def test_gas_variants_with_layers(workdir, layer, mult, n, nd):
     for k in want:
         np.testing.assert_array_equal(four[k], want[k])
         np.testing.assert_array_equal(one[k], want[k])
+
+
+@pytest.mark.parametrize("variant", [21, 22])
+def test_gas_variants_on_reference_shapes(shape_case, variant):   # noqa: F811
+    """The shapes on which the parity tests run the variants 0-20: counts and
+    table indices of the reference, radiances within its bounds."""
+    _against_reference(shape_case, variant)
